@@ -205,10 +205,10 @@ class _RouterLinear(torch.autograd.Function):
 
 class _FusedMoEFunction(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, tokens, topk_idx, topk_prob, layer):
+    def forward(ctx, tokens, topk_idx, topk_prob, layer, train):
         n = tokens.shape[0]
         out = torch.empty_like(tokens)
-        layer.rt.forward(tokens.data_ptr(), topk_idx.data_ptr(), topk_prob.data_ptr(), out.data_ptr(), n)
+        layer.rt.forward(tokens.data_ptr(), topk_idx.data_ptr(), topk_prob.data_ptr(), out.data_ptr(), n, train)
         # Backward reads what this forward left in the layer's buffers (received rows, pre-activations, routing
         # tables): one forward, then its backward.  A second forward in between would silently replace them, so
         # the forward is numbered and backward checks the number.
@@ -234,7 +234,7 @@ class _FusedMoEFunction(torch.autograd.Function):
         dprob = torch.empty_like(topk_prob)
         layer.rt.backward(dout.data_ptr(), dtokens.data_ptr(), dprob.data_ptr(), ctx.n)
         layer.bind_grads()
-        return dtokens, None, dprob, None
+        return dtokens, None, dprob, None, None
 
 
 class FusedMoE(nn.Module):
@@ -449,7 +449,8 @@ class FusedMoE(nn.Module):
     def apply_routed(self, tokens: torch.Tensor, top_idx: torch.Tensor, prob: torch.Tensor) -> torch.Tensor:
         """Expert computation for an externally made routing decision (``top_idx`` int64 ``[N, K]``, ``prob``
         fp32 ``[N, K]``): what a framework binding calls after running its own router."""
-        return _FusedMoEFunction.apply(tokens.contiguous(), top_idx.contiguous(), prob.float().contiguous(), self)
+        return _FusedMoEFunction.apply(tokens.contiguous(), top_idx.contiguous(), prob.float().contiguous(), self,
+                                       torch.is_grad_enabled())
 
     def forward(self, tokens: torch.Tensor) -> torch.Tensor:
         if tokens.dtype != torch.bfloat16 or tokens.dim() != 2 or tokens.shape[1] != self.cfg.hidden:
@@ -463,7 +464,7 @@ class FusedMoE(nn.Module):
             self.rt.forward_fp8(tokens.data_ptr(), top_idx.data_ptr(), prob.data_ptr(), out.data_ptr(), tokens.shape[0])
             self._keep = (tokens, top_idx, prob)  # alive until the enqueued kernels have read them
             return out
-        return _FusedMoEFunction.apply(tokens, top_idx, prob, self)
+        return _FusedMoEFunction.apply(tokens, top_idx, prob, self, torch.is_grad_enabled())
 
     def fused_trace_reset(self) -> None:
         if "gemm_trace" in self.loc:

@@ -10,6 +10,7 @@
 
 #include "grouped_gemm.h"
 #include "grouped_gemm_fp8.h"
+#include "narrow_gemm.h"
 #include "onesided.h"
 #include "optim.h"
 #include "route.h"
@@ -122,7 +123,7 @@ void solve_plan(torch::Tensor omega, torch::Tensor dom, torch::Tensor cost, torc
 //   mode kWgrad:       out[S, M_out, N] = P[T, M_out]^T Q[T, N] per group
 void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor out0, c10::optional<torch::Tensor> out1,
                   torch::Tensor group_off, torch::Tensor group_rows, torch::Tensor group_wslot, torch::Tensor totals,
-                  torch::Tensor status, int64_t num_sms, int64_t ctas) {
+                  torch::Tensor status, int64_t num_sms, int64_t ctas, bool narrow) {
   const c10::cuda::CUDAGuard guard(a.device());
   TORCH_CHECK(ctas == 1 || ctas == 2, "ctas must be 1 or 2");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "bf16 operands only");
@@ -137,30 +138,32 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
   g.n_groups_cap = (int)group_rows.size(0);
   g.row_capacity = (int)a.size(0);
   g.status = dptr<int>(status, "status", torch::kInt32);
-  g.out0 = out0.data_ptr();
+  g.out0 = out0.numel() > 0 ? out0.data_ptr() : nullptr;  // kFwd1 without the pre-activations
   g.out1 = out1.has_value() ? out1->data_ptr() : nullptr;
   CUtensorMap tmA, tmB;
   const uint64_t T = a.size(0);
+  const uint32_t box_rows = narrow ? epb::kNarrowBoxRows : 128;  // token rows of a box
+  TORCH_CHECK(!narrow || mode == epb::kFwd1 || mode == epb::kFwd2 || mode == epb::kDgrad1, "the narrow kernel has modes fwd1, fwd2 and dgrad1");
   bool ok = true;
   switch (mode) {
     case epb::kPlain:
     case epb::kFwd2:
       g.N = (int)b.size(1);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, 128) &&
+      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
            epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 128);
       break;
     case epb::kFwd1:
       g.N = (int)b.size(1) / 2;
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, 128) &&
+      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
            epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 128);
       break;
     case epb::kDgrad1:
     case epb::kDgrad2:
       g.N = (int)b.size(2);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, 128) &&
+      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
            epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 64);
       break;
     case epb::kWgrad:
@@ -173,6 +176,10 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
       TORCH_CHECK(false, "unknown grouped GEMM mode");
   }
   TORCH_CHECK(ok, "cuTensorMapEncodeTiled failed");
+  if (narrow) {
+    cuda_check(epb::launch_narrow_gemm(tmB, tmA, g, (int)num_sms, current_stream()), "launch_narrow_gemm");
+    return;
+  }
   cuda_check(epb::launch_grouped_gemm(tmA, tmB, g, (int)num_sms, current_stream()), "launch_grouped_gemm");
 }
 
@@ -414,7 +421,9 @@ void* mp(uint64_t a) { return reinterpret_cast<void*>(static_cast<uintptr_t>(a))
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "ep_balance_b200 native kernels (sm_100a)";
   m.def("solve_plan", &solve_plan);
-  m.def("grouped_gemm", &grouped_gemm);
+  m.def("grouped_gemm", &grouped_gemm, py::arg("mode"), py::arg("a"), py::arg("b"), py::arg("out0"), py::arg("out1"),
+        py::arg("group_off"), py::arg("group_rows"), py::arg("group_wslot"), py::arg("totals"), py::arg("status"),
+        py::arg("num_sms"), py::arg("ctas"), py::arg("narrow") = false);
   m.def("wait_probe", &wait_probe);
   m.def("adamw_step", &adamw_step, py::arg("param"), py::arg("grad"), py::arg("exp_avg"), py::arg("exp_avg_sq"),
         py::arg("lr"), py::arg("beta1"), py::arg("beta2"), py::arg("eps"), py::arg("weight_decay"), py::arg("step"),
@@ -481,9 +490,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("forward_fp8", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n) {
         r.forward_fp8(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream());
       })
-      .def("forward", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n) {
-        r.forward(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream());
-      })
+      .def("forward", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n, bool train) {
+        r.forward(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream(), train);
+      }, py::arg("tokens"), py::arg("topk_idx"), py::arg("topk_prob"), py::arg("out"), py::arg("num_tokens"), py::arg("train") = true)
       .def("backward", [](MoeRuntime& r, uint64_t dout, uint64_t dtok, uint64_t dprob, int n) {
         r.backward(cp(dout), mp(dtok), (float*)mp(dprob), n, current_stream());
       });

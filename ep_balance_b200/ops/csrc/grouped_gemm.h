@@ -37,7 +37,7 @@ struct GemmArgs {
   int K;                       // reduction extent (ignored for kWgrad: the group's padded rows)
   int M_out;                   // kWgrad only: rows of the output (columns of P)
   // epilogue operands
-  void* out0;                  // kFwd1: h [T, 2N];  kDgrad2: h (in/out);  kWgrad: dW [slots, M_out, N];
+  void* out0;                  // kFwd1: h [T, 2N] (null: not kept, and no padding row of act is written);  kDgrad2: h (in/out);  kWgrad: dW [slots, M_out, N];
                                // kPlain: C [T, N];  scatter modes with out_ptrs == null: local [T, N]
   void* out1;                  // kFwd1: act [T, N]
   const float* row_scale;      // kFwd1: optional [T] factor folded into act (the row's gate weight); null: 1
@@ -51,6 +51,7 @@ struct GemmArgs {
   // pull_cnt[s] >= pull_expected.  kWgrad waits for every M-tile of the group.
   const unsigned* arrive;
   unsigned arrive_expected;
+  int arrive_tile_rows;        // buffer rows per arrival counter (a multiple of this launch's M tile)
   const unsigned* pull_cnt;
   unsigned pull_expected;
   int home_cap;

@@ -1,0 +1,27 @@
+// Grouped GEMM for few rows per expert (narrow_gemm.cu): weights on the M side of the tensor core, token rows on its N
+// side.  Takes the GemmArgs of grouped_gemm.h with mode kFwd1 (out0 may be null: the pre-activations are not kept), kFwd2 or
+// kDgrad1, with or without the fused transport.
+#pragma once
+
+#include "grouped_gemm.h"
+
+namespace epb {
+
+constexpr int kNarrowBoxRows = 32;  // token rows of one TMA box: box of the token map {64 k, kNarrowBoxRows}
+
+// Inference batches with at most this many routed units per weight slot take the narrow kernel.  Measured, GEMM1 + GEMM2 in us,
+// wide / narrow, rows per expert spread by a lognormal of 0.35 around the mean:
+//   hidden x ffn x experts   4 rows       96 rows      128 rows     192 rows     384 rows
+//   2048 x  768 x 128        327 /  212   351 /  254   353 /  260   381 /  322   629 /  536
+//   5120 x 1536 x 160       1856 / 1176  2210 / 1397  2132 / 1867  2246 / 2312  3672 / 3808
+//   2048 x 1408 x  64        302 /  206   295 /  241   311 /  268   337 /  337   570 /  578
+// Below 128 the weights' bytes bound the launch and the narrow tiles win everywhere; from about 190 on the 256-row
+// tiles of the wide kernel are full enough, and move fewer operand bytes per flop.
+constexpr int kNarrowRowsPerSlot = 128;
+
+// tmW: the weight map that grouped_gemm.h's kernels use as B (K-major box {64, 128, 1} for kFwd1 / kFwd2, MN-major box
+// {64, 64, 1} for kDgrad1); tmX: token rows, 2-D, box {64, kNarrowBoxRows}.
+cudaError_t launch_narrow_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmArgs& args, int num_sms,
+                               cudaStream_t stream);
+
+}  // namespace epb

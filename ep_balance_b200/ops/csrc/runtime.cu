@@ -127,6 +127,8 @@ MoeRuntime::MoeRuntime(const LayerConfig& cfg, const std::map<std::string, uint6
   tmap2(&tm_act_k_, ptr<void>("act"), T, F, 64, 128);
   tmap2(&tm_dy_k_, ptr<void>("dybuf"), T, H, 64, 128);
   tmap2(&tm_dh_k_, ptr<void>("hbuf"), T, 2 * F, 64, 128);
+  tmap2(&tm_x_n_, ptr<void>("xbuf"), T, H, 64, kNarrowBoxRows);
+  tmap2(&tm_act_n_, ptr<void>("act"), T, F, 64, kNarrowBoxRows);
   // weights, K-major B: box {64 k, 128 n, 1}
   tmap3(&tm_w1_k_, ptr<void>("w1"), S, 2 * F, H, 64, 128);
   tmap3(&tm_w2_k_, ptr<void>("w2"), S, H, F, 64, 128);
@@ -309,6 +311,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
   if (extra.gate) {
     g.arrive = ptr<const unsigned>("arrive") + (extra.gate == 2 ? n_tiles_ : 0);
     g.arrive_expected = (unsigned)(cfg_.R * (tile_rows_ / block_rows_));
+    g.arrive_tile_rows = tile_rows_;
   }
   if (extra.gate_pull && cfg_.w_slots > cfg_.home_cap) {
     g.pull_cnt = ptr<const unsigned>("arrive") + 2 * n_tiles_;  // counters of w1 (the B operand of GEMM1)
@@ -328,30 +331,42 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
     g.trace = ptr<unsigned long long>("gemm_trace", false);  // optional: phase timestamps of the fused kernels
     if (g.trace != nullptr) g.trace += mode == kFwd1 ? 0 : 12;
   }
-  check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
+  if (extra.narrow)  // a: token rows, b: weights, as for the wide kernel
+    check(launch_narrow_gemm(b, a, g, cfg_.num_sms, stream), extra.comm ? "narrow_gemm+transport" : "narrow_gemm");
+  else
+    check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
 }
 
-void MoeRuntime::gemm1(cudaStream_t stream) {
+// An inference batch with few rows per expert reads the weights once and does little else.  (About num_units rows reach
+// every rank: the plan keeps the ranks near the mean.)
+bool MoeRuntime::use_narrow(int num_units) const { return num_units <= kNarrowRowsPerSlot * cfg_.w_slots; }
+
+void MoeRuntime::gemm1(cudaStream_t stream, bool train, bool narrow) {
   GemmExtra x;
+  x.narrow = narrow;
   x.gate = 1;
   x.gate_pull = true;
   x.row_scale = ptr<const float>("rowp");
-  gemm(kFwd1, tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, ptr<void>("hbuf"), ptr<void>("act"), nullptr, nullptr, stream, x);
+  gemm(kFwd1, narrow ? tm_x_n_ : tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
+       nullptr, nullptr, stream, x);
 }
-void MoeRuntime::gemm1_fused(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream) {
+void MoeRuntime::gemm1_fused(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream, bool train) {
   if (num_units > cfg_.max_units) throw std::runtime_error("MoeRuntime: more routing units than max_units");
-  const CommArgs a = comm_forward(tokens, topk_prob, true, true);
+  const CommArgs a = comm_forward(tokens, topk_prob, train, true);
   GemmExtra x;
+  x.narrow = !train && use_narrow(num_units);
   x.gate = 1;
   x.gate_pull = true;
   x.row_scale = ptr<const float>("rowp");
   x.comm = &a;
-  gemm(kFwd1, tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, ptr<void>("hbuf"), ptr<void>("act"), nullptr, nullptr, stream, x);
+  gemm(kFwd1, x.narrow ? tm_x_n_ : tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
+       nullptr, nullptr, stream, x);
 }
-void MoeRuntime::gemm2(cudaStream_t stream) {
+void MoeRuntime::gemm2(cudaStream_t stream, bool narrow) {
   GemmExtra x;
   x.done_slot = 2;
-  gemm(kFwd2, tm_act_k_, tm_w2_k_, cfg_.H, cfg_.F, 0, nullptr, nullptr, ptr<void* const>("ybuf_ptrs"),
+  x.narrow = narrow;
+  gemm(kFwd2, narrow ? tm_act_n_ : tm_act_k_, tm_w2_k_, cfg_.H, cfg_.F, 0, nullptr, nullptr, ptr<void* const>("ybuf_ptrs"),
        ptr<const int2>("meta"), stream, x);
 }
 UnitReduceWait MoeRuntime::reduce_wait(int slot) const {
@@ -592,8 +607,9 @@ std::vector<std::pair<std::string, float>> MoeRuntime::phase_times() {
 
 // ------------------------------------------------------------------ whole passes
 void MoeRuntime::forward(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out,
-                         int num_tokens, cudaStream_t stream) {
+                         int num_tokens, cudaStream_t stream, bool train) {
   const int U = num_tokens * cfg_.topk;
+  const bool narrow = !train && use_narrow(U);
   mark("fwd_begin", stream);
   publish(topk_idx, U, stream);
   mark("publish", stream);
@@ -602,16 +618,16 @@ void MoeRuntime::forward(const void* tokens, const int64_t* topk_idx, const floa
   route(topk_idx, U, stream);
   mark("route", stream);
   if (cfg_.fused_comm) {
-    gemm1_fused(tokens, topk_prob, U, stream);
+    gemm1_fused(tokens, topk_prob, U, stream, train);
     mark("dispatch+pull+gemm1", stream);
   } else {
-    dispatch_tokens(tokens, topk_prob, U, stream);
+    dispatch_tokens(tokens, topk_prob, U, stream, train);
     pull_weights(stream);
     mark("dispatch+pull", stream);
-    gemm1(stream);
+    gemm1(stream, train, narrow);
     mark("gemm1", stream);
   }
-  gemm2(stream);
+  gemm2(stream, narrow);
   mark("gemm2", stream);
   reduce_out(out, num_tokens, stream, true);
   mark("reduce_out", stream);

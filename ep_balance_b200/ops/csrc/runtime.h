@@ -14,6 +14,7 @@
 
 #include "grouped_gemm.h"
 #include "grouped_gemm_fp8.h"
+#include "narrow_gemm.h"
 #include "route.h"
 #include "solver.h"
 
@@ -53,11 +54,13 @@ class MoeRuntime {
   void dispatch_tokens(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream, bool zero_pad = true);
   void pull_weights(cudaStream_t stream);   // stand-alone replica weight pull (per-slot counters advanced)
   void barrier(int slot, cudaStream_t stream);
-  void gemm1(cudaStream_t stream);          // gated per M-tile on the arrival counters, per replica slot on the pull counters
+  void gemm1(cudaStream_t stream, bool train = true, bool narrow = false);  // gated per M-tile on the arrival counters, per replica slot on the pull counters
   // One kernel: transport warps send this rank's rows and pull its replica weights while the other
   // warps run GEMM1 on the tiles whose rows have arrived.
-  void gemm1_fused(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream);
-  void gemm2(cudaStream_t stream);          // rows stored to their source ranks; the last CTA signals every peer
+  // train = false: nothing is kept for a backward pass (no padding rows, no pre-activations), and a batch with few rows
+  // per expert runs on the narrow kernel.
+  void gemm1_fused(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream, bool train = true);
+  void gemm2(cudaStream_t stream, bool narrow = false);  // rows stored to their source ranks; the last CTA signals every peer
   // Sum of every token's unit rows (already gate-weighted: the weight was folded into the activation).
   // wait_peers: first wait (bounded, in the kernel) for every rank's completion signal of gemm2.
   // unit_scale (fp8 inference path only): the rows are unweighted and scaled here.
@@ -89,7 +92,7 @@ class MoeRuntime {
 
   // ---- whole passes
   void forward(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out, int num_tokens,
-               cudaStream_t stream);
+               cudaStream_t stream, bool train = true);
   void backward(const void* dout, void* dtokens, float* dprob, int num_tokens, cudaStream_t stream);
 
   // Optional per-phase device timing: events are recorded around every phase of forward() and
@@ -118,6 +121,7 @@ class MoeRuntime {
     int done_slot = 0;   // > 0: signal every peer on this slot when the launch is complete
     const float* row_scale = nullptr;
     const CommArgs* comm = nullptr;
+    bool narrow = false; // few rows per expert: weights on the M side (narrow_gemm.h)
   };
   void gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int N, int K, int M_out, void* out0, void* out1,
             void* const* out_ptrs, const int2* meta, cudaStream_t stream, const GemmExtra& extra);
@@ -129,6 +133,7 @@ class MoeRuntime {
   CommArgs comm_forward(const void* tokens, const float* topk_prob, bool pad, bool pull) const;
   CommArgs comm_backward(const void* dout) const;
   void swiglu_pass(cudaStream_t stream);
+  bool use_narrow(int num_units) const;
   bool peers() const { return cfg_.multi_rank_sync && cfg_.R > 1; }
   UnitReduceWait reduce_wait(int slot) const;
   void tmap2(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t bc, uint32_t br);
@@ -152,6 +157,7 @@ class MoeRuntime {
   // tensor maps (built once: every buffer has a fixed address)
   CUtensorMap tm_x_k_, tm_act_k_, tm_dy_k_, tm_dh_k_;           // K-major A operands
   CUtensorMap tm_w1_k_, tm_w2_k_, tm_w1_mn_, tm_w2_mn_;          // weights as B
+  CUtensorMap tm_x_n_, tm_act_n_;                                // token rows as the narrow kernel's N operand
   CUtensorMap tm_dy_mn_, tm_act_mn_, tm_dh_mn_, tm_x_mn_;        // Wgrad operands (MN-major)
   bool fp8_ = false;
   bool fp8_pair_ = true;   // CTA-pair fp8 kernel (256-row tiles); forward_fp8 falls back to 128-row tiles for tiny batches
