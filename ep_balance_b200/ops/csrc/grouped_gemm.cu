@@ -56,7 +56,6 @@ struct Tile {
   int rows;      // real rows of the group
   int row0;      // first buffer row of the group
   int wslot;
-  int kblocks;
 };
 
 struct Shape {
@@ -75,9 +74,12 @@ __device__ __forceinline__ Shape make_shape(const GemmArgs& a) {
   return s;
 }
 
-template <int kMode>
-__device__ __forceinline__ bool find_tile(const GemmArgs& a, const Shape& s, const int* tile_prefix, int t, Tile& out) {
-  int g = 0;
+// Tile t of the list.  `g` is the caller's cursor (0 before its first tile): tile indices only grow, so the walk over the
+// groups goes on where it stopped.  The producer and the MMA issuer call this for their NEXT tile before they work on
+// the current one: the three loads from the group table are then in flight during a whole tile instead of standing
+// between two tiles with nothing queued on the tensor cores (with the walk from group 0 that gap was 1-2 thousand
+// cycles, beside 6 thousand of MMAs in a Wgrad tile of 768 rows).
+__device__ __forceinline__ bool find_tile(const GemmArgs& a, const Shape& s, const int* tile_prefix, int t, int& g, Tile& out) {
   while (g < s.n_groups && t >= tile_prefix[g + 1]) ++g;
   if (g >= s.n_groups) return false;
   const int local = t - tile_prefix[g];
@@ -87,8 +89,11 @@ __device__ __forceinline__ bool find_tile(const GemmArgs& a, const Shape& s, con
   out.rows = a.group_rows[g];
   out.row0 = a.group_off[g];
   out.wslot = a.group_wslot[g];
-  out.kblocks = kMode == kWgrad ? ceil_div(out.rows, BK) : s.kblocks_fixed;
   return true;
+}
+template <int kMode>
+__device__ __forceinline__ int k_blocks(const Shape& s, const Tile& t) {
+  return kMode == kWgrad ? ceil_div(t.rows, BK) : s.kblocks_fixed;
 }
 
 // ---------------------------------------------------------------- staged, row-contiguous stores
@@ -193,13 +198,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_init(&acc_empty[b], 8 * kCtas);
     }
     *abort_flag = 0;
-    int acc = 0;
-    tile_prefix[0] = 0;
-    for (int g = 0; g < shape.n_groups; ++g) {
-      int mt = kMode == kWgrad ? shape.m_tiles_fixed : ceil_div(args.group_rows[g], TILE_M);
-      acc += mt * shape.n_tiles_n;
-      tile_prefix[g + 1] = acc;
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -207,6 +205,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (kCtas == 2) tmem_alloc_pair(tmem_slot, TMEM_COLS);
     else tmem_alloc(tmem_slot, TMEM_COLS);
   }
+  if (warp == 2)
+    warp_tile_prefix(tile_prefix, shape.n_groups, lane, [&](int g) {
+      return (kMode == kWgrad ? shape.m_tiles_fixed : ceil_div(args.group_rows[g], TILE_M)) * shape.n_tiles_n;
+    });
   tc_fence_before();
   __syncthreads();
   if (kCtas == 2) cluster_sync_all();  // the peer's barriers exist before anything signals them
@@ -218,26 +220,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     // The warp walks the tile list together; lane 0 issues the TMA loads.
-    int stage = 0;
+    int stage = 0, cursor = 0;
     uint32_t phase = 0;
-    Tile t;
+    Tile t, next;
+    bool have = find_tile(args, shape, tile_prefix, tile_first, cursor, t);
     const unsigned long long wait_ns = args.wait_ns ? args.wait_ns : kWaitBudgetNs;
-    int seen_mtile = -1, seen_group = -1, seen_slot = -1;  // waits already satisfied
-    for (int ti = tile_first; ti < total_tiles; ti += tile_stride) {
+    int seen_mtile = -1, seen_slot = -1;  // waits already satisfied
+    for (int ti = tile_first; have; ti += tile_stride) {
       int go = 1;
+      const bool have_next = find_tile(args, shape, tile_prefix, ti + tile_stride, cursor, next);
       if (lane == 0) {
-        if (*abort_v || !find_tile<kMode>(args, shape, tile_prefix, ti, t)) go = 0;
-        if (go && args.arrive != nullptr) {
-          // rows of this tile (kWgrad: of the whole group) must have arrived from every sender
+        if (*abort_v) go = 0;
+        if (go && kMode != kWgrad && args.arrive != nullptr) {
+          // rows of this tile must have arrived from every sender
           const int first = t.row0 / TILE_M;
-          if (kMode == kWgrad) {
-            if (t.g != seen_group) {
-              const int n = ceil_div(min(t.rows, args.row_capacity - t.row0), TILE_M);
-              for (int i = 0; i < n && go; ++i)
-                if (!flag_wait<true>(args.arrive + first + i, args.arrive_expected, wait_ns, abort_v, args.status, 5, first + i)) go = 0;
-              seen_group = t.g;
-            }
-          } else if (first + t.mt != seen_mtile && (t.row0 + t.mt * TILE_M) < args.row_capacity) {
+          if (first + t.mt != seen_mtile && (t.row0 + t.mt * TILE_M) < args.row_capacity) {
             if (!flag_wait<true>(args.arrive + first + t.mt, args.arrive_expected, wait_ns, abort_v, args.status, 5, first + t.mt)) go = 0;
             seen_mtile = first + t.mt;
           }
@@ -250,7 +247,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const int m_off = t.mt * TILE_M + cta_rank * BM;            // this CTA's rows of the tile
           const int n_off = t.nt * BN + cta_rank * (BN / 2) * (kCtas - 1);  // this CTA's columns of B
           constexpr int kBoxesB = 4 / kCtas;                          // 64-wide MN-major boxes of B
-          for (int kb = 0; kb < t.kblocks; ++kb) {
+          const int kblocks = k_blocks<kMode>(shape, t);
+          for (int kb = 0; kb < kblocks; ++kb) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_v, args.status, 1)) {
               go = 0;
               break;
@@ -289,17 +287,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
       go = __shfl_sync(0xffffffffu, go, 0);
       if (!go) break;
+      t = next;
+      have = have_next;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (lane == 0 && cta_rank == 0) {
-      int stage = 0;
+      int stage = 0, cursor = 0;
       uint32_t phase = 0;
       uint32_t acc_phase[2] = {0, 0};
       int local = 0;
-      Tile t;
-      for (int ti = tile_first; ti < total_tiles && !*abort_v; ti += tile_stride, ++local) {
-        if (!find_tile<kMode>(args, shape, tile_prefix, ti, t)) break;
+      Tile t, next;
+      bool have = find_tile(args, shape, tile_prefix, tile_first, cursor, t);
+      for (int ti = tile_first; have && !*abort_v; ti += tile_stride, ++local, t = next) {
+        have = find_tile(args, shape, tile_prefix, ti + tile_stride, cursor, next);
         const int buf = local & 1;
         if (!mbar_wait(&acc_empty[buf], acc_phase[buf] ^ 1u, abort_v, args.status, 2)) break;
         acc_phase[buf] ^= 1u;
@@ -318,7 +319,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         const uint32_t idesc = make_idesc(kAMn, kBMn, ncols, TILE_M);
         bool failed = false;
-        for (int kb = 0; kb < t.kblocks; ++kb) {
+        const int kblocks = k_blocks<kMode>(shape, t);
+        for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) {
             failed = true;
             break;
@@ -380,18 +382,36 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int half = (warp - 2) >> 2;  // which half of the tile's column chunks this warp handles
     uint4* stg = stage_tiles + (warp - 2) * (kStageWarpBytes / 16);
     uint32_t acc_phase[2] = {0, 0};
-    int local = 0;
+    int local = 0, cursor = 0;
     Tile t;
     char* out0 = reinterpret_cast<char*>(args.out0);
     char* out1 = reinterpret_cast<char*>(args.out1);
     for (int ti = tile_first; ti < total_tiles && !*abort_v; ti += tile_stride, ++local) {
-      if (!find_tile<kMode>(args, shape, tile_prefix, ti, t)) break;
+      if (!find_tile(args, shape, tile_prefix, ti, cursor, t)) break;
       const int buf = local & 1;
+      const int r_in_tile = cta_rank * BM + quarter * 32 + lane;  // row inside the (pair's) M tile
+      // where this lane's row goes, looked up while the tile is still being computed
+      char* orow = nullptr;
+      if (kMode == kWgrad) {
+        const int m = t.mt * TILE_M + r_in_tile;
+        if (m < args.M_out) orow = out0 + ((size_t)t.wslot * args.M_out + m) * (size_t)args.N * 2;
+      } else if (kMode != kFwd1 && kMode != kDgrad2) {
+        const int row_in_group = t.mt * TILE_M + r_in_tile;
+        const size_t row = (size_t)t.row0 + row_in_group;
+        if (row_in_group < t.rows && row < (size_t)args.row_capacity) {
+          if (args.meta != nullptr) {
+            const int2 mt = args.meta[row];
+            char* base = args.out_ptrs ? reinterpret_cast<char*>(args.out_ptrs[mt.x]) : out0;
+            orow = base + (size_t)mt.y * args.N * 2;
+          } else {
+            orow = out0 + row * (size_t)args.N * 2;
+          }
+        }
+      }
       if (!mbar_wait(&acc_full[buf], acc_phase[buf], abort_v, args.status, 4)) break;
       acc_phase[buf] ^= 1u;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
-      const int r_in_tile = cta_rank * BM + quarter * 32 + lane;  // row inside the (pair's) M tile
 
       if (kMode == kFwd1) {
         const int row_in_group = t.mt * TILE_M + r_in_tile;
@@ -485,28 +505,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       } else {
         // kFwd2 / kDgrad1 / kPlain: plain rows, optionally scattered to the unit's source rank.
         // kWgrad: rows of the weight gradient of this group's slot.
-        char* orow = nullptr;
-        int n_total = args.N;
-        bool have_acc = true;
-        if (kMode == kWgrad) {
-          const int m = t.mt * TILE_M + r_in_tile;
-          if (m < args.M_out) orow = out0 + ((size_t)t.wslot * args.M_out + m) * (size_t)args.N * 2;
-          have_acc = t.kblocks > 0;  // an expert that received no rows has a zero gradient
-        } else {
-          const int row_in_group = t.mt * TILE_M + r_in_tile;
-          const size_t row = (size_t)t.row0 + row_in_group;
-          if (row_in_group < t.rows && row < (size_t)args.row_capacity) {
-            if (args.meta != nullptr) {
-              const int2 mt = args.meta[row];
-              char* base = args.out_ptrs ? reinterpret_cast<char*>(args.out_ptrs[mt.x]) : out0;
-              orow = base + (size_t)mt.y * args.N * 2;
-            } else {
-              orow = out0 + row * (size_t)args.N * 2;
-            }
-          }
-        }
+        const bool have_acc = kMode != kWgrad || t.rows > 0;  // an expert that received no rows has a zero gradient
         const int col0 = t.nt * BN;
-        const int nchunks = min(BN / 32, (n_total - col0) / 32);
+        const int nchunks = min(BN / 32, (args.N - col0) / 32);
         uint32_t v[2][32];
         const int cb = half * 4;  // this warp's four 32-column chunks
         if (have_acc && cb < nchunks) tmem_ld32(taddr + cb * 32, v[0]);

@@ -48,7 +48,8 @@ struct GemmArgs {
   // ---- operand gating (each may be null).  The TMA producer polls before the first load of a tile:
   // the A rows of M-tile i are complete when arrive[i] >= arrive_expected (counters written by the
   // senders' transport, CommArgs); the weights of replica slot s (wslot - home_cap) are complete when
-  // pull_cnt[s] >= pull_expected.  kWgrad waits for every M-tile of the group.
+  // pull_cnt[s] >= pull_expected.  kWgrad takes no gate: it runs after a
+  // GEMM that waited for the same rows.
   const unsigned* arrive;
   unsigned arrive_expected;
   int arrive_tile_rows;        // buffer rows per arrival counter (a multiple of this launch's M tile)

@@ -154,9 +154,10 @@ struct Tile {
   int g, mt, nt, rows, row0, wslot;
 };
 
+// `g` is the caller's cursor (0 before its first tile): tile indices only grow.  The producer and the MMA issuer look their
+// next tile up before they work on the current one, as in grouped_gemm.cu.
 __device__ __forceinline__ bool find_tile(const Fp8GemmArgs& a, int n_groups, int n_tiles_n, const int* tile_prefix,
-                                          int t, Tile& out) {
-  int g = 0;
+                                          int t, int& g, Tile& out) {
   while (g < n_groups && t >= tile_prefix[g + 1]) ++g;
   if (g >= n_groups) return false;
   const int local = t - tile_prefix[g];
@@ -232,16 +233,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       mbar_init(&acc_empty[b], 8);
     }
     *abort_flag = 0;
-    int acc = 0;
-    tile_prefix[0] = 0;
-    for (int g = 0; g < n_groups; ++g) {
-      acc += ceil_div(args.group_rows[g], BM) * n_tiles_n;
-      tile_prefix[g + 1] = acc;
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+  if (warp == 2)
+    warp_tile_prefix(tile_prefix, n_groups, lane, [&](int g) { return ceil_div(args.group_rows[g], BM) * n_tiles_n; });
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -251,13 +248,15 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    int stage = 0;
+    int stage = 0, cursor = 0;
     uint32_t phase = 0;
-    Tile t;
-    for (int ti = blockIdx.x; ti < total_tiles; ti += gridDim.x) {
+    Tile t, next;
+    bool have = find_tile(args, n_groups, n_tiles_n, tile_prefix, blockIdx.x, cursor, t);
+    for (int ti = blockIdx.x; have; ti += gridDim.x, t = next) {
       int go = 1;
+      have = find_tile(args, n_groups, n_tiles_n, tile_prefix, ti + gridDim.x, cursor, next);
       if (lane == 0) {
-        if (*abort_v || !find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) go = 0;
+        if (*abort_v) go = 0;
         if (go) {
           const int row_tile = (t.row0 + t.mt * BM) / BM;
           const uint8_t* sfa = args.sfa + (size_t)row_tile * kgroups * 512;
@@ -297,9 +296,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       uint32_t acc_phase[2] = {0, 0};
       int local = 0;
       uint32_t sf_buf = 0;  // two sets of scale columns: the copy for k-group g+1 never races the MMAs of g
-      Tile t;
-      for (int ti = blockIdx.x; ti < total_tiles && !*abort_v; ti += gridDim.x, ++local) {
-        if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) break;
+      int cursor = 0;
+      Tile t, next;
+      bool have = find_tile(args, n_groups, n_tiles_n, tile_prefix, blockIdx.x, cursor, t);
+      for (int ti = blockIdx.x; have && !*abort_v; ti += gridDim.x, ++local, t = next) {
+        have = find_tile(args, n_groups, n_tiles_n, tile_prefix, ti + gridDim.x, cursor, next);
         const int buf = local & 1;
         if (!mbar_wait(&acc_empty[buf], acc_phase[buf] ^ 1u, abort_v, args.status, 12)) break;
         acc_phase[buf] ^= 1u;
@@ -347,11 +348,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const int half = (warp - 2) >> 2;  // columns [64*half, +64) of the tile
     uint4* stg = stage_tiles + (warp - 2) * (kStageWarpBytes / 16);
     uint32_t acc_phase[2] = {0, 0};
-    int local = 0;
+    int local = 0, cursor = 0;
     Tile t;
     char* out0 = reinterpret_cast<char*>(args.out);
     for (int ti = blockIdx.x; ti < total_tiles && !*abort_v; ti += gridDim.x, ++local) {
-      if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) break;
+      if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, cursor, t)) break;
       const int buf = local & 1;
       if (!mbar_wait(&acc_full[buf], acc_phase[buf], abort_v, args.status, 14)) break;
       acc_phase[buf] ^= 1u;
@@ -518,16 +519,12 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
       mbar_init(&acc_empty[b], 16);   // 8 epilogue warps of each CTA
     }
     *abort_flag = 0;
-    int acc = 0;
-    tile_prefix[0] = 0;
-    for (int g = 0; g < n_groups; ++g) {
-      acc += ceil_div(args.group_rows[g], TILE_M) * n_tiles_n;
-      tile_prefix[g + 1] = acc;
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) tmem_alloc2(tmem_slot, TMEM_COLS);
+  if (warp == 2)
+    warp_tile_prefix(tile_prefix, n_groups, lane, [&](int g) { return ceil_div(args.group_rows[g], TILE_M) * n_tiles_n; });
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the peer's barriers exist before anything signals them
@@ -538,13 +535,15 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
-    int stage = 0;
+    int stage = 0, cursor = 0;
     uint32_t phase = 0;
-    Tile t;
-    for (int ti = tile_first; ti < total_tiles; ti += tile_stride) {
+    Tile t, next;
+    bool have = find_tile(args, n_groups, n_tiles_n, tile_prefix, tile_first, cursor, t);
+    for (int ti = tile_first; have; ti += tile_stride, t = next) {
       int go = 1;
+      have = find_tile(args, n_groups, n_tiles_n, tile_prefix, ti + tile_stride, cursor, next);
       if (lane == 0) {
-        if (*abort_v || !find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) go = 0;
+        if (*abort_v) go = 0;
         if (go) {
           const int row_first = t.row0 + t.mt * TILE_M + cta_rank * BM;
           const int sfa_chunk = (row_first / BM) * kgroups;
@@ -586,9 +585,11 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
       uint32_t acc_phase[2] = {0, 0};
       int local = 0;
       uint32_t sf_buf = 0;
-      Tile t;
-      for (int ti = tile_first; ti < total_tiles && !*abort_v; ti += tile_stride, ++local) {
-        if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) break;
+      int cursor = 0;
+      Tile t, next;
+      bool have = find_tile(args, n_groups, n_tiles_n, tile_prefix, tile_first, cursor, t);
+      for (int ti = tile_first; have && !*abort_v; ti += tile_stride, ++local, t = next) {
+        have = find_tile(args, n_groups, n_tiles_n, tile_prefix, ti + tile_stride, cursor, next);
         const int buf = ACC_BUFS == 2 ? (local & 1) : 0;
         if (!mbar_wait(&acc_empty[buf], acc_phase[buf] ^ 1u, abort_v, args.status, 22)) break;
         acc_phase[buf] ^= 1u;
@@ -641,11 +642,11 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
     const int half = (warp - 2) >> 2;
     uint4* stg = stage_tiles + (warp - 2) * (kStageWarpBytes / 16);
     uint32_t acc_phase[2] = {0, 0};
-    int local = 0;
+    int local = 0, cursor = 0;
     Tile t;
     char* out0 = reinterpret_cast<char*>(args.out);
     for (int ti = tile_first; ti < total_tiles && !*abort_v; ti += tile_stride, ++local) {
-      if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, t)) break;
+      if (!find_tile(args, n_groups, n_tiles_n, tile_prefix, ti, cursor, t)) break;
       const int buf = ACC_BUFS == 2 ? (local & 1) : 0;
       if (!mbar_wait(&acc_full[buf], acc_phase[buf], abort_v, args.status, 24)) break;
       acc_phase[buf] ^= 1u;

@@ -507,10 +507,9 @@ void MoeRuntime::dispatch_grads(const void* dout, int num_units, cudaStream_t st
   const CommArgs a = comm_backward(dout);
   check(launch_comm(a, cfg_.num_sms, sp_.status, stream), "dispatch_grads");
 }
+// No gate: Dgrad2, earlier on this stream, has waited for every gradient row of this rank.
 void MoeRuntime::wgrad2(cudaStream_t stream) {
-  GemmExtra x;
-  x.gate = 2;
-  gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream, x);
+  gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream);
 }
 void MoeRuntime::swiglu_pass(cudaStream_t stream) {
   SwigluBwdArgs a{};

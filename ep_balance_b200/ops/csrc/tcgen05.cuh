@@ -230,26 +230,7 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t v) {
 }
 __device__ __forceinline__ float sigmoidf_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
-// ---------------------------------------------------------------- group walk, completion
-// prefix[g + 1] = tiles of groups 0..g, by one warp: 32 groups per step (`tiles(g)` reads the group's row count from
-// global memory, so a serial walk would pay that latency once per group).
-template <typename F>
-__device__ __forceinline__ void warp_tile_prefix(int* prefix, int n_groups, int lane, F tiles) {
-  int run = 0;
-  for (int g0 = 0; g0 < n_groups; g0 += 32) {
-    const int g = g0 + lane;
-    int incl = g < n_groups ? tiles(g) : 0;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    if (g < n_groups) prefix[g + 1] = run + incl;
-    run += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (lane == 0) prefix[0] = 0;
-}
-
+// ---------------------------------------------------------------- completion
 // One thread per CTA, after the CTA's (peer) stores are fenced: the last CTA of the launch tells every peer.
 __device__ __forceinline__ void signal_launch_done(const GemmArgs& args) {
   __threadfence_system();
