@@ -160,9 +160,26 @@ __device__ __forceinline__ void wide_flush(const uint4* tile, int lane, char* ro
     if (base != 0ull && p < pieces) *reinterpret_cast<uint4*>(base + byte_off + p * 16) = tile[wide_index(r, p)];
   }
 }
+// Accumulating form for fp32 rows: 32 rows x 128 B (32 columns) of `tile` are added to memory, eight passes of four rows.  `p`
+// is the lane's address in the first pass, `step` the bytes between passes, `rows` the rows that exist from the lane's first.
+// A vector reduction needs no load to wait for and no registers for the old values; every element has one writer.  Bound by
+// HBM: 8 bytes a weight.  64 experts of 2048 x 1024, two micro-batches of 1531 tokens: 1.62 ms for the four Wgrads (4.0 TB/s
+// of read and write), where plain Wgrads (0.74) and the pass that added their bf16 slots (1.25) took 1.99.
+__device__ __forceinline__ void wide_add(const uint4* tile, int lane, char* p, size_t step, int rows) {
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    if (it * 4 < rows) {
+      const uint4 v = tile[wide_index(it * 4 + (lane >> 3), lane & 7)];
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + it * step), "f"(__uint_as_float(v.x)),
+                   "f"(__uint_as_float(v.y)), "f"(__uint_as_float(v.z)), "f"(__uint_as_float(v.w))
+                   : "memory");
+    }
+  }
+}
 // ---------------------------------------------------------------- kernel
 // kComm: 0 = GEMM only; 1 = plus two transport warps (token or gradient rows to their hosts, replica weights in).
-template <int kMode, int kCtas, int kComm>
+// kAccum (kWgrad): owned slots are added to args.accum instead of being stored.
+template <int kMode, int kCtas, int kComm, bool kAccum>
 __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ GemmArgs args) {
@@ -413,7 +430,32 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
 
-      if (kMode == kFwd1) {
+      if (kAccum && t.wslot < args.home_cap) {
+        const int col0 = t.nt * BN;
+        const int nchunks = t.rows > 0 ? min(BN / 32, (args.N - col0) / 32) : 0;  // no rows: nothing to add
+        const int cb = half * 4;
+        const int m0 = t.mt * TILE_M + cta_rank * BM + quarter * 32 + (lane >> 3);  // this lane's row of the first pass
+        const int rows = args.M_out - m0;
+        const size_t step = (size_t)args.N * 16;  // four rows of fp32
+        char* p = reinterpret_cast<char*>(args.accum + ((size_t)t.wslot * args.M_out + m0) * (size_t)args.N + col0 + cb * 32) +
+                  (lane & 7) * 16;
+        uint32_t v[2][32];
+        if (cb < nchunks) tmem_ld32(taddr + cb * 32, v[0]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int c = cb + k;
+          if (c < nchunks) {
+            tmem_ld_wait();
+            if (k + 1 < 4 && c + 1 < nchunks) tmem_ld32(taddr + (c + 1) * 32, v[(k + 1) & 1]);
+            uint32_t(&w)[32] = v[k & 1];
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) stg[wide_index(lane, i)] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+            __syncwarp();
+            wide_add(stg, lane, p + k * 128, step, rows);
+          }
+        }
+      } else if (kMode == kFwd1) {
         const int row_in_group = t.mt * TILE_M + r_in_tile;
         const size_t row = (size_t)t.row0 + row_in_group;  // rows up to the padded end exist in the buffers
         const bool in_buf = row < (size_t)args.row_capacity;
@@ -609,14 +651,14 @@ bool make_tmap_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t r
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kMode, int kCtas, int kComm>
+template <int kMode, int kCtas, int kComm, bool kAccum = false>
 static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
                                cudaStream_t stream) {
   static bool configured[kMaxTrackedDevices] = {};
   constexpr size_t smem = smem_bytes<kCtas, kComm>();
   int dev;
   if (device_needs_setup(configured, &dev)) {
-    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kCtas, kComm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     device_setup_done(configured, dev);
@@ -633,7 +675,7 @@ static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, c
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm>, tmA, tmB, args);
+  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, args);
 }
 
 template <int kCtas>
@@ -651,7 +693,9 @@ static cudaError_t launch_ctas(const CUtensorMap& tmA, const CUtensorMap& tmB, c
     case kFwd2: return launch_mode<kFwd2, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kDgrad2: return launch_mode<kDgrad2, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kDgrad1: return launch_mode<kDgrad1, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kWgrad: return launch_mode<kWgrad, kCtas, 0>(tmA, tmB, args, num_sms, stream);
+    case kWgrad:
+      if (args.accum != nullptr) return launch_mode<kWgrad, kCtas, 0, true>(tmA, tmB, args, num_sms, stream);
+      return launch_mode<kWgrad, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kPlain: return launch_mode<kPlain, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     default: return cudaErrorInvalidValue;
   }

@@ -43,6 +43,8 @@ struct GemmArgs {
   const float* row_scale;      // kFwd1: optional [T] factor folded into act (the row's gate weight); null: 1
   void* const* out_ptrs;       // scatter modes: R peer buffers [units, N] (null -> local out0)
   const int2* meta;            // scatter modes: {src rank, row in that rank's buffer} per row
+  float* accum;                // kWgrad, may be null: fp32 [home_cap, M_out, N]; the gradient of a slot below home_cap is added
+                               // there from the fp32 accumulators and its slot of out0 is not written
   int* status;
   unsigned long long wait_ns;  // budget of the waits below (0: the library default)
   // ---- operand gating (each may be null).  The TMA producer polls before the first load of a tile:

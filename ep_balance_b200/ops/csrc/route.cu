@@ -308,7 +308,8 @@ __global__ void __launch_bounds__(512) grad_reduce_kernel(GradReduceArgs a) {
   __syncthreads();
   const int n = n_hosts;
   const bool accumulate = a.accum != nullptr;
-  if (n == 0 && !accumulate) return;  // no replicas: the owner's own slot gradient is already final
+  const bool own_slot = !a.include_self && !a.skip_self;
+  if (n == 0 && (!accumulate || a.skip_self)) return;  // no replicas: the owner's gradient is already where it belongs
   const size_t n_vec = a.elems_per_slot / 8;
   uint4* mine = reinterpret_cast<uint4*>(a.g_ptrs[a.me]) + (size_t)home * n_vec;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -324,11 +325,11 @@ __global__ void __launch_bounds__(512) grad_reduce_kernel(GradReduceArgs a) {
       const size_t i = i0 + (size_t)j * stride;
 #pragma unroll
       for (int c = 0; c < 8; ++c) acc[j][c] = 0.f;
-      own[j] = (!a.include_self && i < n_vec) ? mine[i] : make_uint4(0, 0, 0, 0);
+      own[j] = (own_slot && i < n_vec) ? mine[i] : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int j = 0; j < kUnroll; ++j)
-      if (!a.include_self) add8(acc[j], own[j]);  // the owner's own gradient first, then the hosts in rank order
+      if (own_slot) add8(acc[j], own[j]);  // the owner's own gradient first, then the hosts in rank order
     for (int k = 0; k < n; ++k) {
       const uint4* peer = reinterpret_cast<const uint4*>(a.g_ptrs[host_rank[k]]) + (size_t)host_slot[k] * n_vec;
       uint4 v[kUnroll];

@@ -326,6 +326,10 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
     g.done_R = cfg_.R;
   }
   g.row_scale = extra.row_scale;
+  if (extra.accum != nullptr) {
+    g.accum = extra.accum;
+    g.home_cap = cfg_.home_cap;
+  }
   if (extra.comm != nullptr) {
     g.comm = *extra.comm;
     g.trace = ptr<unsigned long long>("gemm_trace", false);  // optional: phase timestamps of the fused kernels
@@ -507,9 +511,16 @@ void MoeRuntime::dispatch_grads(const void* dout, int num_units, cudaStream_t st
   const CommArgs a = comm_backward(dout);
   check(launch_comm(a, cfg_.num_sms, sp_.status, stream), "dispatch_grads");
 }
+// fp32 accumulation over micro-batches happens in the Wgrad epilogue for the owned slots: the gradient is added from the
+// fp32 accumulators and never takes the detour through the bf16 slot (one write and one read of 2 bytes a weight, and a
+// rounding).  Replica slots keep bf16: their owner adds them (grad_reduce).
+float* MoeRuntime::fused_accum(const char* name) const { return cfg_.accum_fp32 ? ptr<float>(name, false) : nullptr; }
+
 // No gate: Dgrad2, earlier on this stream, has waited for every gradient row of this rank.
 void MoeRuntime::wgrad2(cudaStream_t stream) {
-  gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream);
+  GemmExtra x;
+  x.accum = fused_accum("acc_gw2");
+  gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream, x);
 }
 void MoeRuntime::swiglu_pass(cudaStream_t stream) {
   SwigluBwdArgs a{};
@@ -539,7 +550,9 @@ void MoeRuntime::dgrad2_fused(const void* dout, int num_units, cudaStream_t stre
   swiglu_pass(stream);
 }
 void MoeRuntime::wgrad1(cudaStream_t stream) {
-  gemm(kWgrad, tm_dh_mn_, tm_x_mn_, cfg_.H, 0, 2 * cfg_.F, ptr<void>("gw1"), nullptr, nullptr, nullptr, stream);
+  GemmExtra x;
+  x.accum = fused_accum("acc_gw1");
+  gemm(kWgrad, tm_dh_mn_, tm_x_mn_, cfg_.H, 0, 2 * cfg_.F, ptr<void>("gw1"), nullptr, nullptr, nullptr, stream, x);
 }
 void MoeRuntime::dgrad1(cudaStream_t stream) {
   GemmExtra x;
@@ -556,8 +569,10 @@ void MoeRuntime::reduce_dtokens(void* dtokens, float* dprob, int num_tokens, cud
 void MoeRuntime::reduce_weight_grads(cudaStream_t stream) {
   void* acc1 = ptr<void>("acc_gw1", false);
   void* acc2 = ptr<void>("acc_gw2", false);
-  if (cfg_.R <= 1 && acc1 == nullptr) return;
+  const bool own_done = fused_accum("acc_gw1") != nullptr;  // Wgrad has added the owned slots' own gradients already
+  if (cfg_.R <= 1 && (acc1 == nullptr || own_done)) return;
   GradReduceArgs a{};
+  a.skip_self = own_done;
   a.accum_fp32 = cfg_.accum_fp32;
   a.slot_of = tables_.slot_of;
   a.main_rank = sp_.main_rank;

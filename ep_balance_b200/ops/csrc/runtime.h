@@ -121,6 +121,7 @@ class MoeRuntime {
     int done_slot = 0;   // > 0: signal every peer on this slot when the launch is complete
     const float* row_scale = nullptr;
     const CommArgs* comm = nullptr;
+    float* accum = nullptr;  // Wgrad: fp32 accumulation buffer of the owned slots
     bool narrow = false; // few rows per expert: weights on the M side (narrow_gemm.h)
   };
   void gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int N, int K, int M_out, void* out0, void* out1,
@@ -133,6 +134,7 @@ class MoeRuntime {
   CommArgs comm_forward(const void* tokens, const float* topk_prob, bool pad, bool pull) const;
   CommArgs comm_backward(const void* dout) const;
   void swiglu_pass(cudaStream_t stream);
+  float* fused_accum(const char* name) const;
   bool use_narrow(int num_units) const;
   bool peers() const { return cfg_.multi_rank_sync && cfg_.R > 1; }
   UnitReduceWait reduce_wait(int slot) const;
