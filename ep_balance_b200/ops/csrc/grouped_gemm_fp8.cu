@@ -762,23 +762,30 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16*
     for (int kb = kblocks; kb < kgroups * 4; ++kb) chunk_row[(size_t)(kb >> 2) * 512 + chunk_byte(warp & 127, kb)] = 127;
 }
 
-// One warp per routed unit.  A 128-wide block is held by 16 lanes (8 values each); the block maximum is a
-// 4-step shuffle inside the half-warp.  Stores go to the destination rank's buffers (peer memory).
-__global__ void __launch_bounds__(256) dispatch_fp8_kernel(DispatchFp8Args a) {
+// One warp per token and 1024-wide piece of its row: the piece is read and quantised ONCE and stored to all topk destinations
+// (peer memory).  A 128-wide block is held by 16 lanes (8 values each); the block maximum is a 4-step shuffle inside the
+// half-warp.  The four loads of a piece are issued together.  Bound by the topk stores: 4096 tokens x 8 x 7168 in 113 us
+// (2.1 TB/s) with one warp per routed unit, which read and quantised every token eight times, 75 now; 64 tokens 12.7 -> 5.2.
+constexpr int kDispatchVecs = 4;  // 16-byte vectors of a row that a lane holds
+__global__ void __launch_bounds__(256) dispatch_fp8_kernel(DispatchFp8Args a, int num_tokens, int pieces) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const int u = blockIdx.x * wpb + warp;
-  if (u >= a.num_units) return;
-  const int dst = a.unit_dst[u], row = a.unit_row[u];
-  if (dst < 0 || row >= a.row_capacity) return;
+  const long long item = (long long)blockIdx.x * wpb + warp;
+  const int t = (int)(item / pieces), piece = (int)(item - (long long)t * pieces);
+  if (t >= num_tokens) return;
   const int vec_per_row = a.H / 8;
   const int kgroups = (a.H / 128 + 3) / 4;
-  const uint4* src = reinterpret_cast<const uint4*>(a.rows) + (size_t)(u / a.topk) * vec_per_row;
-  uint8_t* qrow = a.xq_ptrs[dst] + (size_t)row * a.H;
-  uint8_t* chunk_row = a.sfx_ptrs[dst] + (size_t)(row >> 7) * kgroups * 512;
-  for (int v = lane; v < vec_per_row + (32 - vec_per_row % 32) % 32; v += 32) {
-    const bool have = v < vec_per_row;
-    const uint4 raw = have ? src[v] : make_uint4(0, 0, 0, 0);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const uint4* src = reinterpret_cast<const uint4*>(a.rows) + (size_t)t * vec_per_row;
+  uint4 raw[kDispatchVecs];
+#pragma unroll
+  for (int i = 0; i < kDispatchVecs; ++i) {
+    const int v = (piece * kDispatchVecs + i) * 32 + lane;
+    raw[i] = v < vec_per_row ? src[v] : make_uint4(0, 0, 0, 0);
+  }
+  uint2 q[kDispatchVecs];
+  uint8_t exps[kDispatchVecs];
+#pragma unroll
+  for (int i = 0; i < kDispatchVecs; ++i) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[i]);
     float f[8];
     float amax = 0.f;
 #pragma unroll
@@ -790,7 +797,6 @@ __global__ void __launch_bounds__(256) dispatch_fp8_kernel(DispatchFp8Args a) {
     }
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (!have) continue;
     const int e = scale_exponent(amax);
     const float inv = exp2_int(-e);
     uint32_t out[2];
@@ -800,11 +806,35 @@ __global__ void __launch_bounds__(256) dispatch_fp8_kernel(DispatchFp8Args a) {
       const unsigned hi = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
       out[j] = (lo & 0xffffu) | (hi << 16);
     }
-    *reinterpret_cast<uint2*>(qrow + (size_t)v * 8) = make_uint2(out[0], out[1]);
-    const int kb = v >> 4;
-    if ((lane & 15) == 0) chunk_row[(size_t)(kb >> 2) * 512 + chunk_byte(row & 127, kb)] = (uint8_t)(e + 127);
+    q[i] = make_uint2(out[0], out[1]);
+    exps[i] = (uint8_t)(e + 127);
   }
-  if (lane == 0 && a.meta_ptrs != nullptr) a.meta_ptrs[dst][row] = make_int2(a.me, a.unit_pos[u]);
+  for (int k0 = 0; k0 < a.topk; k0 += 32) {
+    // lane k holds the destination of the token's unit k0 + k
+    int my_dst = -1, my_row = 0;
+    if (k0 + lane < a.topk) {
+      const int u = t * a.topk + k0 + lane;
+      my_dst = a.unit_dst[u];
+      my_row = a.unit_row[u];
+      if (my_row >= a.row_capacity) my_dst = -1;
+      if (piece == 0 && my_dst >= 0 && a.meta_ptrs != nullptr) a.meta_ptrs[my_dst][my_row] = make_int2(a.me, a.unit_pos[u]);
+    }
+    const int n = min(32, a.topk - k0);
+    for (int k = 0; k < n; ++k) {
+      const int dst = __shfl_sync(0xffffffffu, my_dst, k), row = __shfl_sync(0xffffffffu, my_row, k);
+      if (dst < 0) continue;
+      uint8_t* qrow = a.xq_ptrs[dst] + (size_t)row * a.H;
+      uint8_t* chunk_row = a.sfx_ptrs[dst] + (size_t)(row >> 7) * kgroups * 512;
+#pragma unroll
+      for (int i = 0; i < kDispatchVecs; ++i) {
+        const int v = (piece * kDispatchVecs + i) * 32 + lane;
+        if (v >= vec_per_row) continue;
+        *reinterpret_cast<uint2*>(qrow + (size_t)v * 8) = q[i];
+        const int kb = v >> 4;
+        if ((lane & 15) == 0) chunk_row[(size_t)(kb >> 2) * 512 + chunk_byte(row & 127, kb)] = exps[i];
+      }
+    }
+  }
 }
 
 // SwiGLU + quantisation in one pass: h [rows, 2F] (gate columns, then up columns) ->
@@ -814,37 +844,56 @@ __global__ void __launch_bounds__(256) swiglu_quantize_kernel(const __nv_bfloat1
                                                               int rows, int F, RowGroups groups) {
   const int warp = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (warp >= rows || !row_is_real(groups, warp, lane)) return;
-  const int kblocks = F / 128, kgroups = (kblocks + 3) / 4;
-  const __nv_bfloat16* hr = h + (size_t)warp * 2 * F;
+  // A half-warp holds a 128-wide block (8 values per lane), a pass of the loop kUnroll x 256 columns: all its loads are
+  // issued before the first is used (512 rows of 2048: 16 us with 8-byte loads and one block per pass, 8.8 now; 32768 rows
+  // 85 -> 75).
+  const int kblocks = F / 128, kgroups = (kblocks + 3) / 4, vec_per_row = F / 8;
+  const uint4* gr = reinterpret_cast<const uint4*>(h + (size_t)warp * 2 * F);
+  const uint4* ur = gr + vec_per_row;
   uint8_t* qr = q + (size_t)warp * F;
   uint8_t* chunk_row = sfa + (size_t)(warp >> 7) * kgroups * 512;
-  for (int kb = 0; kb < kblocks; ++kb) {
-    const uint2 graw = *reinterpret_cast<const uint2*>(hr + kb * 128 + lane * 4);
-    const uint2 uraw = *reinterpret_cast<const uint2*>(hr + F + kb * 128 + lane * 4);
-    const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&graw);
-    const __nv_bfloat162* uh = reinterpret_cast<const __nv_bfloat162*>(&uraw);
-    float v[4];
+  constexpr int kUnroll = 4;
+  for (int v0 = 0; v0 < vec_per_row; v0 += 32 * kUnroll) {
+    uint4 graw[kUnroll], uraw[kUnroll];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const float2 g = __bfloat1622float2(gh[j]), u = __bfloat1622float2(uh[j]);
-      v[2 * j] = g.x * __fdividef(1.f, 1.f + __expf(-g.x)) * u.x;
-      v[2 * j + 1] = g.y * __fdividef(1.f, 1.f + __expf(-g.y)) * u.y;
+    for (int i = 0; i < kUnroll; ++i) {
+      const int v = v0 + i * 32 + lane;
+      graw[i] = v < vec_per_row ? gr[v] : make_uint4(0, 0, 0, 0);
+      uraw[i] = v < vec_per_row ? ur[v] : make_uint4(0, 0, 0, 0);
     }
-    if (act != nullptr) {
-      uint2 o;
-      o.x = pack_bf16(v[0], v[1]);
-      o.y = pack_bf16(v[2], v[3]);
-      *reinterpret_cast<uint2*>(act + (size_t)warp * F + kb * 128 + lane * 4) = o;
-    }
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const int e = scale_exponent(amax);
-    const float inv = exp2_int(-e);
-    const unsigned lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] * inv, v[1] * inv), __NV_SATFINITE, __NV_E4M3);
-    const unsigned hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
-    *reinterpret_cast<uint32_t*>(qr + kb * 128 + lane * 4) = (lo & 0xffffu) | (hi << 16);
-    if (lane == 0) chunk_row[(size_t)(kb >> 2) * 512 + chunk_byte(warp & 127, kb)] = (uint8_t)(e + 127);
+    for (int i = 0; i < kUnroll; ++i) {
+      const int v = v0 + i * 32 + lane;
+      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&graw[i]);
+      const __nv_bfloat162* uh = reinterpret_cast<const __nv_bfloat162*>(&uraw[i]);
+      float f[8];
+      float amax = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 g = __bfloat1622float2(gh[j]), u = __bfloat1622float2(uh[j]);
+        f[2 * j] = g.x * __fdividef(1.f, 1.f + __expf(-g.x)) * u.x;
+        f[2 * j + 1] = g.y * __fdividef(1.f, 1.f + __expf(-g.y)) * u.y;
+        amax = fmaxf(amax, fmaxf(fabsf(f[2 * j]), fabsf(f[2 * j + 1])));
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      if (v >= vec_per_row) continue;
+      if (act != nullptr)
+        *reinterpret_cast<uint4*>(act + (size_t)warp * F + (size_t)v * 8) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+      const int e = scale_exponent(amax);
+      const float inv = exp2_int(-e);
+      uint32_t out[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const unsigned lo = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j] * inv, f[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+        const unsigned hi = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+        out[j] = (lo & 0xffffu) | (hi << 16);
+      }
+      *reinterpret_cast<uint2*>(qr + (size_t)v * 8) = make_uint2(out[0], out[1]);
+      const int kb = v >> 4;
+      if ((lane & 15) == 0) chunk_row[(size_t)(kb >> 2) * 512 + chunk_byte(warp & 127, kb)] = (uint8_t)(e + 127);
+    }
   }
 }
 
@@ -1015,8 +1064,10 @@ cudaError_t launch_quantize_rows(const void* x, uint8_t* q, uint8_t* sfa, int ro
 cudaError_t launch_dispatch_fp8(const DispatchFp8Args& a, cudaStream_t stream) {
   if (a.H % 128 != 0) return cudaErrorInvalidValue;
   if (a.num_units <= 0) return cudaSuccess;
-  const int wpb = 8;
-  dispatch_fp8_kernel<<<(a.num_units + wpb - 1) / wpb, wpb * 32, 0, stream>>>(a);
+  if (a.topk < 1 || a.num_units % a.topk != 0) return cudaErrorInvalidValue;
+  const int wpb = 8, tokens = a.num_units / a.topk, pieces = ceil_div(a.H, kDispatchVecs * 256);
+  const long long items = (long long)tokens * pieces;
+  dispatch_fp8_kernel<<<(unsigned)((items + wpb - 1) / wpb), wpb * 32, 0, stream>>>(a, tokens, pieces);
   return cudaGetLastError();
 }
 
