@@ -1086,6 +1086,94 @@ __global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables
   if (p.trace != nullptr && threadIdx.x == 0) p.trace[6] = (int64_t)globaltimer_ns();
 }
 
+// One rank has nothing to decide: every expert stays where it lives, and the outputs are the load row, its sum and the
+// tables.  One CTA, one thread per expert; two global round trips (signal, load row) and a block scan, where the general
+// kernel walks its phases and builds the tables 32 experts at a time: 16 us for 8 experts and 28 for 128, here 5.
+__global__ void __launch_bounds__(1024) single_rank_kernel(SolverParams p, RankTables t) {
+  __shared__ int ready, warp_rows[kWarp], warp_groups[kWarp], warp_load[kWarp];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  if (tid == 0) {
+    ready = 1;
+    if (p.omega_signal != nullptr && !wait_ge<true>(p.omega_signal, *p.omega_epoch, kWaitBudgetNs)) {
+      set_status(p.status, kStatusSignalTimeout, 10);
+      ready = 0;
+    } else if (p.dom[0] != 0) {
+      set_status(p.status, kStatusBadArgument, 13, 0);
+      ready = 0;
+    }
+  }
+  __syncthreads();
+  if (!ready) return;
+  int rows = 0, groups = 0, load = 0;  // running totals before this chunk of experts, the same in every thread
+  for (int e0 = 0; e0 < p.E; e0 += blockDim.x) {
+    const int e = e0 + tid;
+    const bool hosted = e < p.E && p.main_rank[e] == 0;
+    const int need = e < p.E ? __ldcg(p.omega + e) : 0;
+    const int size = hosted && need > 0 ? need : 0;
+    const int padded = t.me >= 0 ? round_up(size, t.row_align) : 0;
+    int incl = padded, sum = size;
+    const unsigned m = __ballot_sync(kFull, hosted);
+    for (int off = 1; off < kWarp; off <<= 1) {
+      const int o = __shfl_up_sync(kFull, incl, off);
+      if (lane >= off) incl += o;
+    }
+    for (int off = kWarp / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
+    if (lane == kWarp - 1) {
+      warp_rows[warp] = incl;
+      warp_groups[warp] = __popc(m);
+      warp_load[warp] = sum;
+    }
+    __syncthreads();
+    int row = rows + incl - padded, group = groups + __popc(m & ((1u << lane) - 1u));
+    for (int w = 0; w < nwarps; ++w) {
+      if (w < warp) {
+        row += warp_rows[w];
+        group += warp_groups[w];
+      }
+      rows += warp_rows[w];
+      groups += warp_groups[w];
+      load += warp_load[w];
+    }
+    __syncthreads();
+    if (e >= p.E) continue;
+    p.x[e] = hosted ? 1 : 0;
+    p.q[e] = size;
+    p.erl[e] = size;
+    if (t.me < 0) continue;
+    const int wslot = hosted ? (t.home_index != nullptr ? t.home_index[e] : group) : -1;
+    if (t.slot_of) t.slot_of[e] = wslot;
+    if (t.row_base) t.row_base[e] = hosted ? row : -1;
+    if (t.send_off != nullptr) t.send_off[e] = 0;
+    if (hosted && group < t.n_slot) {
+      t.group_expert[group] = e;
+      t.group_wslot[group] = wslot;
+      t.group_off[group] = row;
+      t.group_rows[group] = size;
+    }
+  }
+  if (t.me >= 0) {
+    for (int g = groups + tid; g < t.n_slot; g += blockDim.x) {
+      t.group_expert[g] = -1;
+      t.group_wslot[g] = 0;
+      t.group_off[g] = rows;
+      t.group_rows[g] = 0;
+    }
+    if (tid == 0) {
+      t.group_off[t.n_slot] = rows;
+      t.totals[0] = rows;
+      t.totals[1] = groups < t.n_slot ? groups : t.n_slot;
+      if (t.tiles_of != nullptr) t.tiles_of[0] = (t.row_capacity > 0 && rows > t.row_capacity ? t.row_capacity : rows) / t.row_align;
+      if (t.row_capacity > 0 && rows > t.row_capacity) set_status(p.status, kStatusRowOverflow, 30, rows);
+    }
+  }
+  if (tid == 0) {
+    p.rank_load[0] = load;
+    p.slot_used[0] = groups;
+    p.stuck[0] = p.iters > 0 && load > 0 ? 1 : 0;  // the repair loop looks at the busiest rank once and finds no target
+    p.theta[0] = load;
+  }
+}
+
 __global__ void __launch_bounds__(1024) tables_kernel(SolverParams p, RankTables tables) {
   build_tables(p, tables, tables.me);
 }
@@ -1113,6 +1201,12 @@ cudaError_t launch_solver(const SolverParams& p, const RankTables& tables, cudaS
   if (err != cudaSuccess) return err;
   err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (err != cudaSuccess) return err;
+  const int threads = pow2_threads(p.R, p.E);
+  // (probe mode reports control words and a trace wants phases: both keep the general kernel)
+  if (p.R == 1 && p.D == 1 && !p.probe && p.trace == nullptr) {
+    single_rank_kernel<<<1, threads, 0, stream>>>(p, tables);
+    return cudaGetLastError();
+  }
   SolverParams pc = p;
   const size_t base = solver_base_smem(p.R, p.E);
   pc.cache_stage2 = base + solver_cache_smem(p.R, p.E) <= kCacheBudget ? 1 : 0;
@@ -1130,7 +1224,6 @@ cudaError_t launch_solver(const SolverParams& p, const RankTables& tables, cudaS
   }
   int grid = p.D < sms ? p.D : sms;
   if (grid < 1) grid = 1;
-  const int threads = pow2_threads(p.R, p.E);
   RankTables tc = tables;
   void* args[] = {&pc, &tc};
   if (grid > 1) return cudaLaunchCooperativeKernel((void*)solver_kernel, dim3(grid), dim3(threads), args, smem, stream);
