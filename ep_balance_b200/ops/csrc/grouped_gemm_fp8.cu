@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include "block_scale.cuh"
 #include "common.cuh"
 
 namespace epb {
@@ -100,19 +101,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-// 512-byte scale chunk (32 rows x 16 B) -> 4 TMEM columns, replicated to the four 32-lane groups
-__device__ __forceinline__ void tmem_cp_sf(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-__device__ __forceinline__ void umma_fp8_scaled(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -137,19 +125,6 @@ __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-__device__ __forceinline__ uint64_t make_desc_sf(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(128 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-// Instruction descriptor of the block-scaled kind: e4m3 x e4m3, both K-major, UE8M0 scales;
-// sf ids select which of the four scale bytes of a TMEM word this MMA uses.
-__device__ __forceinline__ uint32_t make_idesc_scaled(int n, int m, uint32_t a_sf_id, uint32_t b_sf_id) {
-  return (b_sf_id << 4) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((uint32_t)(m >> 4) << 24) | (a_sf_id << 29);
-}
-
 struct Tile {
   int g, mt, nt, rows, row0, wslot;
 };
@@ -709,17 +684,6 @@ constexpr size_t kSmemBytes = STAGES * TILE_BYTES + STAGES * SF_BYTES + 1024 + k
 static_assert(kSmemBytes <= 232448, "shared memory budget exceeded");
 
 // ---------------------------------------------------------------- quantisers
-// Power-of-two scale of a block with absolute maximum `amax`: the smallest 2^e with amax / 2^e <= 448.
-__device__ __forceinline__ int scale_exponent(float amax) {
-  if (!(amax > 0.f)) return -126;
-  int ex;
-  const float m = frexpf(amax * (1.f / 448.f), &ex);  // amax/448 = m * 2^ex, m in [0.5, 1)
-  int e = (m == 0.5f) ? ex - 1 : ex;
-  return max(-126, min(126, e));
-}
-__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }  // e in [-126, 127]
-__device__ __forceinline__ int chunk_byte(int r_in_128, int kb) { return (r_in_128 & 31) * 16 + (r_in_128 >> 5) * 4 + (kb & 3); }
-
 // Is `row` inside one of the groups?  The whole warp calls this with the same row.
 __device__ __forceinline__ bool row_is_real(const RowGroups& g, int row, int lane) {
   if (g.group_off == nullptr) return true;
@@ -765,7 +729,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16*
 // One warp per token and 1024-wide piece of its row: the piece is read and quantised ONCE and stored to all topk destinations
 // (peer memory).  A 128-wide block is held by 16 lanes (8 values each); the block maximum is a 4-step shuffle inside the
 // half-warp.  The four loads of a piece are issued together.  Bound by the topk stores: 4096 tokens x 8 x 7168 in 113 us
-// (2.1 TB/s) with one warp per routed unit, which read and quantised every token eight times, 75 now; 64 tokens 12.7 -> 5.2.
+// (2.1 TB/s) with one warp per routed unit, which read and quantised every token eight times, 50 now; 64 tokens 12.7 -> 5.2.
 constexpr int kDispatchVecs = 4;  // 16-byte vectors of a row that a lane holds
 __global__ void __launch_bounds__(256) dispatch_fp8_kernel(DispatchFp8Args a, int num_tokens, int pieces) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -968,12 +932,12 @@ EncodeTiledFn encode_fn() {
 
 }  // namespace
 
-bool make_tmap_fp8_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols) {
+bool make_tmap_fp8_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols};
-  cuuint32_t box[2] = {128, 128};
+  cuuint32_t box[2] = {128, box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -41,7 +41,7 @@ struct Fp8GemmArgs {
 };
 
 // Tensor maps over the e4m3 bytes: A [rows, K], B [slots, N, K]; boxes of 128 x 128 bytes, 128-byte swizzle.
-bool make_tmap_fp8_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols);
+bool make_tmap_fp8_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows = 128);
 bool make_tmap_fp8_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols,
                       uint32_t box_rows = 128);
 // Scale chunks as a [chunks, 128] int32 tensor (one 512-byte chunk per row, no swizzle).

@@ -10,7 +10,7 @@
 // There is no stand-alone barrier on the critical path: consumers of transferred rows wait per M-tile
 // on arrival counters that the senders advance, consumers of combined rows on one signal per peer.
 // Inference with fp8 experts: publish -> solve -> route -> dispatch fused with the 1 x 128 quantisation ->
-// fp8 replica pull -> [barrier] -> fp8 gemm1 -> SwiGLU + quantise -> fp8 gemm2 (scattered) -> [barrier] -> reduce_out.
+// fp8 replica pull -> [barrier] -> fp8 gemm1 -> SwiGLU + quantise (in gemm1's epilogue for few rows per expert) -> fp8 gemm2 (scattered) -> [barrier] -> reduce_out.
 // This is the schedule the reference drives from Python over NCCL on three streams
 // (eplb_manager.py:710-886, 905-1167, manual_block.py:127-367, overlap.py:257-328), restated as
 // device-side kernels that overlap transfer and compute tile by tile.
@@ -150,7 +150,11 @@ MoeRuntime::MoeRuntime(const LayerConfig& cfg, const std::map<std::string, uint6
     // weight boxes: 128 rows for the single-CTA kernel; the CTA-pair kernel stages half a tile's columns per CTA
     const bool pair = c.gemm_ctas == 2;
     const uint32_t box1 = pair ? ((2 * F) % 256 == 0 ? 128 : 64) : 128, box2 = pair ? (H % 256 == 0 ? 128 : 64) : 128;
-    if (!make_tmap_fp8_2d(&tm_xq_, ptr<void>("xq"), T, H) || !make_tmap_fp8_2d(&tm_actq_, ptr<void>("actq"), T, F) ||
+    w1q_box_ = (int)box1;
+    w2q_box_ = (int)box2;
+    if (!make_tmap_fp8_2d(&tm_xq_n_, ptr<void>("xq"), T, H, kNarrowFp8BoxRows) ||
+        !make_tmap_fp8_2d(&tm_actq_n_, ptr<void>("actq"), T, F, kNarrowFp8BoxRows) ||
+        !make_tmap_fp8_2d(&tm_xq_, ptr<void>("xq"), T, H) || !make_tmap_fp8_2d(&tm_actq_, ptr<void>("actq"), T, F) ||
         !make_tmap_fp8_3d(&tm_w1q_, ptr<void>("w1q"), S, 2 * F, H, box1) ||
         !make_tmap_fp8_3d(&tm_w2q_, ptr<void>("w2q"), S, H, F, box2))
       throw std::runtime_error("MoeRuntime: cuTensorMapEncodeTiled (fp8) failed");
@@ -445,9 +449,7 @@ void MoeRuntime::gemm_fp8(const CUtensorMap& a, const CUtensorMap& b, const CUte
   g.out_ptrs = out_ptrs;
   g.meta = meta;
   g.status = sp_.status;
-  // the single-CTA kernel can share the pair kernel's weight map only when that map has 128-row boxes
-  const bool pair = cfg_.gemm_ctas == 2 && (fp8_pair_ || N % 256 != 0);
-  if (pair)
+  if (cfg_.gemm_ctas == 2)
     check(launch_grouped_gemm_fp8_pair(a, b, sfa_map, sfb_map, g, cfg_.num_sms, stream), "grouped_gemm_fp8_pair");
   else
     check(launch_grouped_gemm_fp8(a, b, g, cfg_.num_sms, stream), "grouped_gemm_fp8");
@@ -471,7 +473,34 @@ void MoeRuntime::dispatch_fp8(const void* tokens, int num_units, cudaStream_t st
   check(launch_dispatch_fp8(a, stream), "dispatch_fp8");
 }
 
-void MoeRuntime::gemm1_fp8(cudaStream_t stream) {
+void MoeRuntime::narrow_fp8(const CUtensorMap& w, const CUtensorMap& x, int w_box, int N, int K, const uint8_t* sfa, const uint8_t* sfb,
+                            uint8_t* q_out, uint8_t* sf_out, void* const* out_ptrs, const int2* meta, cudaStream_t stream) {
+  NarrowFp8Args a{};
+  a.g.group_off = tables_.group_off;
+  a.g.group_rows = tables_.group_rows;
+  a.g.group_wslot = tables_.group_wslot;
+  a.g.totals = tables_.totals;
+  a.g.n_groups_cap = cfg_.w_slots;
+  a.g.row_capacity = cfg_.row_capacity;
+  a.g.N = N;
+  a.g.K = K;
+  a.g.sfa = sfa;
+  a.g.sfb = sfb;
+  a.g.out_ptrs = out_ptrs;
+  a.g.meta = meta;
+  a.g.status = sp_.status;
+  a.w_box_rows = w_box;
+  a.q_out = q_out;
+  a.sf_out = sf_out;
+  check(launch_narrow_gemm_fp8(w, x, a, cfg_.num_sms, stream), q_out != nullptr ? "narrow_gemm_fp8+act" : "narrow_gemm_fp8");
+}
+
+void MoeRuntime::gemm1_fp8(cudaStream_t stream, bool narrow) {
+  if (narrow) {
+    narrow_fp8(tm_w1q_, tm_xq_n_, w1q_box_, cfg_.F, cfg_.H, ptr<uint8_t>("sfx"), ptr<uint8_t>("sfb1"), ptr<uint8_t>("actq"),
+               ptr<uint8_t>("sfact"), nullptr, nullptr, stream);
+    return;
+  }
   gemm_fp8(tm_xq_, tm_w1q_, tm_sfx_, tm_sfb1_, 2 * cfg_.F, cfg_.H, ptr<uint8_t>("sfx"), ptr<uint8_t>("sfb1"),
            ptr<void>("hbuf"), nullptr, nullptr, stream);
 }
@@ -481,7 +510,12 @@ void MoeRuntime::act_fp8(cudaStream_t stream) {
                                cfg_.F, &groups, stream),
         "swiglu_quantize");
 }
-void MoeRuntime::gemm2_fp8(cudaStream_t stream) {
+void MoeRuntime::gemm2_fp8(cudaStream_t stream, bool narrow) {
+  if (narrow) {
+    narrow_fp8(tm_w2q_, tm_actq_n_, w2q_box_, cfg_.H, cfg_.F, ptr<uint8_t>("sfact"), ptr<uint8_t>("sfb2"), nullptr, nullptr,
+               ptr<void* const>("ybuf_ptrs"), ptr<const int2>("meta"), stream);
+    return;
+  }
   gemm_fp8(tm_actq_, tm_w2q_, tm_sfact_, tm_sfb2_, cfg_.H, cfg_.F, ptr<uint8_t>("sfact"), ptr<uint8_t>("sfb2"), nullptr,
            ptr<void* const>("ybuf_ptrs"), ptr<const int2>("meta"), stream);
 }
@@ -490,17 +524,17 @@ void MoeRuntime::forward_fp8(const void* tokens, const int64_t* topk_idx, const 
                              int num_tokens, cudaStream_t stream) {
   if (!fp8_) throw std::runtime_error("MoeRuntime: fp8 regions were not provided");
   const int U = num_tokens * cfg_.topk;
-  // about U rows reach this rank; with few rows per expert the 256-row tiles of the pair kernel are mostly padding
-  fp8_pair_ = U >= 192 * cfg_.w_slots;
+  // about U rows reach this rank; with few rows per expert the weights' bytes bound the launch (narrow_gemm_fp8.h)
+  const bool narrow = U < kNarrowFp8RowsPerSlot * cfg_.w_slots;
   publish(topk_idx, U, stream);
   solve(stream);
   route(topk_idx, U, stream);
   dispatch_fp8(tokens, U, stream);  // rows cross NVLink as e4m3 + scales; padding rows stay stale (never stored)
   pull_weights_fp8(stream);
   barrier(1, stream);
-  gemm1_fp8(stream);
-  act_fp8(stream);
-  gemm2_fp8(stream);
+  gemm1_fp8(stream, narrow);
+  if (!narrow) act_fp8(stream);
+  gemm2_fp8(stream, narrow);
   barrier(2, stream);
   reduce_out(out, num_tokens, stream, false, topk_prob);
 }

@@ -15,6 +15,7 @@
 #include "grouped_gemm.h"
 #include "grouped_gemm_fp8.h"
 #include "narrow_gemm.h"
+#include "narrow_gemm_fp8.h"
 #include "route.h"
 #include "solver.h"
 
@@ -84,9 +85,9 @@ class MoeRuntime {
   void quantize_own_weights(cudaStream_t stream);   // bf16 home slots -> e4m3 + 128 x 128 scales
   void pull_weights_fp8(cudaStream_t stream);       // replicas pull e4m3 bytes and scale chunks: half the bytes of bf16
   void dispatch_fp8(const void* tokens, int num_units, cudaStream_t stream);  // dispatch fused with the 1 x 128 quantisation
-  void gemm1_fp8(cudaStream_t stream);              // h = x W1^T on the quantised rows
+  void gemm1_fp8(cudaStream_t stream, bool narrow = false);  // h = x W1^T on the quantised rows; narrow: up to the quantised activation
   void act_fp8(cudaStream_t stream);                // SwiGLU + quantise
-  void gemm2_fp8(cudaStream_t stream);              // y = act W2^T, rows scattered to their sources
+  void gemm2_fp8(cudaStream_t stream, bool narrow = false);  // y = act W2^T, rows scattered to their sources
   void forward_fp8(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out, int num_tokens,
                    cudaStream_t stream);
 
@@ -162,9 +163,12 @@ class MoeRuntime {
   CUtensorMap tm_x_n_, tm_act_n_;                                // token rows as the narrow kernel's N operand
   CUtensorMap tm_dy_mn_, tm_act_mn_, tm_dh_mn_, tm_x_mn_;        // Wgrad operands (MN-major)
   bool fp8_ = false;
-  bool fp8_pair_ = true;   // CTA-pair fp8 kernel (256-row tiles); forward_fp8 falls back to 128-row tiles for tiny batches
   CUtensorMap tm_xq_, tm_actq_, tm_w1q_, tm_w2q_;                // e4m3 operands
+  CUtensorMap tm_xq_n_, tm_actq_n_;                              // token rows as the narrow kernel's N operand
+  int w1q_box_ = 128, w2q_box_ = 128;                            // rows of the weight maps' boxes
   CUtensorMap tm_sfx_, tm_sfact_, tm_sfb1_, tm_sfb2_;            // scale chunks (CTA-pair fp8 kernel)
+  void narrow_fp8(const CUtensorMap& w, const CUtensorMap& x, int w_box, int N, int K, const uint8_t* sfa, const uint8_t* sfb,
+                  uint8_t* q_out, uint8_t* sf_out, void* const* out_ptrs, const int2* meta, cudaStream_t stream);
   void gemm_fp8(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& sfa_map, const CUtensorMap& sfb_map, int N,
                 int K, const uint8_t* sfa, const uint8_t* sfb, void* out, void* const* out_ptrs, const int2* meta,
                 cudaStream_t stream);
