@@ -38,6 +38,10 @@ struct Fp8GemmArgs {
   void* const* out_ptrs;       // R peer buffers [units, N]: row r goes to out_ptrs[meta[r].x] row meta[r].y
   const int2* meta;
   int* status;
+  // CTA-pair kernel only, both or none: SwiGLU + 1 x 128 quantisation in the epilogue.  N is then F, the weights hold F gate
+  // rows and F up rows, and nothing else is stored.
+  uint8_t* q_out;              // e4m3 [row_capacity, N]
+  uint8_t* sf_out;             // its scale chunks
 };
 
 // Tensor maps over the e4m3 bytes: A [rows, K], B [slots, N, K]; boxes of 128 x 128 bytes, 128-byte swizzle.

@@ -10,7 +10,7 @@
 // There is no stand-alone barrier on the critical path: consumers of transferred rows wait per M-tile
 // on arrival counters that the senders advance, consumers of combined rows on one signal per peer.
 // Inference with fp8 experts: publish -> solve -> route -> dispatch fused with the 1 x 128 quantisation ->
-// fp8 replica pull -> [barrier] -> fp8 gemm1 -> SwiGLU + quantise (in gemm1's epilogue for few rows per expert) -> fp8 gemm2 (scattered) -> [barrier] -> reduce_out.
+// fp8 replica pull -> [barrier] -> fp8 gemm1 -> SwiGLU + quantise (in gemm1's epilogue, except for single-CTA tiles) -> fp8 gemm2 (scattered) -> [barrier] -> reduce_out.
 // This is the schedule the reference drives from Python over NCCL on three streams
 // (eplb_manager.py:710-886, 905-1167, manual_block.py:127-367, overlap.py:257-328), restated as
 // device-side kernels that overlap transfer and compute tile by tile.
@@ -433,8 +433,10 @@ void MoeRuntime::pull_weights_fp8(cudaStream_t stream) {
 
 void MoeRuntime::gemm_fp8(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& sfa_map,
                           const CUtensorMap& sfb_map, int N, int K, const uint8_t* sfa, const uint8_t* sfb, void* out,
-                          void* const* out_ptrs, const int2* meta, cudaStream_t stream) {
+                          void* const* out_ptrs, const int2* meta, cudaStream_t stream, uint8_t* q_out, uint8_t* sf_out) {
   Fp8GemmArgs g{};
+  g.q_out = q_out;
+  g.sf_out = sf_out;
   g.group_off = tables_.group_off;
   g.group_rows = tables_.group_rows;
   g.group_wslot = tables_.group_wslot;
@@ -450,7 +452,8 @@ void MoeRuntime::gemm_fp8(const CUtensorMap& a, const CUtensorMap& b, const CUte
   g.meta = meta;
   g.status = sp_.status;
   if (cfg_.gemm_ctas == 2)
-    check(launch_grouped_gemm_fp8_pair(a, b, sfa_map, sfb_map, g, cfg_.num_sms, stream), "grouped_gemm_fp8_pair");
+    check(launch_grouped_gemm_fp8_pair(a, b, sfa_map, sfb_map, g, cfg_.num_sms, stream),
+          q_out != nullptr ? "grouped_gemm_fp8_pair+act" : "grouped_gemm_fp8_pair");
   else
     check(launch_grouped_gemm_fp8(a, b, g, cfg_.num_sms, stream), "grouped_gemm_fp8");
 }
@@ -495,10 +498,15 @@ void MoeRuntime::narrow_fp8(const CUtensorMap& w, const CUtensorMap& x, int w_bo
   check(launch_narrow_gemm_fp8(w, x, a, cfg_.num_sms, stream), q_out != nullptr ? "narrow_gemm_fp8+act" : "narrow_gemm_fp8");
 }
 
-void MoeRuntime::gemm1_fp8(cudaStream_t stream, bool narrow) {
+void MoeRuntime::gemm1_fp8(cudaStream_t stream, bool narrow, bool act) {
   if (narrow) {
     narrow_fp8(tm_w1q_, tm_xq_n_, w1q_box_, cfg_.F, cfg_.H, ptr<uint8_t>("sfx"), ptr<uint8_t>("sfb1"), ptr<uint8_t>("actq"),
                ptr<uint8_t>("sfact"), nullptr, nullptr, stream);
+    return;
+  }
+  if (act) {
+    gemm_fp8(tm_xq_, tm_w1q_, tm_sfx_, tm_sfb1_, cfg_.F, cfg_.H, ptr<uint8_t>("sfx"), ptr<uint8_t>("sfb1"), nullptr, nullptr, nullptr,
+             stream, ptr<uint8_t>("actq"), ptr<uint8_t>("sfact"));
     return;
   }
   gemm_fp8(tm_xq_, tm_w1q_, tm_sfx_, tm_sfb1_, 2 * cfg_.F, cfg_.H, ptr<uint8_t>("sfx"), ptr<uint8_t>("sfb1"),
@@ -532,8 +540,9 @@ void MoeRuntime::forward_fp8(const void* tokens, const int64_t* topk_idx, const 
   dispatch_fp8(tokens, U, stream);  // rows cross NVLink as e4m3 + scales; padding rows stay stale (never stored)
   pull_weights_fp8(stream);
   barrier(1, stream);
-  gemm1_fp8(stream, narrow);
-  if (!narrow) act_fp8(stream);
+  const bool act = !narrow && cfg_.gemm_ctas == 2;  // the single-CTA kernel's 128-column tiles cannot hold a gate and an up block
+  gemm1_fp8(stream, narrow, act);
+  if (!narrow && !act) act_fp8(stream);
   gemm2_fp8(stream, narrow);
   barrier(2, stream);
   reduce_out(out, num_tokens, stream, false, topk_prob);

@@ -85,7 +85,8 @@ class MoeRuntime {
   void quantize_own_weights(cudaStream_t stream);   // bf16 home slots -> e4m3 + 128 x 128 scales
   void pull_weights_fp8(cudaStream_t stream);       // replicas pull e4m3 bytes and scale chunks: half the bytes of bf16
   void dispatch_fp8(const void* tokens, int num_units, cudaStream_t stream);  // dispatch fused with the 1 x 128 quantisation
-  void gemm1_fp8(cudaStream_t stream, bool narrow = false);  // h = x W1^T on the quantised rows; narrow: up to the quantised activation
+  void gemm1_fp8(cudaStream_t stream, bool narrow = false, bool act = false);  // h = x W1^T on the quantised rows;
+                                                    // narrow or act: up to the quantised activation
   void act_fp8(cudaStream_t stream);                // SwiGLU + quantise
   void gemm2_fp8(cudaStream_t stream, bool narrow = false);  // y = act W2^T, rows scattered to their sources
   void forward_fp8(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out, int num_tokens,
@@ -171,7 +172,8 @@ class MoeRuntime {
                   uint8_t* q_out, uint8_t* sf_out, void* const* out_ptrs, const int2* meta, cudaStream_t stream);
   void gemm_fp8(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& sfa_map, const CUtensorMap& sfb_map, int N,
                 int K, const uint8_t* sfa, const uint8_t* sfb, void* out, void* const* out_ptrs, const int2* meta,
-                cudaStream_t stream);
+                cudaStream_t stream,
+                uint8_t* q_out = nullptr, uint8_t* sf_out = nullptr);
 };
 
 }  // namespace epb

@@ -32,5 +32,6 @@ def test_matches_the_wide_kernels(H, F, E, K, N, skew, ctas):
     layer.rt.trace_launches(False)
     layer.check_status()
     assert any("narrow" in n for n in log) == (N * K < 192 * E), log
+    assert ("swiglu_quantize" in log) == (ctas == 1 and N * K >= 192 * E), log  # every other path finishes it in the first GEMM
     # same quantised operands; fp32 sums of K products in another order can move a pre-activation's bf16 rounding
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 1e-2
