@@ -18,6 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..core.config import EPLBConfig
+from ..ops.fused import token_cross_entropy
 from ..parallel.symm import SymmetricHeap
 from ..utils.status import StatusBoard
 from .moe_layer import FusedMoE, MoEConfig, heap_layout
@@ -172,7 +173,7 @@ class GPTMoE(nn.Module):
         logits = self.head(self.norm(x))
         if targets is None:
             return logits
-        loss = F.cross_entropy(logits.float().view(-1, logits.shape[-1]), targets.reshape(-1))
+        loss = token_cross_entropy(logits.view(-1, logits.shape[-1]), targets.reshape(-1))
         for b in self.blocks:  # router balancing pressure, when switched on
             if b.moe.aux_loss is not None:
                 loss = loss + b.moe.aux_loss

@@ -10,6 +10,7 @@
 
 #include "grouped_gemm.h"
 #include "grouped_gemm_fp8.h"
+#include "loss.h"
 #include "narrow_gemm.h"
 #include "onesided.h"
 #include "optim.h"
@@ -388,6 +389,25 @@ void router_topk(torch::Tensor logits, c10::optional<torch::Tensor> bias, int64_
              "launch_router_topk");
 }
 
+// grad (bf16) of the mean cross-entropy: log_prob fp32 [rows, vocab], targets int64 [rows], weight and grad_out fp32 scalars
+void cross_entropy_backward(torch::Tensor log_prob, torch::Tensor targets, torch::Tensor weight, torch::Tensor grad_out,
+                            torch::Tensor grad) {
+  const c10::cuda::CUDAGuard guard(log_prob.device());
+  TORCH_CHECK(log_prob.dim() == 2 && targets.dim() == 1 && targets.size(0) == log_prob.size(0) && weight.numel() == 1 &&
+                  grad_out.numel() == 1 && grad.sizes() == log_prob.sizes(),
+              "cross_entropy_backward: log_prob and grad [rows, vocab], targets [rows], weight [], grad_out []");
+  epb::CrossEntropyGradArgs a{};
+  a.log_prob = dptr<const float>(log_prob, "log_prob", torch::kFloat32);
+  a.targets = dptr<const int64_t>(targets, "targets", torch::kInt64);
+  a.weight = dptr<const float>(weight, "weight", torch::kFloat32);
+  a.grad_out = dptr<const float>(grad_out, "grad_out", torch::kFloat32);
+  a.grad = dptr<void>(grad, "grad", torch::kBFloat16);
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(a.log_prob) | reinterpret_cast<uintptr_t>(a.grad)) % 16 == 0, "16-byte alignment");
+  a.rows = (int)log_prob.size(0);
+  a.vocab = (int)log_prob.size(1);
+  cuda_check(epb::launch_cross_entropy_backward(a, current_stream()), "launch_cross_entropy_backward");
+}
+
 // ---- symmetric heap over CUDA IPC: one cudaMalloc per rank, mapped into every peer process
 py::tuple ipc_alloc(int64_t nbytes) {
   void* p = nullptr;
@@ -435,6 +455,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("symm_barrier", &symm_barrier);
   m.def("grad_reduce", &grad_reduce);
   m.def("router_topk", &router_topk);
+  m.def("cross_entropy_backward", &cross_entropy_backward);
   m.def("quantize_rows", &quantize_rows);
   m.def("quantize_weights", &quantize_weights);
   m.def("grouped_gemm_fp8", &grouped_gemm_fp8);
