@@ -18,7 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..core.config import EPLBConfig
-from ..ops.fused import token_cross_entropy
+from ..ops.fused import split_rotate, token_cross_entropy
 from ..parallel.symm import SymmetricHeap
 from ..utils.status import StatusBoard
 from .moe_layer import FusedMoE, MoEConfig, heap_layout
@@ -78,8 +78,12 @@ class Attention(nn.Module):
 
     def forward(self, x, cos, sin):
         B, S, H = x.shape
-        q, k, v = self.qkv(x).view(B, S, 3, self.heads, self.dim).permute(2, 0, 3, 1, 4)
-        q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
+        qkv = self.qkv(x).view(B, S, 3, self.heads, self.dim)
+        parts = split_rotate(qkv, cos, sin)
+        if parts is None:
+            q, k, v = qkv.permute(2, 0, 3, 1, 4)
+            parts = apply_rope(q, cos, sin), apply_rope(k, cos, sin), v
+        q, k, v = parts
         out = F.scaled_dot_product_attention(q, k, v, is_causal=True)
         return self.proj(out.transpose(1, 2).reshape(B, S, H))
 

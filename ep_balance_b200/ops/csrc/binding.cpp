@@ -14,6 +14,7 @@
 #include "narrow_gemm.h"
 #include "onesided.h"
 #include "optim.h"
+#include "rope.h"
 #include "route.h"
 #include "router.h"
 #include "runtime.h"
@@ -408,6 +409,37 @@ void cross_entropy_backward(torch::Tensor log_prob, torch::Tensor targets, torch
   cuda_check(epb::launch_cross_entropy_backward(a, current_stream()), "launch_cross_entropy_backward");
 }
 
+// packed [B, S, 3, heads, dim] -> q, k [B, heads, S, dim]; backward: the gradients of q, k and v -> that of packed (any strides that
+// are multiples of 8, dense last dimension)
+void rope(torch::Tensor packed, torch::Tensor q, torch::Tensor k, c10::optional<torch::Tensor> v, torch::Tensor cos, torch::Tensor sin, bool backward) {
+  const c10::cuda::CUDAGuard guard(packed.device());
+  TORCH_CHECK(packed.dim() == 5 && packed.size(2) == 3, "rope: packed is [B, S, 3, heads, dim]");
+  epb::RopeArgs a{};
+  a.B = (int)packed.size(0);
+  a.S = (int)packed.size(1);
+  a.heads = (int)packed.size(3);
+  a.dim = (int)packed.size(4);
+  void* p = dptr<void>(packed, "packed", torch::kBFloat16);
+  a.qkv = p;
+  a.cos = dptr<const void>(cos, "cos", torch::kBFloat16);
+  a.sin = dptr<const void>(sin, "sin", torch::kBFloat16);
+  TORCH_CHECK(cos.numel() >= (int64_t)a.S * (a.dim / 2) && sin.numel() >= (int64_t)a.S * (a.dim / 2), "rope: tables shorter than the sequence");
+  TORCH_CHECK(!backward || v.has_value(), "rope: the backward pass needs the gradient of v");
+  const torch::Tensor* parts[3] = {&q, &k, backward ? &*v : nullptr};
+  bool aligned = reinterpret_cast<uintptr_t>(p) % 16 == 0 && reinterpret_cast<uintptr_t>(a.cos) % 16 == 0 && reinterpret_cast<uintptr_t>(a.sin) % 16 == 0;
+  for (int i = 0; i < (backward ? 3 : 2); ++i) {
+    const torch::Tensor& t = *parts[i];
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 4 && t.size(0) == a.B && t.size(1) == a.heads &&
+                    t.size(2) == a.S && t.size(3) == a.dim && (t.stride(3) == 1 || t.numel() == 0),
+                "rope: q, k and v are bf16 [B, heads, S, dim] with a dense last dimension");
+    a.out[i] = t.data_ptr();
+    aligned = aligned && reinterpret_cast<uintptr_t>(a.out[i]) % 16 == 0;
+    for (int j = 0; j < 3; ++j) a.stride[i][j] = t.stride(j);
+  }
+  TORCH_CHECK(aligned, "rope: every tensor must start on a 16-byte boundary");
+  cuda_check(backward ? epb::launch_rope_backward(a, p, current_stream()) : epb::launch_rope(a, current_stream()), "launch_rope");
+}
+
 // ---- symmetric heap over CUDA IPC: one cudaMalloc per rank, mapped into every peer process
 py::tuple ipc_alloc(int64_t nbytes) {
   void* p = nullptr;
@@ -455,6 +487,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("symm_barrier", &symm_barrier);
   m.def("grad_reduce", &grad_reduce);
   m.def("router_topk", &router_topk);
+  m.def("rope", &rope);
   m.def("cross_entropy_backward", &cross_entropy_backward);
   m.def("quantize_rows", &quantize_rows);
   m.def("quantize_weights", &quantize_weights);

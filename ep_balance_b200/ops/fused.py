@@ -45,3 +45,38 @@ def token_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Te
             and logits.is_contiguous() and logits.data_ptr() % 16 == 0 and plain_autograd()):
         return _TokenCrossEntropy.apply(logits, targets.contiguous())
     return F.cross_entropy(logits.float(), targets)
+
+
+def _dense_heads(g: torch.Tensor) -> torch.Tensor:
+    ok = g.dtype == torch.bfloat16 and g.stride(3) == 1 and g.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in g.stride()[:3])
+    return g if ok else g.to(torch.bfloat16).contiguous(memory_format=torch.contiguous_format).clone()
+
+
+class _SplitRotate(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, qkv, cos, sin):
+        B, S, _, heads, dim = qkv.shape
+        q, k = (qkv.new_empty((B, heads, S, dim)) for _ in range(2))
+        load().rope(qkv, q, k, None, cos, sin, False)
+        ctx.save_for_backward(cos, sin)
+        ctx.shape = qkv.shape
+        return q, k, qkv[:, :, 2].transpose(1, 2)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dq, dk, dv):
+        cos, sin = ctx.saved_tensors
+        dqkv = torch.empty(ctx.shape, dtype=torch.bfloat16, device=cos.device)
+        load().rope(dqkv, _dense_heads(dq), _dense_heads(dk), _dense_heads(dv), cos, sin, True)
+        return dqkv, None, None
+
+
+def split_rotate(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
+    """``qkv`` [B, S, 3, heads, dim] -> q and k with rotary embedding in one kernel, and v (a view), each
+    [B, heads, S, dim]; None where the kernel does not apply.  ``cos`` / ``sin``: [S, dim / 2] tables without gradients."""
+    tables = all(t.dtype == torch.bfloat16 and t.device == qkv.device and t.is_contiguous() and t.data_ptr() % 16 == 0
+                 and t.shape == (qkv.shape[1], qkv.shape[4] // 2) and not t.requires_grad for t in (cos, sin))
+    if (tables and qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
+            and qkv.shape[4] % 16 == 0 and qkv.numel() > 0 and plain_autograd()):
+        return _SplitRotate.apply(qkv, cos, sin)
+    return None
