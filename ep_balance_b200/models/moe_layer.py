@@ -415,20 +415,31 @@ class FusedMoE(nn.Module):
             self._acc_gw2.zero_()
 
     # ---- routing -----------------------------------------------------------
+    def _fused_routing(self) -> bool:
+        """Do forwards without autograd select experts with the fused kernel?"""
+        return bool(self.fused_router or (self.fused_router is None and self.route_fn is None))
+
     def route_tokens(self, tokens: torch.Tensor):
         """fp32 router: logits = x . W_r^T (+ bias), top-k, softmax over the selected logits."""
         with profiling.record("apply/route", time_it=True, device=tokens.device):
+            parts = 1
             if tokens.is_cuda and tokens.dtype == torch.bfloat16 and self.router.dtype == torch.float32:
-                logits = _RouterLinear.apply(tokens, self.router)
+                if not torch.is_grad_enabled() and self._fused_routing():
+                    # the three terms of _RouterLinear's product stay apart: the selection kernel adds them
+                    parts, stacked = 3, torch.empty((3 * self.router.shape[0], self.router.shape[1]), dtype=torch.bfloat16,
+                                                    device=tokens.device)
+                    load().router_split(self.router.detach().contiguous(), stacked)
+                    logits = torch.mm(tokens, stacked.t(), out_dtype=torch.float32)
+                else:
+                    logits = _RouterLinear.apply(tokens, self.router)
             else:
                 logits = tokens.to(self.router.dtype) @ self.router.t()
-            if tokens.is_cuda and not torch.is_grad_enabled() and logits.dtype == torch.float32 and (
-                    self.fused_router or (self.fused_router is None and self.route_fn is None)):
+            if tokens.is_cuda and not torch.is_grad_enabled() and logits.dtype == torch.float32 and self._fused_routing():
                 fr = self.fused_router or dict(mode=0 if self.cfg.normalize_topk else 1, n_groups=1, topk_groups=1, scale=1.0)
                 top_idx = torch.empty((tokens.shape[0], self.cfg.top_k), dtype=torch.int64, device=tokens.device)
                 prob = torch.empty((tokens.shape[0], self.cfg.top_k), dtype=torch.float32, device=tokens.device)
                 load().router_topk(logits.contiguous(), self.router_bias, fr["mode"], fr["n_groups"], fr["topk_groups"],
-                                   fr["scale"], top_idx, prob)
+                                   fr["scale"], top_idx, prob, parts)
                 return top_idx, prob
             if self.router_bias is not None:
                 logits = logits + self.router_bias

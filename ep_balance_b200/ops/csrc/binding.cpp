@@ -374,20 +374,31 @@ void grouped_gemm_fp8(torch::Tensor aq, torch::Tensor sfa, torch::Tensor bq, tor
 
 // Fused inference router: logits [N, E] -> (expert ids int64 [N, K], gate weights fp32 [N, K]).
 void router_topk(torch::Tensor logits, c10::optional<torch::Tensor> bias, int64_t mode, int64_t n_groups,
-                 int64_t topk_groups, double scale, torch::Tensor idx, torch::Tensor weights) {
+                 int64_t topk_groups, double scale, torch::Tensor idx, torch::Tensor weights, int64_t parts) {
   const c10::cuda::CUDAGuard guard(logits.device());
-  TORCH_CHECK(logits.dim() == 2 && idx.dim() == 2 && weights.sizes() == idx.sizes() && idx.size(0) == logits.size(0),
-              "logits [N, E], idx/weights [N, K]");
+  TORCH_CHECK(logits.dim() == 2 && idx.dim() == 2 && weights.sizes() == idx.sizes() && idx.size(0) == logits.size(0) && parts > 0 &&
+                  logits.size(1) % parts == 0,
+              "logits [N, parts * E], idx/weights [N, K]");
+  const int E = (int)(logits.size(1) / parts);
   const float* b = nullptr;
   if (bias.has_value() && bias->defined()) {
-    TORCH_CHECK(bias->numel() == logits.size(1), "bias must be [E]");
+    TORCH_CHECK(bias->numel() == E, "bias must be [E]");
     b = dptr<float>(*bias, "bias", torch::kFloat32);
   }
   cuda_check(epb::launch_router_topk(dptr<float>(logits, "logits", torch::kFloat32), b, (int)logits.size(0),
-                                     (int)logits.size(1), (int)idx.size(1), (int)mode, (int)n_groups, (int)topk_groups,
+                                     E, (int)idx.size(1), (int)mode, (int)n_groups, (int)topk_groups,
                                      (float)scale, dptr<int64_t>(idx, "idx", torch::kInt64),
-                                     dptr<float>(weights, "weights", torch::kFloat32), current_stream()),
+                                     dptr<float>(weights, "weights", torch::kFloat32), current_stream(), (int)parts),
              "launch_router_topk");
+}
+
+// fp32 [E, H] -> bf16 [3 E, H]
+void router_split(torch::Tensor w, torch::Tensor stacked) {
+  const c10::cuda::CUDAGuard guard(w.device());
+  TORCH_CHECK(stacked.numel() == 3 * w.numel(), "router_split: stacked is [3 E, H]");
+  cuda_check(epb::launch_router_split(dptr<float>(w, "w", torch::kFloat32), w.numel(), dptr<void>(stacked, "stacked", torch::kBFloat16),
+                                      current_stream()),
+             "launch_router_split");
 }
 
 // grad (bf16) of the mean cross-entropy: log_prob fp32 [rows, vocab], targets int64 [rows], weight and grad_out fp32 scalars
@@ -486,7 +497,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("wait_signal", &wait_signal);
   m.def("symm_barrier", &symm_barrier);
   m.def("grad_reduce", &grad_reduce);
-  m.def("router_topk", &router_topk);
+  m.def("router_topk", &router_topk, py::arg("logits"), py::arg("bias"), py::arg("mode"), py::arg("n_groups"), py::arg("topk_groups"),
+        py::arg("scale"), py::arg("idx"), py::arg("weights"), py::arg("parts") = 1);
+  m.def("router_split", &router_split);
   m.def("rope", &rope);
   m.def("cross_entropy_backward", &cross_entropy_backward);
   m.def("quantize_rows", &quantize_rows);

@@ -3,6 +3,7 @@
 // masking the winner; 2*G + topk_groups + K steps in group-limited mode.
 #include "router.h"
 
+#include <cuda_bf16.h>
 #include <math_constants.h>
 
 namespace epb {
@@ -10,6 +11,9 @@ namespace {
 
 constexpr int kMaxSlots = 32;
 constexpr unsigned kFull = 0xffffffffu;
+constexpr float kTinySum = 1e-20f;  // floor of the sum that the group-limited weights are normalised by
+
+__device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
 struct Best {
   float v;
@@ -29,19 +33,26 @@ template <int kSlots>
 __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
                                                          int N, int E, int K, int mode, int n_groups, int topk_groups,
                                                          float scale, int64_t* __restrict__ idx,
-                                                         float* __restrict__ weights) {
+                                                         float* __restrict__ weights, int parts) {
   const int lane = threadIdx.x & 31;
   const int t = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   if (t >= N) return;
   const float kNone = -CUDART_INF_F;
-  float s[kSlots];        // selection score of each element held by this lane (-inf: absent or taken)
+  float s[kSlots];        // selection score of each element held by this lane (-inf: absent)
+  bool nan_row = false;   // a NaN logit competes as +inf and makes every weight of the row NaN
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) {
     const int e = j * 32 + lane;
     float v = kNone;
     if (e < E) {
-      v = logits[(size_t)t * E + e] + (bias ? bias[e] : 0.f);
-      if (mode == kRouterGroupLimited) v = __fdividef(1.f, 1.f + __expf(-v));
+      const float* row = logits + (size_t)t * parts * E + e;
+      v = parts == 3 ? (row[0] + row[E]) + row[2 * E] : row[0];
+      if (bias) v += bias[e];
+      if (mode == kRouterGroupLimited) v = sigmoid(v);
+      if (isnan(v)) {
+        nan_row = true;
+        v = CUDART_INF_F;
+      }
     }
     s[j] = v;
   }
@@ -82,17 +93,16 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
   // top-K of s
   float my_val = 0.f;   // lane r keeps the r-th winner
   int my_idx = 0;
+  unsigned taken = 0u;  // bit j: this lane's element j has won (a logit of -inf stays a candidate, a winner does not)
   for (int r = 0; r < K; ++r) {
     Best b{kNone, 0x7fffffff};
 #pragma unroll
     for (int j = 0; j < kSlots; ++j) {
       const int e = j * 32 + lane;
-      if (e < E) b = better(b, Best{s[j], e});
+      if (e < E && !((taken >> j) & 1u)) b = better(b, Best{s[j], e});
     }
     b = warp_argmax(b);
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j)
-      if (j * 32 + lane == b.i) s[j] = kNone;
+    if ((b.i & 31) == lane) taken |= 1u << (b.i >> 5);
     if (lane == r) {
       my_val = b.v;
       my_idx = b.i;
@@ -102,30 +112,51 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
   float w;
   if (mode == kRouterSoftmaxTopk) {
     const float top = __shfl_sync(kFull, my_val, 0);   // winners are in descending order
-    float ex = lane < K ? __expf(my_val - top) : 0.f;
+    float ex = lane < K ? expf(my_val - top) : 0.f;
     float sum = ex;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
     w = ex / sum;
   } else if (mode == kRouterSigmoidTopk) {
-    w = __fdividef(1.f, 1.f + __expf(-my_val));
+    w = sigmoid(my_val);
   } else {
     float sum = lane < K ? my_val : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-    w = my_val / fmaxf(sum, 1e-20f) * scale;
+    w = my_val / fmaxf(sum, kTinySum) * scale;
   }
+  if (__any_sync(kFull, nan_row)) w = CUDART_NAN_F;
   if (lane < K) {
     idx[(size_t)t * K + lane] = my_idx;
     weights[(size_t)t * K + lane] = w;
   }
 }
 
+// x = hi + mid + lo to 24 bits, each term bf16
+__device__ __forceinline__ void split3(float x, __nv_bfloat16 (&out)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    out[i] = __float2bfloat16_rn(x);
+    x -= __bfloat162float(out[i]);
+  }
+}
+
+__global__ void __launch_bounds__(256) router_split_kernel(const float* __restrict__ w, int64_t numel, __nv_bfloat16* __restrict__ out) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += stride) {
+    __nv_bfloat16 s[3];
+    split3(w[i], s);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) out[j * numel + i] = s[j];
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_router_topk(const float* logits, const float* bias, int N, int E, int K, int mode, int n_groups,
-                               int topk_groups, float scale, int64_t* idx, float* weights, cudaStream_t stream) {
+                               int topk_groups, float scale, int64_t* idx, float* weights, cudaStream_t stream, int parts) {
   if (N <= 0) return cudaSuccess;
+  if (parts != 1 && parts != 3) return cudaErrorInvalidValue;
   if (E < K || E > 32 * kMaxSlots || K < 1 || K > 32) return cudaErrorInvalidValue;
   if (mode == kRouterGroupLimited && (n_groups < 1 || n_groups > 32 || E % n_groups != 0 || topk_groups < 1 || topk_groups > n_groups))
     return cudaErrorInvalidValue;
@@ -133,13 +164,20 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int N, in
   const int slots = (E + 31) / 32;
 #define EPB_ROUTER(S)                                                                                              \
   router_topk_kernel<S><<<blocks, 256, 0, stream>>>(logits, bias, N, E, K, mode, n_groups, topk_groups, scale, idx, \
-                                                    weights)
+                                                    weights, parts)
   if (slots <= 2) EPB_ROUTER(2);
   else if (slots <= 4) EPB_ROUTER(4);
   else if (slots <= 8) EPB_ROUTER(8);
   else if (slots <= 16) EPB_ROUTER(16);
   else EPB_ROUTER(32);
 #undef EPB_ROUTER
+  return cudaGetLastError();
+}
+
+cudaError_t launch_router_split(const float* w, int64_t numel, void* stacked, cudaStream_t stream) {
+  if (numel <= 0) return cudaSuccess;
+  const int64_t blocks = (numel + 255) / 256;
+  router_split_kernel<<<(unsigned)(blocks < 2048 ? blocks : 2048), 256, 0, stream>>>(w, numel, reinterpret_cast<__nv_bfloat16*>(stacked));
   return cudaGetLastError();
 }
 

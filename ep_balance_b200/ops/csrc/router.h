@@ -1,6 +1,6 @@
-// Fused top-k routing for inference (router.cu): one warp per token turns a row of fp32 logits into
-// the selected expert ids and their gate weights.  Replaces the chain of PyTorch kernels (sigmoid / topk /
-// scatter / where / topk / normalise: ~15 launches) that dominates a small-batch forward.
+// Fused top-k routing for inference (router.cu): the fp32 weight split into bf16 terms, and one warp per token that turns a row
+// of logits into the selected expert ids and their gate weights.  Replaces chains of PyTorch kernels (split: ~9 launches;
+// sigmoid / topk / scatter / where / topk / normalise: ~15) that dominate a small-batch forward.
 // Forward only: training keeps the differentiable PyTorch formulation.
 #pragma once
 
@@ -16,9 +16,12 @@ enum RouterMode : int {
                             // top-k among the experts of the best `topk_groups` groups, weights normalised
 };
 
-// logits fp32 [N, E] (E <= 1024, E % n_groups == 0), optional bias fp32 [E] added first.
-// idx int64 [N, K], weights fp32 [N, K]; K <= 32.
+// w fp32 [E, H] -> bf16 [3 E, H]: three row blocks that sum to w to 24 mantissa bits.
+cudaError_t launch_router_split(const float* w, int64_t numel, void* stacked, cudaStream_t stream);
+
+// logits fp32 [N, parts * E]: the logits of a row are the sum of its `parts` (1 or 3) blocks of E (E <= 1024,
+// E % n_groups == 0), optional bias fp32 [E] added.  idx int64 [N, K], weights fp32 [N, K]; K <= 32.
 cudaError_t launch_router_topk(const float* logits, const float* bias, int N, int E, int K, int mode, int n_groups,
-                               int topk_groups, float scale, int64_t* idx, float* weights, cudaStream_t stream);
+                               int topk_groups, float scale, int64_t* idx, float* weights, cudaStream_t stream, int parts = 1);
 
 }  // namespace epb
