@@ -15,9 +15,9 @@ from typing import List, Optional
 import torch
 import torch.distributed as dist
 import torch.nn as nn
-import torch.nn.functional as F
 
 from ..core.config import EPLBConfig
+from ..ops.fused import add3, swiglu
 from ..parallel.symm import SymmetricHeap
 from ..utils.status import StatusBoard
 from .moe_layer import FusedMoE, MoEConfig, heap_layout
@@ -63,8 +63,7 @@ class SharedExpert(nn.Module):
         self.down = nn.Linear(ffn, hidden, bias=False)
 
     def forward(self, x):
-        gate, up = self.up(x).chunk(2, dim=-1)
-        return self.down(F.silu(gate) * up)
+        return self.down(swiglu(self.up(x)))
 
 
 class DSv3Block(nn.Module):
@@ -78,7 +77,7 @@ class DSv3Block(nn.Module):
 
     def forward(self, x):
         h = self.norm(x)
-        return x + self.moe(h) + self.shared(h)
+        return add3(x, self.moe(h), self.shared(h))
 
 
 class DSv3Stack(nn.Module):

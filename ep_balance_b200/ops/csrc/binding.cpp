@@ -8,6 +8,7 @@
 #include <map>
 #include <string>
 
+#include "dense.h"
 #include "grouped_gemm.h"
 #include "grouped_gemm_fp8.h"
 #include "loss.h"
@@ -451,6 +452,25 @@ void rope(torch::Tensor packed, torch::Tensor q, torch::Tensor k, c10::optional<
   cuda_check(backward ? epb::launch_rope_backward(a, p, current_stream()) : epb::launch_rope(a, current_stream()), "launch_rope");
 }
 
+const void* vec_ptr(const torch::Tensor& t, const char* name) {
+  const void* p = dptr<const void>(t, name, torch::kBFloat16);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(p) % 16 == 0, name, " must start on a 16-byte boundary");
+  return p;
+}
+// x bf16 [rows, 2F] -> out [rows, F]
+void swiglu(torch::Tensor x, torch::Tensor out) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.dim() == 2 && out.dim() == 2 && x.size(0) == out.size(0) && x.size(1) == 2 * out.size(1), "swiglu: x [rows, 2F], out [rows, F]");
+  cuda_check(epb::launch_swiglu(vec_ptr(x, "x"), const_cast<void*>(vec_ptr(out, "out")), x.size(0), (int)out.size(1), current_stream()),
+             "launch_swiglu");
+}
+void add3(torch::Tensor a, torch::Tensor b, torch::Tensor c, torch::Tensor out) {
+  const c10::cuda::CUDAGuard guard(a.device());
+  TORCH_CHECK(a.sizes() == b.sizes() && a.sizes() == c.sizes() && a.sizes() == out.sizes(), "add3: equal shapes");
+  cuda_check(epb::launch_add3(vec_ptr(a, "a"), vec_ptr(b, "b"), vec_ptr(c, "c"), const_cast<void*>(vec_ptr(out, "out")), a.numel(), current_stream()),
+             "launch_add3");
+}
+
 // ---- symmetric heap over CUDA IPC: one cudaMalloc per rank, mapped into every peer process
 py::tuple ipc_alloc(int64_t nbytes) {
   void* p = nullptr;
@@ -501,6 +521,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("scale"), py::arg("idx"), py::arg("weights"), py::arg("parts") = 1);
   m.def("router_split", &router_split);
   m.def("rope", &rope);
+  m.def("swiglu", &swiglu);
+  m.def("add3", &add3);
   m.def("cross_entropy_backward", &cross_entropy_backward);
   m.def("quantize_rows", &quantize_rows);
   m.def("quantize_weights", &quantize_weights);

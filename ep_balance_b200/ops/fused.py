@@ -80,3 +80,30 @@ def split_rotate(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
             and qkv.shape[4] % 16 == 0 and qkv.numel() > 0 and plain_autograd()):
         return _SplitRotate.apply(qkv, cos, sin)
     return None
+
+
+def _plain_bf16(*tensors: torch.Tensor) -> bool:
+    """No autograd on any of them, and vectors of eight bf16 values at 16-byte addresses on one GPU."""
+    return (not torch.is_grad_enabled() and plain_autograd() and not torch.is_autocast_enabled("cuda")
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()
+                    and t.numel() > 0 and t.data_ptr() % 16 == 0 and t.device == tensors[0].device for t in tensors))
+
+
+def swiglu(packed: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up`` of ``packed`` [..., 2F] = (gate, up); one kernel where autograd is off (the same bits)."""
+    f = packed.shape[-1] // 2
+    if packed.dim() == 2 and packed.shape[1] % 16 == 0 and _plain_bf16(packed):
+        out = packed.new_empty((packed.shape[0], f))
+        load().swiglu(packed, out)
+        return out
+    gate, up = packed.chunk(2, dim=-1)
+    return F.silu(gate) * up
+
+
+def add3(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -> torch.Tensor:
+    """``a + b + c``; one kernel where autograd is off (the same bits)."""
+    if a.shape == b.shape == c.shape and a.numel() % 8 == 0 and _plain_bf16(a, b, c):
+        out = torch.empty_like(a)
+        load().add3(a, b, c, out)
+        return out
+    return a + b + c
