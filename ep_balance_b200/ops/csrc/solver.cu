@@ -16,6 +16,8 @@
 
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace epb {
@@ -737,49 +739,54 @@ __device__ void stage2_domain(const SolverParams& p, Smem& s, int d, int iters, 
             }
           }
           // prefix over source ranks: source s gives min(q_s, max(delta - sum_{s'<s} q_s', 0))
-          int carry = 0;
-          // quotas that are not cached: both columns of the first 64 sources are requested together, so that the move waits
-          // for one global round trip and not for one per 32 sources and one more per target
-          int pre_have[2] = {0, 0}, pre_there[2] = {0, 0};
-          if (!qcached) {
+          auto move = [&](auto in_shared) {
+            constexpr bool kShared = decltype(in_shared)::value;
+            int carry = 0;
+            // quotas that are not cached: both columns of the first 64 sources are requested together, so that the move
+            // waits for one global round trip and not for one per 32 sources and one more per target
+            int pre_have[2] = {0, 0}, pre_there[2] = {0, 0};
+            if (!kShared) {
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              const int sr = b * kWarp + lane;
-              if (sr < R) {
-                const int* row = p.q + ((size_t)sr * E + best.expert) * R;
-                pre_have[b] = row[src];
-                pre_there[b] = row[best.target];
+              for (int b = 0; b < 2; ++b) {
+                const int sr = b * kWarp + lane;
+                if (sr < R) {
+                  const int* row = p.q + ((size_t)sr * E + best.expert) * R;
+                  pre_have[b] = row[src];
+                  pre_there[b] = row[best.target];
+                }
               }
             }
-          }
-          for (int base = 0; base < R && carry < best.delta; base += kWarp) {
-            const int sr = base + lane;
-            int* from = p.q + ((size_t)sr * E + best.expert) * R + src;
-            int* to = p.q + ((size_t)sr * E + best.expert) * R + best.target;
-            int* cfrom = qcached && sr < R ? s.q_c + ((size_t)sr * E + best.expert) * n + bidx : nullptr;
-            int* cto = qcached && sr < R ? s.q_c + ((size_t)sr * E + best.expert) * n + sel : nullptr;
-            const bool ahead = !qcached && base < 2 * kWarp;
-            const int have = sr < R ? (cfrom ? *cfrom : ahead ? pre_have[base / kWarp] : *from) : 0;
-            int incl = have;
-            for (int off = 1; off < kWarp; off <<= 1) {
-              int o = __shfl_up_sync(kFull, incl, off);
-              if (lane >= off) incl += o;
-            }
-            const int before = carry + incl - have;
-            const int mv = min(have, max(best.delta - before, 0));
-            if (sr < R && mv > 0) {
-              *from = have - mv;
-              if (cfrom) {
-                *cfrom = have - mv;
-                *to = (*cto += mv);
-              } else if (ahead) {
-                *to = pre_there[base / kWarp] + mv;
-              } else {
-                *to += mv;
+            for (int base = 0; base < R && carry < best.delta; base += kWarp) {
+              const int sr = base + lane;
+              int* from = p.q + ((size_t)sr * E + best.expert) * R + src;
+              int* to = p.q + ((size_t)sr * E + best.expert) * R + best.target;
+              int* cfrom = kShared ? s.q_c + ((size_t)sr * E + best.expert) * n + bidx : nullptr;
+              int* cto = kShared ? s.q_c + ((size_t)sr * E + best.expert) * n + sel : nullptr;
+              const bool ahead = !kShared && base < 2 * kWarp;
+              const int have = sr < R ? (kShared ? *cfrom : ahead ? (base == 0 ? pre_have[0] : pre_have[1]) : *from) : 0;
+              int incl = have;
+              for (int off = 1; off < kWarp; off <<= 1) {
+                int o = __shfl_up_sync(kFull, incl, off);
+                if (lane >= off) incl += o;
               }
+              const int before = carry + incl - have;
+              const int mv = min(have, max(best.delta - before, 0));
+              if (sr < R && mv > 0) {
+                *from = have - mv;
+                if (kShared) {
+                  *cfrom = have - mv;
+                  *to = (*cto += mv);
+                } else if (ahead) {
+                  *to = (base == 0 ? pre_there[0] : pre_there[1]) + mv;
+                } else {
+                  *to += mv;
+                }
+              }
+              carry += __shfl_sync(kFull, incl, kWarp - 1);
             }
-            carry += __shfl_sync(kFull, incl, kWarp - 1);
-          }
+          };
+          if (qcached) move(std::true_type{});
+          else move(std::false_type{});
           if (lane == 0) {
             if (cached) {
               const int a = (s.erl_c[best.expert * n + bidx] -= best.delta);
@@ -1244,7 +1251,7 @@ cudaError_t launch_solver(const SolverParams& p, const RankTables& tables, cudaS
   if (grid < 1) grid = 1;
   // Where the quotas do not fit in shared memory the whole grid shares out the routing phase (R * E * R quotas and E * R
   // sums over R sources), which one CTA per domain spends most of the kernel on; the extra CTAs only take part in that
-  // phase, four (source, expert) pairs per warp.  64 ranks, 256 experts: kernel and casts 369 -> 229 us with the coalesced
+  // phase, four (source, expert) pairs per warp.  64 ranks, 256 experts: kernel and casts 379 -> 223 us with the coalesced
   // rows of q and the moves' single round trip.
   const bool own_columns = pc.cache_q && p.u_min == 1 && p.R <= 64 && grid >= p.D && !p.probe;
   if (!own_columns && p.R <= 64) {
