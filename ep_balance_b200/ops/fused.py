@@ -1,8 +1,7 @@
 """Autograd wrappers of the dense models' native kernels.
 
 Each public function takes the native path for the tensors its kernels cover and the PyTorch formulation for everything
-else (other devices, types, alignments, function transforms and forward-mode AD, which a custom autograd function has
-no rule for).
+else: other devices, types and alignments, and whoever has to see the operations themselves (:func:`eager`).
 """
 
 from __future__ import annotations
@@ -11,13 +10,24 @@ import torch
 import torch.nn.functional as F
 from torch.autograd import forward_ad
 from torch.autograd.function import once_differentiable
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
+from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
 from .extension import load
 
 
-def plain_autograd() -> bool:
-    """No function transform (vmap, grad, jvp) and no forward-mode level is active."""
-    return not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0
+def eager(*tensors: torch.Tensor) -> bool:
+    """Plain tensors, executed now, with nobody watching.  A kernel launched through the extension is invisible to PyTorch:
+    a tracer (``jit.trace``, ``make_fx``, ``compile``, ``export``) would record the allocation of its output and nothing
+    that fills it, a dispatch or function mode would miss it, a subclass (a fake tensor, an fx proxy) has no memory to run
+    it on, and function transforms and forward-mode AD have no rule for it.  All of them get the PyTorch operations."""
+    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
+            and torch._C._len_torch_dispatch_stack() == 0 and not is_in_torch_dispatch_mode()
+            and (torch._C._len_torch_function_stack() == 0  # `with torch.device(...)` is a function mode that only sets defaults
+                 or all(type(m) is DeviceContext for m in _get_current_function_mode_stack()))
+            and not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0)
 
 
 class _TokenCrossEntropy(torch.autograd.Function):
@@ -40,9 +50,9 @@ class _TokenCrossEntropy(torch.autograd.Function):
 def token_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """``F.cross_entropy(logits.float(), targets)`` for ``logits`` [rows, vocab] and ``targets`` [rows] (mean over the rows whose
     target is not -100), with the gradient of bf16 logits on a GPU taken from the log-probabilities in one pass."""
-    if (logits.is_cuda and logits.dtype == torch.bfloat16 and targets.dtype == torch.int64 and targets.device == logits.device
-            and logits.dim() == 2 and targets.shape == logits.shape[:1] and logits.shape[0] > 0 and logits.shape[1] % 8 == 0
-            and logits.is_contiguous() and logits.data_ptr() % 16 == 0 and plain_autograd()):
+    if (eager(logits, targets) and logits.is_cuda and logits.dtype == torch.bfloat16 and targets.dtype == torch.int64
+            and targets.device == logits.device and logits.dim() == 2 and targets.shape == logits.shape[:1]
+            and logits.shape[0] > 0 and logits.shape[1] % 8 == 0 and logits.is_contiguous() and logits.data_ptr() % 16 == 0):
         return _TokenCrossEntropy.apply(logits, targets.contiguous())
     return F.cross_entropy(logits.float(), targets)
 
@@ -74,36 +84,39 @@ class _SplitRotate(torch.autograd.Function):
 def split_rotate(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor):
     """``qkv`` [B, S, 3, heads, dim] -> q and k with rotary embedding in one kernel, and v (a view), each
     [B, heads, S, dim]; None where the kernel does not apply.  ``cos`` / ``sin``: [S, dim / 2] tables without gradients."""
+    if not eager(qkv, cos, sin):
+        return None
     tables = all(t.dtype == torch.bfloat16 and t.device == qkv.device and t.is_contiguous() and t.data_ptr() % 16 == 0
                  and t.shape == (qkv.shape[1], qkv.shape[4] // 2) and not t.requires_grad for t in (cos, sin))
     if (tables and qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
-            and qkv.shape[4] % 16 == 0 and qkv.numel() > 0 and plain_autograd()):
+            and qkv.shape[4] % 16 == 0 and qkv.numel() > 0):
         return _SplitRotate.apply(qkv, cos, sin)
     return None
 
 
 def _plain_bf16(*tensors: torch.Tensor) -> bool:
     """No autograd on any of them, and vectors of eight bf16 values at 16-byte addresses on one GPU."""
-    return (not torch.is_grad_enabled() and plain_autograd() and not torch.is_autocast_enabled("cuda")
-            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()
-                    and t.numel() > 0 and t.data_ptr() % 16 == 0 and t.device == tensors[0].device for t in tensors))
+    return (eager(*tensors) and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+            and all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and t.numel() > 0 and t.data_ptr() % 16 == 0
+                    and t.device == tensors[0].device for t in tensors))
 
 
 def swiglu(packed: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` of ``packed`` [..., 2F] = (gate, up); one kernel where autograd is off (the same bits)."""
-    f = packed.shape[-1] // 2
-    if packed.dim() == 2 and packed.shape[1] % 16 == 0 and _plain_bf16(packed):
-        out = packed.new_empty((packed.shape[0], f))
-        load().swiglu(packed, out)
-        return out
+    if not torch.jit.is_scripting():
+        if _plain_bf16(packed) and packed.dim() == 2 and packed.shape[1] % 16 == 0:
+            out = packed.new_empty((packed.shape[0], packed.shape[1] // 2))
+            load().swiglu(packed, out)
+            return out
     gate, up = packed.chunk(2, dim=-1)
     return F.silu(gate) * up
 
 
 def add3(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -> torch.Tensor:
     """``a + b + c``; one kernel where autograd is off (the same bits)."""
-    if a.shape == b.shape == c.shape and a.numel() % 8 == 0 and _plain_bf16(a, b, c):
-        out = torch.empty_like(a)
-        load().add3(a, b, c, out)
-        return out
+    if not torch.jit.is_scripting():
+        if _plain_bf16(a, b, c) and a.shape == b.shape == c.shape and a.numel() % 8 == 0:
+            out = torch.empty_like(a)
+            load().add3(a, b, c, out)
+            return out
     return a + b + c
