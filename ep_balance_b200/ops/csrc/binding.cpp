@@ -33,12 +33,23 @@ void cuda_check(cudaError_t e, const char* what) {
   TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e));
 }
 
+// The tensor's memory.  A fake or functional tensor says that it is on a GPU and has none.
+void* memory(const torch::Tensor& t, const char* name) {
+  void* p = t.data_ptr();
+  TORCH_CHECK(t.numel() == 0 || p != nullptr, name, " has no memory (a fake or wrapped tensor)");
+  return p;
+}
+c10::Device device_with_memory(const torch::Tensor& t) {
+  memory(t, "the first tensor");
+  return t.device();
+}
+
 template <typename T>
 T* dptr(const torch::Tensor& t, const char* name, c10::ScalarType st) {
   TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
   TORCH_CHECK(t.scalar_type() == st, name, " has the wrong dtype");
-  return reinterpret_cast<T*>(t.data_ptr());
+  return reinterpret_cast<T*>(memory(t, name));
 }
 
 int get_int(const py::dict& d, const char* key, int fallback) {
@@ -81,7 +92,7 @@ void solve_plan(torch::Tensor omega, torch::Tensor dom, torch::Tensor cost, torc
                 int64_t patience, bool allow_cross, bool probe, torch::Tensor x, torch::Tensor q, torch::Tensor erl,
                 torch::Tensor rank_load, torch::Tensor slot_used, torch::Tensor stuck, torch::Tensor theta,
                 torch::Tensor control, torch::Tensor sync, torch::Tensor status) {
-  const c10::cuda::CUDAGuard guard(omega.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(omega));
   epb::SolverParams p{};
   p.omega = dptr<const int32_t>(omega, "omega", torch::kInt32);
   p.dom = dptr<const int32_t>(dom, "dom", torch::kInt32);
@@ -127,7 +138,7 @@ void solve_plan(torch::Tensor omega, torch::Tensor dom, torch::Tensor cost, torc
 void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor out0, c10::optional<torch::Tensor> out1,
                   torch::Tensor group_off, torch::Tensor group_rows, torch::Tensor group_wslot, torch::Tensor totals,
                   torch::Tensor status, int64_t num_sms, int64_t ctas, bool narrow) {
-  const c10::cuda::CUDAGuard guard(a.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(a));
   TORCH_CHECK(ctas == 1 || ctas == 2, "ctas must be 1 or 2");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "bf16 operands only");
   TORCH_CHECK(a.is_contiguous() && b.is_contiguous() && out0.is_contiguous(), "operands must be contiguous");
@@ -141,8 +152,8 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
   g.n_groups_cap = (int)group_rows.size(0);
   g.row_capacity = (int)a.size(0);
   g.status = dptr<int>(status, "status", torch::kInt32);
-  g.out0 = out0.numel() > 0 ? out0.data_ptr() : nullptr;  // kFwd1 without the pre-activations
-  g.out1 = out1.has_value() ? out1->data_ptr() : nullptr;
+  g.out0 = out0.numel() > 0 ? memory(out0, "out0") : nullptr;  // kFwd1 without the pre-activations
+  g.out1 = out1.has_value() ? memory(*out1, "out1") : nullptr;
   CUtensorMap tmA, tmB;
   const uint64_t T = a.size(0);
   const uint32_t box_rows = narrow ? epb::kNarrowBoxRows : 128;  // token rows of a box
@@ -153,27 +164,27 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
     case epb::kFwd2:
       g.N = (int)b.size(1);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
-           epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 128);
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
+           epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 128);
       break;
     case epb::kFwd1:
       g.N = (int)b.size(1) / 2;
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
-           epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 128);
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
+           epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 128);
       break;
     case epb::kDgrad1:
     case epb::kDgrad2:
       g.N = (int)b.size(2);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, box_rows) &&
-           epb::make_tmap_3d(&tmB, b.data_ptr(), b.size(0), b.size(1), b.size(2), 64, 64);
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
+           epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 64);
       break;
     case epb::kWgrad:
       g.N = (int)b.size(1);
       g.M_out = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, a.data_ptr(), T, a.size(1), 64, 64) &&
-           epb::make_tmap_2d(&tmB, b.data_ptr(), b.size(0), b.size(1), 64, 64);
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, 64) &&
+           epb::make_tmap_2d(&tmB, memory(b, "b"), b.size(0), b.size(1), 64, 64);
       break;
     default:
       TORCH_CHECK(false, "unknown grouped GEMM mode");
@@ -190,7 +201,7 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
 void adamw_step(torch::Tensor param, torch::Tensor grad, torch::Tensor exp_avg, torch::Tensor exp_avg_sq, double lr,
                 double beta1, double beta2, double eps, double weight_decay, int64_t step,
                 c10::optional<torch::Tensor> step_tensor, c10::optional<torch::Tensor> status_guard) {
-  const c10::cuda::CUDAGuard guard(param.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(param));
   TORCH_CHECK(param.is_contiguous() && grad.is_contiguous() && exp_avg.is_contiguous() && exp_avg_sq.is_contiguous(),
               "adamw_step needs contiguous tensors");
   const bool grad_f32 = param.scalar_type() == torch::kBFloat16 && grad.scalar_type() == torch::kFloat32;
@@ -201,10 +212,10 @@ void adamw_step(torch::Tensor param, torch::Tensor grad, torch::Tensor exp_avg, 
   TORCH_CHECK(grad.numel() == param.numel() && exp_avg.numel() == param.numel() && exp_avg_sq.numel() == param.numel(),
               "adamw_step size mismatch");
   epb::AdamArgs a{};
-  a.param = param.data_ptr();
-  a.grad = grad.data_ptr();
-  a.exp_avg = exp_avg.data_ptr();
-  a.exp_avg_sq = exp_avg_sq.data_ptr();
+  a.param = memory(param, "param");
+  a.grad = memory(grad, "grad");
+  a.exp_avg = memory(exp_avg, "exp_avg");
+  a.exp_avg_sq = memory(exp_avg_sq, "exp_avg_sq");
   a.numel = (size_t)param.numel();
   a.lr = (float)lr;
   a.beta1 = (float)beta1;
@@ -230,7 +241,7 @@ void adamw_step(torch::Tensor param, torch::Tensor grad, torch::Tensor exp_avg, 
 }
 
 void wait_probe(torch::Tensor flag, int64_t target, int64_t budget_ns, torch::Tensor status) {
-  const c10::cuda::CUDAGuard guard(flag.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(flag));
   cuda_check(epb::launch_wait_probe(reinterpret_cast<const unsigned*>(dptr<int32_t>(flag, "flag", torch::kInt32)),
                                     (unsigned)target, (unsigned long long)budget_ns,
                                     dptr<int>(status, "status", torch::kInt32), current_stream()),
@@ -240,7 +251,7 @@ void wait_probe(torch::Tensor flag, int64_t target, int64_t budget_ns, torch::Te
 // ---- one-sided transfers over peer-mapped windows (descriptors: int64 [K, 4] on the device)
 void copy_batched(bool is_put, torch::Tensor desc, torch::Tensor window_ptrs, uint64_t local_base, bool use_bulk,
                   int64_t blocks_per_desc, torch::Tensor status) {
-  const c10::cuda::CUDAGuard guard(desc.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(desc));
   TORCH_CHECK(desc.dim() == 2 && desc.size(1) == 4, "descriptors must be int64 [K, 4]");
   epb::BatchedCopyArgs a{};
   a.desc = reinterpret_cast<const epb::CopyDesc*>(dptr<int64_t>(desc, "desc", torch::kInt64));
@@ -263,20 +274,20 @@ void put_batched(torch::Tensor desc, torch::Tensor window_ptrs, uint64_t local_b
   copy_batched(true, desc, window_ptrs, local_base, use_bulk, blocks_per_desc, status);
 }
 void signal_peers(torch::Tensor signal_ptrs, int64_t peer, int64_t idx, int64_t value) {
-  const c10::cuda::CUDAGuard guard(signal_ptrs.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(signal_ptrs));
   cuda_check(epb::launch_signal(reinterpret_cast<unsigned* const*>(dptr<int64_t>(signal_ptrs, "signal_ptrs", torch::kInt64)),
                                 (int)signal_ptrs.numel(), (int)peer, (int)idx, (unsigned)value, current_stream()),
              "launch_signal");
 }
 void wait_signal(uint64_t word, int64_t expected, int64_t idx, int64_t budget_ns, torch::Tensor status) {
-  const c10::cuda::CUDAGuard guard(status.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(status));
   cuda_check(epb::launch_wait_signal(reinterpret_cast<const unsigned*>(static_cast<uintptr_t>(word)), (unsigned)expected,
                                      (int)idx, (unsigned long long)budget_ns, dptr<int>(status, "status", torch::kInt32),
                                      current_stream()),
              "launch_wait_signal");
 }
 void symm_barrier(torch::Tensor signal_ptrs, int64_t slot, int64_t me, torch::Tensor epoch_word, torch::Tensor status) {
-  const c10::cuda::CUDAGuard guard(signal_ptrs.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(signal_ptrs));
   cuda_check(epb::launch_symm_barrier(reinterpret_cast<unsigned* const*>(dptr<int64_t>(signal_ptrs, "signal_ptrs", torch::kInt64)),
                                       (int)slot, (int)signal_ptrs.numel(), (int)me,
                                       reinterpret_cast<unsigned*>(dptr<int32_t>(epoch_word, "epoch_word", torch::kInt32)),
@@ -288,7 +299,7 @@ void symm_barrier(torch::Tensor signal_ptrs, int64_t slot, int64_t me, torch::Te
 void grad_reduce(torch::Tensor g_ptrs, int64_t elems_per_slot, torch::Tensor slot_of, torch::Tensor main_rank,
                  torch::Tensor home_index, int64_t me, int64_t home_cap, torch::Tensor accum, bool include_self,
                  bool overwrite) {
-  const c10::cuda::CUDAGuard guard(g_ptrs.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(g_ptrs));
   epb::GradReduceArgs a{};
   a.g_ptrs = reinterpret_cast<void* const*>(dptr<int64_t>(g_ptrs, "g_ptrs", torch::kInt64));
   a.elems_per_slot = (size_t)elems_per_slot;
@@ -303,7 +314,7 @@ void grad_reduce(torch::Tensor g_ptrs, int64_t elems_per_slot, torch::Tensor slo
   TORCH_CHECK(accum.is_cuda() && accum.is_contiguous(), "accum must be a contiguous CUDA tensor");
   TORCH_CHECK(accum.scalar_type() == torch::kFloat32 || accum.scalar_type() == torch::kBFloat16, "accum: fp32 or bf16");
   TORCH_CHECK(accum.numel() == home_cap * elems_per_slot, "accum must be [home_cap, elems_per_slot]");
-  a.accum = accum.data_ptr();
+  a.accum = memory(accum, "accum");
   a.accum_fp32 = accum.scalar_type() == torch::kFloat32 ? 1 : 0;
   a.include_self = include_self ? 1 : 0;
   a.overwrite = overwrite ? 1 : 0;
@@ -312,7 +323,7 @@ void grad_reduce(torch::Tensor g_ptrs, int64_t elems_per_slot, torch::Tensor slo
 
 // ---- block-scaled fp8 grouped GEMM and its quantisers
 void quantize_rows(torch::Tensor x, torch::Tensor q, torch::Tensor sfa) {
-  const c10::cuda::CUDAGuard guard(x.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(x));
   TORCH_CHECK(x.dim() == 2 && q.dim() == 2 && q.sizes() == x.sizes(), "x and q must be [rows, K]");
   const int rows = (int)x.size(0), K = (int)x.size(1);
   TORCH_CHECK(rows % 128 == 0 && K % 128 == 0, "rows and K must be multiples of 128");
@@ -322,7 +333,7 @@ void quantize_rows(torch::Tensor x, torch::Tensor q, torch::Tensor sfa) {
              "launch_quantize_rows");
 }
 void quantize_weights(torch::Tensor w, torch::Tensor q, torch::Tensor sfb) {
-  const c10::cuda::CUDAGuard guard(w.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(w));
   TORCH_CHECK(w.dim() == 3 && q.sizes() == w.sizes(), "w and q must be [slots, N, K]");
   const int S = (int)w.size(0), N = (int)w.size(1), K = (int)w.size(2);
   TORCH_CHECK(N % 128 == 0 && K % 128 == 0, "N and K must be multiples of 128");
@@ -334,7 +345,7 @@ void quantize_weights(torch::Tensor w, torch::Tensor q, torch::Tensor sfb) {
 void grouped_gemm_fp8(torch::Tensor aq, torch::Tensor sfa, torch::Tensor bq, torch::Tensor sfb, torch::Tensor out,
                       torch::Tensor group_off, torch::Tensor group_rows, torch::Tensor group_wslot, torch::Tensor totals,
                       torch::Tensor status, int64_t num_sms, int64_t ctas) {
-  const c10::cuda::CUDAGuard guard(aq.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(aq));
   TORCH_CHECK(aq.dim() == 2 && bq.dim() == 3 && out.dim() == 2, "aq [T, K], bq [slots, N, K], out [T, N]");
   const int64_t T = aq.size(0), K = aq.size(1), N = bq.size(1);
   TORCH_CHECK(bq.size(2) == K && out.size(0) == T && out.size(1) == N, "shape mismatch");
@@ -376,7 +387,7 @@ void grouped_gemm_fp8(torch::Tensor aq, torch::Tensor sfa, torch::Tensor bq, tor
 // Fused inference router: logits [N, E] -> (expert ids int64 [N, K], gate weights fp32 [N, K]).
 void router_topk(torch::Tensor logits, c10::optional<torch::Tensor> bias, int64_t mode, int64_t n_groups,
                  int64_t topk_groups, double scale, torch::Tensor idx, torch::Tensor weights, int64_t parts) {
-  const c10::cuda::CUDAGuard guard(logits.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(logits));
   TORCH_CHECK(logits.dim() == 2 && idx.dim() == 2 && weights.sizes() == idx.sizes() && idx.size(0) == logits.size(0) && parts > 0 &&
                   logits.size(1) % parts == 0,
               "logits [N, parts * E], idx/weights [N, K]");
@@ -395,7 +406,7 @@ void router_topk(torch::Tensor logits, c10::optional<torch::Tensor> bias, int64_
 
 // fp32 [E, H] -> bf16 [3 E, H]
 void router_split(torch::Tensor w, torch::Tensor stacked) {
-  const c10::cuda::CUDAGuard guard(w.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(w));
   TORCH_CHECK(stacked.numel() == 3 * w.numel(), "router_split: stacked is [3 E, H]");
   cuda_check(epb::launch_router_split(dptr<float>(w, "w", torch::kFloat32), w.numel(), dptr<void>(stacked, "stacked", torch::kBFloat16),
                                       current_stream()),
@@ -405,7 +416,7 @@ void router_split(torch::Tensor w, torch::Tensor stacked) {
 // grad (bf16) of the mean cross-entropy: log_prob fp32 [rows, vocab], targets int64 [rows], weight and grad_out fp32 scalars
 void cross_entropy_backward(torch::Tensor log_prob, torch::Tensor targets, torch::Tensor weight, torch::Tensor grad_out,
                             torch::Tensor grad) {
-  const c10::cuda::CUDAGuard guard(log_prob.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(log_prob));
   TORCH_CHECK(log_prob.dim() == 2 && targets.dim() == 1 && targets.size(0) == log_prob.size(0) && weight.numel() == 1 &&
                   grad_out.numel() == 1 && grad.sizes() == log_prob.sizes(),
               "cross_entropy_backward: log_prob and grad [rows, vocab], targets [rows], weight [], grad_out []");
@@ -424,7 +435,7 @@ void cross_entropy_backward(torch::Tensor log_prob, torch::Tensor targets, torch
 // packed [B, S, 3, heads, dim] -> q, k [B, heads, S, dim]; backward: the gradients of q, k and v -> that of packed (any strides that
 // are multiples of 8, dense last dimension)
 void rope(torch::Tensor packed, torch::Tensor q, torch::Tensor k, c10::optional<torch::Tensor> v, torch::Tensor cos, torch::Tensor sin, bool backward) {
-  const c10::cuda::CUDAGuard guard(packed.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(packed));
   TORCH_CHECK(packed.dim() == 5 && packed.size(2) == 3, "rope: packed is [B, S, 3, heads, dim]");
   epb::RopeArgs a{};
   a.B = (int)packed.size(0);
@@ -444,7 +455,7 @@ void rope(torch::Tensor packed, torch::Tensor q, torch::Tensor k, c10::optional<
     TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 4 && t.size(0) == a.B && t.size(1) == a.heads &&
                     t.size(2) == a.S && t.size(3) == a.dim && (t.stride(3) == 1 || t.numel() == 0),
                 "rope: q, k and v are bf16 [B, heads, S, dim] with a dense last dimension");
-    a.out[i] = t.data_ptr();
+    a.out[i] = memory(t, "q, k or v");
     aligned = aligned && reinterpret_cast<uintptr_t>(a.out[i]) % 16 == 0;
     for (int j = 0; j < 3; ++j) a.stride[i][j] = t.stride(j);
   }
@@ -459,13 +470,13 @@ const void* vec_ptr(const torch::Tensor& t, const char* name) {
 }
 // x bf16 [rows, 2F] -> out [rows, F]
 void swiglu(torch::Tensor x, torch::Tensor out) {
-  const c10::cuda::CUDAGuard guard(x.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(x));
   TORCH_CHECK(x.dim() == 2 && out.dim() == 2 && x.size(0) == out.size(0) && x.size(1) == 2 * out.size(1), "swiglu: x [rows, 2F], out [rows, F]");
   cuda_check(epb::launch_swiglu(vec_ptr(x, "x"), const_cast<void*>(vec_ptr(out, "out")), x.size(0), (int)out.size(1), current_stream()),
              "launch_swiglu");
 }
 void add3(torch::Tensor a, torch::Tensor b, torch::Tensor c, torch::Tensor out) {
-  const c10::cuda::CUDAGuard guard(a.device());
+  const c10::cuda::CUDAGuard guard(device_with_memory(a));
   TORCH_CHECK(a.sizes() == b.sizes() && a.sizes() == c.sizes() && a.sizes() == out.sizes(), "add3: equal shapes");
   cuda_check(epb::launch_add3(vec_ptr(a, "a"), vec_ptr(b, "b"), vec_ptr(c, "c"), const_cast<void*>(vec_ptr(out, "out")), a.numel(), current_stream()),
              "launch_add3");
@@ -498,6 +509,9 @@ torch::Tensor tensor_from_ptr(uint64_t p, int64_t nbytes, int64_t device) {
 
 const void* cp(uint64_t a) { return reinterpret_cast<const void*>(static_cast<uintptr_t>(a)); }
 void* mp(uint64_t a) { return reinterpret_cast<void*>(static_cast<uintptr_t>(a)); }
+void whole_pass(int n, std::initializer_list<uint64_t> addresses) {
+  for (uint64_t a : addresses) TORCH_CHECK(n <= 0 || a != 0, "MoeRuntime: a tensor of the pass has no memory (a fake or wrapped tensor)");
+}
 
 }  // namespace
 
@@ -577,12 +591,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("act_fp8", [](MoeRuntime& r) { r.act_fp8(current_stream()); })
       .def("gemm2_fp8", [](MoeRuntime& r) { r.gemm2_fp8(current_stream()); })
       .def("forward_fp8", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n) {
+        whole_pass(n, {tok, idx, prob, out});
         r.forward_fp8(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream());
       })
       .def("forward", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n, bool train) {
+        whole_pass(n, {tok, idx, prob, out});
         r.forward(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream(), train);
       }, py::arg("tokens"), py::arg("topk_idx"), py::arg("topk_prob"), py::arg("out"), py::arg("num_tokens"), py::arg("train") = true)
       .def("backward", [](MoeRuntime& r, uint64_t dout, uint64_t dtok, uint64_t dprob, int n) {
+        whole_pass(n, {dout, dtok, dprob});
         r.backward(cp(dout), mp(dtok), (float*)mp(dprob), n, current_stream());
       });
 }
