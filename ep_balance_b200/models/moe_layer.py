@@ -40,6 +40,7 @@ from ..core.config import EPLBConfig
 from ..core.problem import ProblemSpec
 from ..core.topology import Topology
 from ..ops.extension import load
+from ..ops.fused import eager
 from ..parallel.symm import HeapLayout, SymmetricHeap
 from ..utils import profiling
 
@@ -424,7 +425,7 @@ class FusedMoE(nn.Module):
         with profiling.record("apply/route", time_it=True, device=tokens.device):
             parts = 1
             if tokens.is_cuda and tokens.dtype == torch.bfloat16 and self.router.dtype == torch.float32:
-                if not torch.is_grad_enabled() and self._fused_routing():
+                if not torch.is_grad_enabled() and self._fused_routing() and eager(tokens, self.router):
                     # the three terms of _RouterLinear's product stay apart: the selection kernel adds them
                     parts, stacked = 3, torch.empty((3 * self.router.shape[0], self.router.shape[1]), dtype=torch.bfloat16,
                                                     device=tokens.device)

@@ -100,3 +100,31 @@ def test_traced_shared_expert_computes(pretend_cuda, monkeypatch, tracer):
             f = torch.export.export(m, (x,)).module()
         gate, up = F.linear(y, m.up.weight).chunk(2, dim=-1)
         assert torch.equal(f(y), F.linear(F.silu(gate) * up, m.down.weight))
+
+
+def test_inference_router(pretend_cuda, monkeypatch):
+    """Forward-mode AD and modes get _RouterLinear, which refuses what it has no rule for; a plain call splits natively."""
+    from types import SimpleNamespace
+
+    from torch.autograd import forward_ad
+
+    from ep_balance_b200.models import moe_layer
+
+    class Reached(Exception):
+        pass
+
+    def general(*args):
+        raise Reached
+    monkeypatch.setattr(moe_layer, "load", fused.load)
+    monkeypatch.setattr(moe_layer._RouterLinear, "apply", general)
+    layer = SimpleNamespace(router=torch.nn.Parameter(torch.randn(8, 16)), _fused_routing=lambda: True)
+    x = _bf16(4, 16)
+    with torch.no_grad():
+        with pytest.raises(AssertionError):
+            moe_layer.FusedMoE.route_tokens(layer, x)
+        with FlopCounterMode(display=False), pytest.raises(Reached):
+            moe_layer.FusedMoE.route_tokens(layer, x)
+        with forward_ad.dual_level(), pytest.raises(Reached):
+            moe_layer.FusedMoE.route_tokens(layer, forward_ad.make_dual(x, x))
+        with pytest.raises(Reached):
+            torch.vmap(lambda z: moe_layer.FusedMoE.route_tokens(layer, z)[1])(_bf16(3, 4, 16))
