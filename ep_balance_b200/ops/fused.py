@@ -9,7 +9,6 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 from torch.autograd import forward_ad
-from torch.autograd.function import once_differentiable
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 from torch.utils._python_dispatch import is_in_torch_dispatch_mode
@@ -31,20 +30,34 @@ def eager(*tensors: torch.Tensor) -> bool:
 
 
 class _TokenCrossEntropy(torch.autograd.Function):
+    """(loss, log-probabilities).  The second output is there for second derivatives: backward's formula reads it, and as an
+    output it is connected to the logits."""
+
     @staticmethod
     def forward(ctx, logits, targets):
         log_prob = torch.log_softmax(logits.float(), -1)
         loss, weight = torch.ops.aten.nll_loss_forward(log_prob, targets, None, 1, -100)  # 1: mean
         ctx.save_for_backward(log_prob, targets, weight)
-        return loss
+        ctx.set_materialize_grads(False)
+        ctx.dtype = logits.dtype
+        return loss, log_prob
 
     @staticmethod
-    @once_differentiable
-    def backward(ctx, dloss):
+    def backward(ctx, dloss, dlog_prob):
         log_prob, targets, weight = ctx.saved_tensors
-        grad = torch.empty_like(log_prob, dtype=torch.bfloat16)
-        load().cross_entropy_backward(log_prob, targets, weight, dloss.contiguous(), grad)
-        return grad, None
+        if dlog_prob is None and not torch.is_grad_enabled() and eager(log_prob, targets, dloss):
+            grad = torch.empty_like(log_prob, dtype=torch.bfloat16)
+            load().cross_entropy_backward(log_prob, targets, weight, dloss.contiguous(), grad)
+            return grad, None
+        prob = log_prob.exp()
+        grad = torch.zeros_like(prob)
+        if dloss is not None:
+            counted = targets != -100
+            scale = torch.where(counted, dloss / weight, 0.0).unsqueeze(1)
+            grad = (prob * scale).scatter_add(1, torch.where(counted, targets, 0).unsqueeze(1), -scale)
+        if dlog_prob is not None:
+            grad = grad + dlog_prob - prob * dlog_prob.sum(-1, keepdim=True)
+        return grad.to(ctx.dtype), None
 
 
 def token_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
@@ -53,13 +66,18 @@ def token_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Te
     if (eager(logits, targets) and logits.is_cuda and logits.dtype == torch.bfloat16 and targets.dtype == torch.int64
             and targets.device == logits.device and logits.dim() == 2 and targets.shape == logits.shape[:1]
             and logits.shape[0] > 0 and logits.shape[1] % 8 == 0 and logits.is_contiguous() and logits.data_ptr() % 16 == 0):
-        return _TokenCrossEntropy.apply(logits, targets.contiguous())
+        return _TokenCrossEntropy.apply(logits, targets.contiguous())[0]
     return F.cross_entropy(logits.float(), targets)
 
 
 def _dense_heads(g: torch.Tensor) -> torch.Tensor:
     ok = g.dtype == torch.bfloat16 and g.stride(3) == 1 and g.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in g.stride()[:3])
     return g if ok else g.to(torch.bfloat16).contiguous(memory_format=torch.contiguous_format).clone()
+
+
+def _rotate_back(g, cos, sin):
+    g1, g2 = g[..., : g.shape[-1] // 2], g[..., g.shape[-1] // 2:]
+    return torch.cat([g1 * cos + g2 * sin, g2 * cos - g1 * sin], dim=-1)
 
 
 class _SplitRotate(torch.autograd.Function):
@@ -73,9 +91,11 @@ class _SplitRotate(torch.autograd.Function):
         return q, k, qkv[:, :, 2].transpose(1, 2)
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dq, dk, dv):
         cos, sin = ctx.saved_tensors
+        if torch.is_grad_enabled() or not eager(dq, dk, dv, cos, sin):  # second derivatives: the operations themselves
+            back = _rotate_back(dq, cos, sin), _rotate_back(dk, cos, sin), dv
+            return torch.stack([g.transpose(1, 2) for g in back], 2), None, None
         dqkv = torch.empty(ctx.shape, dtype=torch.bfloat16, device=cos.device)
         load().rope(dqkv, _dense_heads(dq), _dense_heads(dk), _dense_heads(dv), cos, sin, True)
         return dqkv, None, None
