@@ -42,3 +42,20 @@ def test_special_rows():
     assert bool(token_cross_entropy(x, t).isnan())
     full = torch.full((4, 64), float("-inf"), device="cuda").bfloat16()
     assert bool(token_cross_entropy(full, t).isnan())
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 8), (65, 1000), (4096, 32000)])
+@pytest.mark.parametrize("spread", [0.9, 8.0])
+def test_gradient_has_the_bits_of_the_operations_it_replaces(rows, vocab, spread):
+    from ep_balance_b200.ops.fused import token_cross_entropy
+
+    torch.manual_seed(1)
+    x = (torch.randn(rows, vocab, device="cuda") * spread).bfloat16()
+    t = torch.randint(0, vocab, (rows,), device="cuda")
+    t[1::7] = -100
+    grads = []
+    for f in (token_cross_entropy, lambda z, y: F.cross_entropy(z.float(), y)):
+        z = x.clone().requires_grad_(True)
+        (f(z, t) * 0.3).backward()
+        grads.append(z.grad)
+    assert torch.equal(*grads)

@@ -43,3 +43,28 @@ def test_other_layouts_take_the_general_path():
     assert split_rotate(x.float(), cos, cos) is None
     assert split_rotate(x, cos.float(), cos) is None
     assert split_rotate(x[..., :8], cos[:, :4], cos[:, :4]) is None
+
+
+@pytest.mark.parametrize("B,S,heads,dim", [(1, 1, 1, 16), (3, 37, 3, 48), (2, 2048, 16, 128)])
+def test_gradient_has_the_bits_of_the_operations_it_replaces(B, S, heads, dim):
+    """Gradients laid out as attention's backward hands them over: q and k per head, v per position."""
+    from ep_balance_b200.models.gpt_moe import apply_rope, rope_tables
+    from ep_balance_b200.ops.fused import split_rotate
+
+    torch.manual_seed(1)
+    cos, sin = rope_tables(S, dim, 10000.0, "cuda", torch.bfloat16)
+    x = torch.randn(B, S, 3, heads, dim, device="cuda").bfloat16()
+    dq, dk = (torch.randn(B, heads, S, dim, device="cuda").bfloat16() for _ in range(2))
+    dv = torch.randn(B, S, heads, dim, device="cuda").bfloat16().transpose(1, 2)
+    grads, strides = [], []
+    for general in (False, True):
+        z = x.clone().requires_grad_(True)
+        if general:
+            q, k, v = z.permute(2, 0, 3, 1, 4)
+            parts = apply_rope(q, cos, sin), apply_rope(k, cos, sin), v
+        else:
+            parts = split_rotate(z, cos, sin)
+        torch.autograd.backward(parts, [dq, dk, dv])
+        grads.append(z.grad)
+        strides.append([p.stride() for p in parts])
+    assert torch.equal(*grads) and strides[0] == strides[1]  # (the strides choose attention's kernel)
