@@ -39,15 +39,18 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
   if (t >= N) return;
   const float kNone = -CUDART_INF_F;
   float s[kSlots];        // selection score of each element held by this lane (-inf: absent)
-  bool nan_row = false;   // a NaN logit competes as +inf and makes every weight of the row NaN
+  bool nan_row = false;   // a NaN logit competes as +inf; its weight, or where weights are normalised the row's, are NaN
+  auto logit = [&](int e) {
+    const float* row = logits + (size_t)t * parts * E + e;
+    const float v = parts == 3 ? (row[0] + row[E]) + row[2 * E] : row[0];
+    return bias ? v + bias[e] : v;
+  };
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) {
     const int e = j * 32 + lane;
     float v = kNone;
     if (e < E) {
-      const float* row = logits + (size_t)t * parts * E + e;
-      v = parts == 3 ? (row[0] + row[E]) + row[2 * E] : row[0];
-      if (bias) v += bias[e];
+      v = logit(e);
       if (mode == kRouterGroupLimited) v = sigmoid(v);
       if (isnan(v)) {
         nan_row = true;
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
     w = my_val / fmaxf(sum, kTinySum) * scale;
   }
-  if (__any_sync(kFull, nan_row)) w = CUDART_NAN_F;
+  if (__any_sync(kFull, nan_row) && (mode != kRouterSigmoidTopk || (lane < K && isnan(logit(my_idx))))) w = CUDART_NAN_F;
   if (lane < K) {
     idx[(size_t)t * K + lane] = my_idx;
     weights[(size_t)t * K + lane] = w;

@@ -52,3 +52,16 @@ def test_masked_equal_and_nan_logits():
         assert torch.allclose(prob[r], want[r], atol=1e-6)
     assert bool(prob[3].isnan().all()) and bool(prob[4].isnan().all())
     assert idx[2].tolist() == list(range(8)) and int(idx[3, 0]) == 11
+
+
+def test_a_nan_logit_spoils_its_own_sigmoid_weight_only():
+    from ep_balance_b200.ops.extension import load
+
+    x = torch.randn(3, 40, device="cuda")
+    x[0, 33] = float("nan")
+    x[1, 2] = float("inf")
+    idx, prob = torch.empty((3, 4), dtype=torch.int64, device="cuda"), torch.empty((3, 4), device="cuda")
+    load().router_topk(x, None, 1, 1, 1, 1.0, idx, prob)
+    val, ridx = torch.topk(x, 4, dim=-1)
+    assert torch.equal(idx, ridx)
+    assert torch.allclose(prob, torch.sigmoid(val), atol=1e-6, equal_nan=True) and int(prob.isnan().sum()) == 1
