@@ -82,9 +82,38 @@ class EmulatedCluster:
         return [(outs[r], dtok[r], dprob[r], routing[r][0], routing[r][1]) for r in range(self.world)]
 
     @torch.no_grad()
-    def forward_fp8(self, tokens: List[torch.Tensor], routing=None):
+    def infer(self, tokens: List[torch.Tensor], routing=None):
+        """bf16 inference forward of every rank with the kernels that a layer's own forward picks without autograd (each
+        rank by its own batch).  Returns (outputs, routing)."""
+        L, K = self.layers, self.cfg.top_k
+        if routing is None:
+            routing = [l.route_tokens(t) for l, t in zip(L, tokens)]
+        n = [t.shape[0] for t in tokens]
+        narrow = [l.rt.use_narrow(m * K) for l, m in zip(L, n)]
+        outs = [torch.empty_like(t) for t in tokens]
+        for l, (idx, _), m in zip(L, routing, n):
+            l.rt.publish(idx.data_ptr(), m * K)
+        for l in L:
+            l.rt.solve()
+        for l, (idx, _), m in zip(L, routing, n):
+            l.rt.route(idx.data_ptr(), m * K)
+        for l, t, (_, p), m in zip(L, tokens, routing, n):
+            l.rt.dispatch_tokens(t.data_ptr(), p.data_ptr(), m * K, zero_pad=False)
+        for l in L:
+            l.rt.pull_weights()
+        for l, few in zip(L, narrow):
+            l.rt.gemm1(train=False, narrow=few)
+        for l, few in zip(L, narrow):
+            l.rt.gemm2(narrow=few)
+        for l, o, m in zip(L, outs, n):
+            l.rt.reduce_out(o.data_ptr(), m)
+        return outs, routing
+
+    @torch.no_grad()
+    def forward_fp8(self, tokens: List[torch.Tensor], routing=None, general: bool = True):
         """Inference forward of every rank with block-scaled fp8 expert GEMMs (``MoEConfig.fp8_inference``;
-        call ``quantize_weights()`` on every layer first).  Returns (outputs, routing)."""
+        call ``quantize_weights()`` on every layer first).  ``general``: the wide GEMMs with the activation as a pass of its
+        own; otherwise the kernels that a layer's own forward picks.  Returns (outputs, routing)."""
         L, K = self.layers, self.cfg.top_k
         if routing is None:
             routing = [l.route_tokens(t) for l, t in zip(L, tokens)]
@@ -100,11 +129,14 @@ class EmulatedCluster:
             l.rt.dispatch_fp8(t.data_ptr(), m * K)
         for l in L:
             l.rt.pull_weights_fp8()
-        for l in L:
-            l.rt.gemm1_fp8()
-            l.rt.act_fp8()
-        for l in L:
-            l.rt.gemm2_fp8()
+        narrow = [not general and l.rt.use_narrow_fp8(m * K) for l, m in zip(L, n)]
+        for l, few in zip(L, narrow):
+            act = not general and not few and self.cfg.gemm_ctas == 2
+            l.rt.gemm1_fp8(narrow=few, act=act)
+            if not few and not act:
+                l.rt.act_fp8()
+        for l, few in zip(L, narrow):
+            l.rt.gemm2_fp8(narrow=few)
         for l, (_, p), o, m in zip(L, routing, outs, n):
             l.rt.reduce_out(o.data_ptr(), m, False, p.data_ptr())
         return outs, routing

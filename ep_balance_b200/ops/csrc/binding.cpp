@@ -558,13 +558,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("publish", [](MoeRuntime& r, uint64_t idx, int u) { r.publish((const int64_t*)cp(idx), u, current_stream()); })
       .def("solve", [](MoeRuntime& r) { r.solve(current_stream()); })
       .def("route", [](MoeRuntime& r, uint64_t idx, int u) { r.route((const int64_t*)cp(idx), u, current_stream()); })
-      .def("dispatch_tokens", [](MoeRuntime& r, uint64_t tok, uint64_t prob, int u) {
-        r.dispatch_tokens(cp(tok), (const float*)cp(prob), u, current_stream());
-      })
+      .def("dispatch_tokens", [](MoeRuntime& r, uint64_t tok, uint64_t prob, int u, bool zero_pad) {
+        r.dispatch_tokens(cp(tok), (const float*)cp(prob), u, current_stream(), zero_pad);
+      }, py::arg("tokens"), py::arg("topk_prob"), py::arg("num_units"), py::arg("zero_pad") = true)
       .def("pull_weights", [](MoeRuntime& r) { r.pull_weights(current_stream()); })
       .def("barrier", [](MoeRuntime& r, int slot) { r.barrier(slot, current_stream()); })
-      .def("gemm1", [](MoeRuntime& r) { r.gemm1(current_stream()); })
-      .def("gemm2", [](MoeRuntime& r) { r.gemm2(current_stream()); })
+      .def("use_narrow", &MoeRuntime::use_narrow)
+      .def("use_narrow_fp8", &MoeRuntime::use_narrow_fp8)
+      .def("gemm1", [](MoeRuntime& r, bool train, bool narrow) { r.gemm1(current_stream(), train, narrow); },
+           py::arg("train") = true, py::arg("narrow") = false)
+      .def("gemm2", [](MoeRuntime& r, bool narrow) { r.gemm2(current_stream(), narrow); }, py::arg("narrow") = false)
       .def("gemm1_fused", [](MoeRuntime& r, uint64_t tok, uint64_t prob, int u) {
         r.gemm1_fused(cp(tok), (const float*)cp(prob), u, current_stream());
       })
@@ -587,9 +590,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("quantize_own_weights", [](MoeRuntime& r) { r.quantize_own_weights(current_stream()); })
       .def("pull_weights_fp8", [](MoeRuntime& r) { r.pull_weights_fp8(current_stream()); })
       .def("dispatch_fp8", [](MoeRuntime& r, uint64_t tok, int u) { r.dispatch_fp8(cp(tok), u, current_stream()); })
-      .def("gemm1_fp8", [](MoeRuntime& r) { r.gemm1_fp8(current_stream()); })
+      .def("gemm1_fp8", [](MoeRuntime& r, bool narrow, bool act) { r.gemm1_fp8(current_stream(), narrow, act); },
+           py::arg("narrow") = false, py::arg("act") = false)
       .def("act_fp8", [](MoeRuntime& r) { r.act_fp8(current_stream()); })
-      .def("gemm2_fp8", [](MoeRuntime& r) { r.gemm2_fp8(current_stream()); })
+      .def("gemm2_fp8", [](MoeRuntime& r, bool narrow) { r.gemm2_fp8(current_stream(), narrow); }, py::arg("narrow") = false)
       .def("forward_fp8", [](MoeRuntime& r, uint64_t tok, uint64_t idx, uint64_t prob, uint64_t out, int n) {
         whole_pass(n, {tok, idx, prob, out});
         r.forward_fp8(cp(tok), (const int64_t*)cp(idx), (const float*)cp(prob), mp(out), n, current_stream());

@@ -348,6 +348,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
 // An inference batch with few rows per expert reads the weights once and does little else.  (About num_units rows reach
 // every rank: the plan keeps the ranks near the mean.)
 bool MoeRuntime::use_narrow(int num_units) const { return num_units <= kNarrowRowsPerSlot * cfg_.w_slots; }
+bool MoeRuntime::use_narrow_fp8(int num_units) const { return num_units < kNarrowFp8RowsPerSlot * cfg_.w_slots; }
 
 void MoeRuntime::gemm1(cudaStream_t stream, bool train, bool narrow) {
   GemmExtra x;
@@ -532,8 +533,7 @@ void MoeRuntime::forward_fp8(const void* tokens, const int64_t* topk_idx, const 
                              int num_tokens, cudaStream_t stream) {
   if (!fp8_) throw std::runtime_error("MoeRuntime: fp8 regions were not provided");
   const int U = num_tokens * cfg_.topk;
-  // about U rows reach this rank; with few rows per expert the weights' bytes bound the launch (narrow_gemm_fp8.h)
-  const bool narrow = U < kNarrowFp8RowsPerSlot * cfg_.w_slots;
+  const bool narrow = use_narrow_fp8(U);
   publish(topk_idx, U, stream);
   solve(stream);
   route(topk_idx, U, stream);

@@ -92,6 +92,10 @@ class MoeRuntime {
   void forward_fp8(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out, int num_tokens,
                    cudaStream_t stream);
 
+  // Which kernels an inference pass of num_units routed units takes (each rank decides from its own).
+  bool use_narrow(int num_units) const;
+  bool use_narrow_fp8(int num_units) const;
+
   // ---- whole passes
   void forward(const void* tokens, const int64_t* topk_idx, const float* topk_prob, void* out, int num_tokens,
                cudaStream_t stream, bool train = true);
@@ -137,7 +141,6 @@ class MoeRuntime {
   CommArgs comm_backward(const void* dout) const;
   void swiglu_pass(cudaStream_t stream);
   float* fused_accum(const char* name) const;
-  bool use_narrow(int num_units) const;
   bool peers() const { return cfg_.multi_rank_sync && cfg_.R > 1; }
   UnitReduceWait reduce_wait(int slot) const;
   void tmap2(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t bc, uint32_t br);
