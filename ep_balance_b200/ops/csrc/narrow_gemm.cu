@@ -220,6 +220,10 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tc_fence_after();
         const uint32_t d0 = tmem_base + (uint32_t)(buf * 2 * NT), d1 = d0 + NT;
         const uint32_t idesc = make_idesc(kAMn, false, max(16, round_up(t.n, 16)), BM);
+        if (args.trace != nullptr && local == 0) {
+          // profiling aid: when did the first tile of the launch have its operands? (the wait repeats below)
+          if (mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) atomicMin(args.trace + 3, globaltimer_ns());
+        }
         bool failed = false;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) {
@@ -246,6 +250,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           }
         }
         if (failed) break;
+        if (args.trace != nullptr) atomicMax(args.trace + 2, globaltimer_ns());
         umma_commit(&acc_full[buf]);
       }
     }
@@ -253,8 +258,11 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   } else if (kComm != 0 && warp >= NUM_THREADS / 32) {
     // ------------------------------------------------------------ transport (warps 10, 11)
     const int w = warp - NUM_THREADS / 32;
+    if (args.trace != nullptr && lane == 0) atomicMin(args.trace, globaltimer_ns());
     comm_run<COMM_SLOTS>(args.comm, (int)blockIdx.x * COMM_WARPS + w, (int)gridDim.x * COMM_WARPS,
-                         stage_tiles + 2 * kStageHalfBytes + w * comm_warp_bytes<COMM_SLOTS>(), args.status);
+                         stage_tiles + 2 * kStageHalfBytes + w * comm_warp_bytes<COMM_SLOTS>(), args.status,
+                         args.trace != nullptr ? args.trace + 8 : nullptr);
+    if (args.trace != nullptr && lane == 0) atomicMax(args.trace + 1, globaltimer_ns());
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     // Lane = output feature (TMEM lane), column = token.  Four warps (one half) cover 128 features; kFwd1 splits a tile's

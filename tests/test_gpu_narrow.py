@@ -120,3 +120,20 @@ def test_inference_forward_both_sides_of_the_rule(tokens, experts, fused_comm):
     layer.check_status()
     for g in (tok.grad, layer.w1.grad, layer.w2.grad):
         assert torch.isfinite(g.float()).all()
+
+
+@pytest.mark.parametrize("tokens", [65, 700])
+def test_fused_trace_of_an_inference_forward(tokens, monkeypatch):
+    """The profiling aid sees the transport and the GEMM on both sides of the rule."""
+    from ep_balance_b200.models.emulated import EmulatedCluster
+    from ep_balance_b200.models.moe_layer import MoEConfig
+
+    monkeypatch.setenv("EPLB_TRACE_FUSED", "1")
+    layer = EmulatedCluster(MoEConfig(hidden=320, ffn=384, num_experts=8, top_k=2, max_tokens=700), world=1).layers[0]
+    layer.fused_trace_reset()
+    with torch.no_grad():
+        layer(torch.randn(tokens, 320, device="cuda").bfloat16())
+    layer.check_status()
+    trace = layer.fused_trace()
+    assert 0 < trace["fwd_first_tile_us"] <= trace["fwd_mma_end_us"] < 1e5 and 0 < trace["fwd_transport_us"] < 1e5
+    assert trace["fwd_warp_segments"] > 0
