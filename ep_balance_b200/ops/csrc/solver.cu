@@ -1,5 +1,5 @@
-// On-device plan solver: one cooperative launch computes placement x, routing quota q and
-// the per-rank routing tables, with no host decision and no q memset.
+// On-device plan solver: placement x, routing quota q and the per-rank routing tables, with no host decision
+// and no q memset, in one launch (three where routing is most of the work).
 //
 // Semantics (must equal solver/device_semantics.py element for element; they restate the
 // reference's CUDA path, eplb/cuda_solve.py:36-68 and eplb/csrc/fast_solver.cu:34-643):
@@ -12,6 +12,7 @@
 // ranks, the domain's quota columns fit in shared memory) a CTA routes exactly its own domain's columns
 // straight into the shared-memory state the repair loop works on, so phases 1 and 2 need no barrier and no
 // cache fill between them; walks that cannot change anything (no free slot left, nothing movable) stop early.
+// Larger quotas are routed by a launch of many CTAs between placement and repair, with no barrier at all.
 #include "solver.h"
 
 #include <cooperative_groups.h>
@@ -24,6 +25,7 @@ namespace epb {
 namespace {
 
 constexpr int kWarp = 32;
+constexpr int kRouteThreads = 512;  // CTA of the routing launch
 constexpr unsigned kFull = 0xffffffffu;
 
 struct Cand {
@@ -335,19 +337,28 @@ __device__ __forceinline__ int even_share(int need, unsigned long long act, int 
   return pos < n ? need / n + (pos < need % n ? 1 : 0) : 0;
 }
 
-// R <= 64: one thread per (src, e) pair writes its row of q, one thread per (e, dst) pair sums
-// erl; host sets are 64-bit masks held in shared memory.  Every pair is independent, so the whole
-// grid works on them at once instead of one warp walking an expert's sources serially.
-__device__ void phase1_routing_masks(const SolverParams& p, Smem& s) {
-  __shared__ unsigned long long dom_mask[64];
-  const int R = p.R, E = p.E, u_min = p.u_min;
+// Host sets of every expert and the members of every rank's domain as 64-bit masks (R <= 64), by the whole CTA.
+__device__ void host_masks(const SolverParams& p, unsigned long long* host, unsigned long long* dom_mask) {
+  const int R = p.R, E = p.E;
   const int tid = threadIdx.x, nt = blockDim.x;
-  unsigned long long* host = reinterpret_cast<unsigned long long*>(s.prio);  // [E]
-  __syncthreads();
-  for (int e = tid; e < E; e += nt) {
-    unsigned long long m = 0;
-    for (int dst = 0; dst < R; ++dst) m |= (unsigned long long)(p.x[(size_t)e * R + dst] != 0) << dst;
-    host[e] = m;
+  if ((R & 7) == 0) {
+    // a row of x is R bytes, 8-byte aligned: eight hosts per load
+    for (int e = tid; e < E; e += nt) {
+      unsigned long long m = 0;
+      const unsigned long long* row = reinterpret_cast<const unsigned long long*>(p.x + (size_t)e * R);
+      for (int w = 0; w < R / 8; ++w) {
+        const unsigned long long v = row[w];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) m |= (unsigned long long)(((v >> (8 * b)) & 0xffull) != 0) << (8 * w + b);
+      }
+      host[e] = m;
+    }
+  } else {
+    for (int e = tid; e < E; e += nt) {
+      unsigned long long m = 0;
+      for (int dst = 0; dst < R; ++dst) m |= (unsigned long long)(p.x[(size_t)e * R + dst] != 0) << dst;
+      host[e] = m;
+    }
   }
   for (int r = tid; r < R; r += nt) {
     unsigned long long m = 0;
@@ -355,16 +366,27 @@ __device__ void phase1_routing_masks(const SolverParams& p, Smem& s) {
     for (int o = 0; o < R; ++o) m |= (unsigned long long)(p.dom[o] == dr) << o;
     dom_mask[r] = m;
   }
+}
+
+// R <= 64: every (src, e) pair's row of q and every (e, dst) pair's sum, shared out over the grid; host sets are 64-bit
+// masks in shared memory (`host`: [E]).  Every pair is independent.
+__device__ void phase1_routing_masks(const SolverParams& p, unsigned long long* host) {
+  __shared__ unsigned long long dom_mask[64];
+  const int R = p.R, E = p.E, u_min = p.u_min;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  __syncthreads();
+  host_masks(p, host, dom_mask);
   __syncthreads();
   const int gtid = blockIdx.x * nt + tid, gthreads = gridDim.x * nt;
-  // a warp per pair: its row of q leaves as whole 128-byte lines
-  for (int pair = gtid / kWarp; pair < R * E; pair += gthreads / kWarp) {
+  // as many threads per pair as its row has entries (at most a warp): the row of q leaves as whole lines
+  const int width = min(pow2_at_least(R), kWarp), sub = tid & (width - 1);
+  for (int pair = gtid / width; pair < R * E; pair += gthreads / width) {
     const int src = pair / E, e = pair - src * E;
     const int need = p.omega[pair];
     const unsigned long long loc = host[e] & dom_mask[src];
     const unsigned long long act = loc ? loc : host[e];
     int* qrow = p.q + (size_t)pair * R;
-    for (int dst = tid & (kWarp - 1); dst < R; dst += kWarp) qrow[dst] = ((act >> dst) & 1ull) ? even_share(need, act, dst, u_min) : 0;
+    for (int dst = sub; dst < R; dst += width) qrow[dst] = ((act >> dst) & 1ull) ? even_share(need, act, dst, u_min) : 0;
   }
   for (int cell = gtid; cell < E * R; cell += gthreads) {
     const int e = cell / R, dst = cell - e * R;
@@ -453,31 +475,7 @@ __device__ void phase1_domain(const SolverParams& p, Smem& s, int d, int n_known
   const int n = n_known >= 0 ? n_known : collect_domain(p, s, d);
   if (n == 0) return;
   unsigned long long* host = reinterpret_cast<unsigned long long*>(s.prio);  // [E]
-  if ((R & 7) == 0) {
-    // a row of x is R bytes, 8-byte aligned: eight hosts per load
-    for (int e = tid; e < E; e += nt) {
-      unsigned long long m = 0;
-      const unsigned long long* row = reinterpret_cast<const unsigned long long*>(p.x + (size_t)e * R);
-      for (int w = 0; w < R / 8; ++w) {
-        const unsigned long long v = row[w];
-#pragma unroll
-        for (int b = 0; b < 8; ++b) m |= (unsigned long long)(((v >> (8 * b)) & 0xffull) != 0) << (8 * w + b);
-      }
-      host[e] = m;
-    }
-  } else {
-    for (int e = tid; e < E; e += nt) {
-      unsigned long long m = 0;
-      for (int dst = 0; dst < R; ++dst) m |= (unsigned long long)(p.x[(size_t)e * R + dst] != 0) << dst;
-      host[e] = m;
-    }
-  }
-  for (int r = tid; r < R; r += nt) {
-    unsigned long long m = 0;
-    const int dr = p.dom[r];
-    for (int o = 0; o < R; ++o) m |= (unsigned long long)(p.dom[o] == dr) << o;
-    dom_mask[r] = m;
-  }
+  host_masks(p, host, dom_mask);
   // clear the caches while those loads are in flight (q_c and erl_c are contiguous ints; x_c is written below)
   {
     const int q_ints = R * E * n, e_ints = E * n;
@@ -970,12 +968,10 @@ __device__ __forceinline__ void trace_mark(const SolverParams& p, int slot) {
   if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[slot] = (int64_t)globaltimer_ns();
 }
 
-__global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables tables) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem s = carve(smem_raw, p.R, p.E);
-  trace_mark(p, 0);
-
-  // Wait (bounded) until every rank's row of omega has landed in the gather buffer.
+// Wait (bounded) until every rank's row of omega has landed in the gather buffer, and check that every rank belongs to one
+// of the D domains: a plan solved with an out-of-range id would leave that rank's load unset.  Every CTA evaluates the same
+// input and fails the same bounded wait, so all of them get the same answer.
+__device__ bool inputs_ready(const SolverParams& p) {
   if (p.omega_signal != nullptr) {
     __shared__ int sig_ok;
     if (threadIdx.x == 0) {
@@ -983,23 +979,56 @@ __global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables
       if (!sig_ok) set_status(p.status, kStatusSignalTimeout, 10);
     }
     __syncthreads();
-    if (!sig_ok) return;  // every CTA fails the same bounded wait; nobody is left at a barrier
+    if (!sig_ok) return false;
   }
+  __shared__ int bad_rank;
+  if (threadIdx.x == 0) bad_rank = -1;
+  __syncthreads();
+  for (int r = threadIdx.x; r < p.R; r += blockDim.x)
+    if (p.dom[r] < 0 || p.dom[r] >= p.D) bad_rank = r;
+  __syncthreads();
+  if (bad_rank >= 0) {
+    if (threadIdx.x == 0) set_status(p.status, kStatusBadArgument, 13, bad_rank);
+    return false;
+  }
+  return true;
+}
 
-  // Every rank must belong to one of the D domains; a plan solved with an out-of-range id would leave that
-  // rank's load unset.  Every CTA evaluates the same input, so all of them return together.
-  {
-    __shared__ int bad_rank;
-    if (threadIdx.x == 0) bad_rank = -1;
-    __syncthreads();
-    for (int r = threadIdx.x; r < p.R; r += blockDim.x)
-      if (p.dom[r] < 0 || p.dom[r] >= p.D) bad_rank = r;
-    __syncthreads();
-    if (bad_rank >= 0) {
-      if (threadIdx.x == 0) set_status(p.status, kStatusBadArgument, 13, bad_rank);
-      return;
+// No barrier before the tail: every CTA publishes its results and counts itself out; the LAST one to leave sees
+// all domains' results, so it computes theta, builds the routing tables and rewinds the barrier counters.
+__device__ void finish(const SolverParams& p, const RankTables& tables, bool ok, bool theta_by_atomics) {
+  __shared__ int last_out;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last_out = 1;
+    if (gridDim.x > 1) {
+      __threadfence();
+      last_out = atomicAdd(p.sync + 1, 1u) == gridDim.x - 1 ? 1 : 0;
+      __threadfence();
     }
   }
+  __syncthreads();
+  if (!last_out) return;
+  if (ok && (gridDim.x == 1 || *reinterpret_cast<volatile int*>(p.status) == 0)) {
+    if (!theta_by_atomics && threadIdx.x < kWarp) {
+      const int th = global_theta_warp(p);
+      if (threadIdx.x == 0) p.theta[0] = th;
+    }
+    if (tables.me >= 0) build_tables(p, tables, tables.me);
+  }
+  if (threadIdx.x == 0) {
+    p.sync[0] = 0;
+    p.sync[1] = 0;
+    __threadfence();
+  }
+  if (p.trace != nullptr && threadIdx.x == 0) p.trace[6] = (int64_t)globaltimer_ns();
+}
+
+__global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables tables) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem s = carve(smem_raw, p.R, p.E);
+  trace_mark(p, 0);
+  if (!inputs_ready(p)) return;  // (in every CTA: nobody is left at a barrier)
 
   bool ok = true;
   trace_mark(p, 1);
@@ -1029,7 +1058,7 @@ __global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables
   ok = ok && grid_barrier(p, 11);
   trace_mark(p, 3);
   if (ok && !own_columns) {
-    if (p.R <= 64) phase1_routing_masks(p, s);
+    if (p.R <= 64) phase1_routing_masks(p, reinterpret_cast<unsigned long long*>(s.prio));
     else phase1_routing(p);
   }
   if (!own_columns) ok = ok && grid_barrier(p, 12);
@@ -1082,33 +1111,33 @@ __global__ void __launch_bounds__(1024) solver_kernel(SolverParams p, RankTables
       }
     }
   }
-  // No barrier before the tail: every CTA publishes its results and counts itself out; the LAST one to leave sees
-  // all domains' results, so it computes theta, builds the routing tables and rewinds the barrier counters.
-  __shared__ int last_out;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    last_out = 1;
-    if (gridDim.x > 1) {
-      __threadfence();
-      last_out = atomicAdd(p.sync + 1, 1u) == gridDim.x - 1 ? 1 : 0;
-      __threadfence();
-    }
+  finish(p, tables, ok, theta_by_atomics);
+}
+
+// The same plan as three launches, where routing is too much for one CTA per domain: placement (a CTA per domain), routing
+// (any number of CTAs), repair and tables (a CTA per domain).  No CTA waits for another one, so none of them has to be
+// resident together: a plan starts beside a GEMM that leaves it a single SM.  sync[0] is 1 from a placement that found its
+// inputs unfit to the end of the repair.
+__global__ void __launch_bounds__(1024) solver_place_kernel(SolverParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem s = carve(smem_raw, p.R, p.E);
+  if (!inputs_ready(p)) {
+    if (threadIdx.x == 0) atomicOr(p.sync, 1u);
+    return;
   }
-  __syncthreads();
-  if (!last_out) return;
-  if (ok && (gridDim.x == 1 || *reinterpret_cast<volatile int*>(p.status) == 0)) {
-    if (!theta_by_atomics && threadIdx.x < kWarp) {
-      const int th = global_theta_warp(p);
-      if (threadIdx.x == 0) p.theta[0] = th;
-    }
-    if (tables.me >= 0) build_tables(p, tables, tables.me);
-  }
-  if (threadIdx.x == 0 && gridDim.x > 1) {
-    p.sync[0] = 0;
-    p.sync[1] = 0;
-    __threadfence();
-  }
-  if (p.trace != nullptr && threadIdx.x == 0) p.trace[6] = (int64_t)globaltimer_ns();
+  for (int d = blockIdx.x; d < p.D; d += gridDim.x) phase0_domain(p, s, d);
+}
+__global__ void __launch_bounds__(kRouteThreads) solver_route_kernel(SolverParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (*p.sync == 0u) phase1_routing_masks(p, reinterpret_cast<unsigned long long*>(smem_raw));
+}
+__global__ void __launch_bounds__(1024) solver_repair_kernel(SolverParams p, RankTables tables) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem s = carve(smem_raw, p.R, p.E);
+  const bool ok = *p.sync == 0u;
+  if (ok)
+    for (int d = blockIdx.x; d < p.D; d += gridDim.x) stage2_domain(p, s, d, p.iters, ProbeState{false, 0}, true);
+  finish(p, tables, ok, false);
 }
 
 // One rank has nothing to decide: every expert stays where it lives, and the outputs are the load row, its sum and the
@@ -1210,12 +1239,26 @@ size_t solver_base_smem(int R, int E) {
 size_t solver_cache_smem(int R, int E) { return (((size_t)E * R * 5 + 15) / 16) * 16; }  // erl (int) + x (byte) per (e, rank)
 size_t solver_qcache_smem(int R, int E) { return (size_t)R * E * R * 4; }
 constexpr size_t kCacheBudget = 200 * 1024;
+constexpr int kSplitPairs = 1024;  // (source, expert) pairs from which a plan is three launches (launch_solver)
 
 int pow2_threads(int R, int E) {
   int want = E > R ? E : R;
   int t = 256;
   while (t < want && t < 1024) t <<= 1;
   return t;
+}
+
+// The dynamic shared-memory limit is an attribute of (kernel, device): raised per device, only when needed.
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, size_t smem, int dev, int which) {
+  constexpr int kMaxDevices = 64;
+  static size_t configured[3][kMaxDevices] = {};
+  const bool tracked = dev >= 0 && dev < kMaxDevices;
+  const size_t have = tracked && configured[which][dev] ? configured[which][dev] : 48 * 1024;
+  if (smem <= (tracked ? have : (size_t)48 * 1024)) return cudaSuccess;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err == cudaSuccess && tracked) configured[which][dev] = smem;
+  return err;
 }
 
 }  // namespace
@@ -1237,27 +1280,27 @@ cudaError_t launch_solver(const SolverParams& p, const RankTables& tables, cudaS
   pc.cache_stage2 = base + solver_cache_smem(p.R, p.E) <= kCacheBudget ? 1 : 0;
   pc.cache_q = pc.cache_stage2 && base + solver_cache_smem(p.R, p.E) + solver_qcache_smem(p.R, p.E) <= kCacheBudget ? 1 : 0;
   const size_t smem = base + (pc.cache_stage2 ? solver_cache_smem(p.R, p.E) : 0) + (pc.cache_q ? solver_qcache_smem(p.R, p.E) : 0);
-  // The dynamic shared-memory limit is an attribute of (kernel, device): raise it per device, only when needed.
-  constexpr int kMaxDevices = 64;
-  static size_t configured_smem[kMaxDevices] = {};
-  const bool tracked = dev >= 0 && dev < kMaxDevices;
-  const size_t have = tracked && configured_smem[dev] ? configured_smem[dev] : 48 * 1024;
-  if (smem > have || (!tracked && smem > 48 * 1024)) {
-    err = cudaFuncSetAttribute(solver_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    if (tracked) configured_smem[dev] = smem;
-  }
   int grid = p.D < sms ? p.D : sms;
   if (grid < 1) grid = 1;
-  // Where the quotas do not fit in shared memory the whole grid shares out the routing phase (R * E * R quotas and E * R
-  // sums over R sources), which one CTA per domain spends most of the kernel on; the extra CTAs only take part in that
-  // phase, four (source, expert) pairs per warp.  64 ranks, 256 experts: kernel and casts 379 -> 223 us with the coalesced
-  // rows of q and the moves' single round trip.
-  const bool own_columns = pc.cache_q && p.u_min == 1 && p.R <= 64 && grid >= p.D && !p.probe;
-  if (!own_columns && p.R <= 64) {
-    const int want = ceil_div(p.R * p.E, 1024 / kWarp * 4);
-    grid = want > sms ? sms : want > grid ? want : grid;
+  // Quotas that fit in shared memory (cache_q, u_min 1): each domain's CTA routes its own columns.  Otherwise the routing phase
+  // (R * E * R quotas and E * R sums over R sources) is up to half of a plan, and has a launch of its own, four pairs per warp.
+  // us a call, one launch of a CTA per domain / three launches (R x E, domains; * u_min 2):
+  //   8 x 64, 2 *   78.6 /  80.6     16 x 128, 2 *   270 / 237     16 x 256, 2   177 / 103
+  //   8 x 64, 1 *  136.3 / 140.1     16 x 128, 1 *   339 / 266     64 x  64, 8   215 / 189
+  //  16 x 64, 2 *    151 / 135       16 x 192, 2     242 / 197     64 x 256, 8   423 / 241
+  const bool own_columns = pc.cache_q && p.u_min == 1 && p.R <= 64 && !p.probe;
+  const size_t masks = sizeof(unsigned long long) * (size_t)p.E;
+  if (!own_columns && !p.probe && p.trace == nullptr && p.R <= 64 && p.R * p.E >= kSplitPairs && masks <= 40 * 1024) {
+    if ((err = allow_smem(solver_place_kernel, smem, dev, 0)) != cudaSuccess) return err;
+    if ((err = allow_smem(solver_repair_kernel, smem, dev, 1)) != cudaSuccess) return err;
+    const int per_cta = kRouteThreads / kWarp * 4;  // (source, expert) pairs
+    const int want = ceil_div(p.R * p.E, per_cta);
+    solver_place_kernel<<<grid, threads, smem, stream>>>(pc);
+    solver_route_kernel<<<want < 2 * sms ? want : 2 * sms, kRouteThreads, masks, stream>>>(pc);
+    solver_repair_kernel<<<grid, threads, smem, stream>>>(pc, tables);
+    return cudaGetLastError();
   }
+  if ((err = allow_smem(solver_kernel, smem, dev, 2)) != cudaSuccess) return err;
   RankTables tc = tables;
   void* args[] = {&pc, &tc};
   if (grid > 1) return cudaLaunchCooperativeKernel((void*)solver_kernel, dim3(grid), dim3(threads), args, smem, stream);
