@@ -157,7 +157,7 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
   CUtensorMap tmA, tmB;
   const uint64_t T = a.size(0);
   const uint32_t box_rows = narrow ? epb::kNarrowBoxRows : 128;  // token rows of a box
-  TORCH_CHECK(!narrow || mode == epb::kFwd1 || mode == epb::kFwd2 || mode == epb::kDgrad1, "the narrow kernel has modes fwd1, fwd2 and dgrad1");
+  TORCH_CHECK(!narrow || mode == epb::kFwd1 || mode == epb::kFwd2, "the narrow kernel has modes fwd1 and fwd2");
   bool ok = true;
   switch (mode) {
     case epb::kPlain:
@@ -177,7 +177,7 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
     case epb::kDgrad2:
       g.N = (int)b.size(2);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, 128) &&
            epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 64);
       break;
     case epb::kWgrad:

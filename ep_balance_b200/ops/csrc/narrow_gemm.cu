@@ -9,9 +9,8 @@
 // rows each: GEMM1 141 us (805 MB of weights: 5.7 TB/s) against 203, GEMM2 71 (5.7 TB/s) against 124.  Four 48 KB
 // stages keep 128 KB of weights in flight per SM; pairing SMs would halve the token bytes only, which are few.
 //
-//   kFwd1    act = SwiGLU(X W1^T) (and, for training, the pre-activations h)   gate block + up block of a tile
+//   kFwd1    act = SwiGLU(X W1^T)   gate block + up block of a tile
 //   kFwd2    y = act W2^T, rows scattered to their sources
-//   kDgrad1  C = A W (weights MN-major): local rows or scattered to their sources
 //
 // Warps as in grouped_gemm.cu: 0 TMA producer, 1 tensor memory + MMA issue, 2-9 epilogue, 10-11 transport (kComm).
 // Every mbarrier wait is bounded; on a timeout the CTA raises its abort flag, records a status, lets issued copies
@@ -69,14 +68,14 @@ __device__ __forceinline__ bool find_tile(const GemmArgs& a, int n_groups, const
 }
 
 // Write 32 token rows x 128 features (256 B per row) staged by the four warps of a half: two rows per instruction.
-// `mine` is the lane's own token's row pointer (null: not stored); lane = token of the chunk, the same in all four warps.
-__device__ __forceinline__ void flush_rows(const uint4* tile, int quarter, int lane, char* mine, int byte_off, int pieces) {
+// `mine` is where the lane's own token's features go (null: not stored); lane = token of the chunk, the same in all four warps.
+__device__ __forceinline__ void flush_rows(const uint4* tile, int quarter, int lane, char* mine, int pieces) {
   const unsigned long long p = reinterpret_cast<unsigned long long>(mine);
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int tok = quarter * 8 + it * 2 + (lane >> 4), piece = lane & 15;
     const unsigned long long base = __shfl_sync(0xffffffffu, p, tok);
-    if (base != 0ull && piece < pieces) *reinterpret_cast<uint4*>(base + byte_off + piece * 16) = tile[tok * 16 + piece];
+    if (base != 0ull && piece < pieces) *reinterpret_cast<uint4*>(base + piece * 16) = tile[tok * 16 + piece];
   }
 }
 // All four warps of a half agree (and meet): true if `ok` holds in each of them.
@@ -95,13 +94,12 @@ __device__ __forceinline__ bool half_all(int half, bool ok) {
 __device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
 // Stage one value per (token, feature): lane = feature, element j = token.  A warp writes 64 contiguous bytes per token.
 template <typename F>
-__device__ __forceinline__ void stage_and_flush(__nv_bfloat16* stg, int half, int quarter, int lane, char* mine, int byte_off,
-                                                int pieces, F value) {
+__device__ __forceinline__ void stage_and_flush(__nv_bfloat16* stg, int half, int quarter, int lane, char* mine, int pieces, F value) {
   half_sync(half);  // the previous flush has read the tile
 #pragma unroll
   for (int j = 0; j < 32; ++j) stg[j * BM + quarter * 32 + lane] = value(j);
   half_sync(half);
-  flush_rows(reinterpret_cast<const uint4*>(stg), quarter, lane, mine, byte_off, pieces);
+  flush_rows(reinterpret_cast<const uint4*>(stg), quarter, lane, mine, pieces);
 }
 
 template <int kMode, int kComm>
@@ -109,7 +107,6 @@ __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1
 narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                    const __grid_constant__ GemmArgs args) {
   constexpr int STAGES = stages<kComm>();
-  constexpr bool kAMn = kMode == kDgrad1;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -187,14 +184,10 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           uint8_t* sB = sA + A_BYTES;
           uint64_t* fb = &full_bar[stage];
           mbar_expect_tx(fb, (two ? A_BYTES : A_BYTES / 2) + boxes * BOX_N * BK * 2);
-          if (kAMn) {
-            for (int j = 0; j < (two ? 4 : 2); ++j) tma_load_3d(sA + j * 8192, &tmW, fb, t.mt * 2 * BM + 64 * j, kb * BK, t.wslot);
-          } else {
-            const int m0 = kMode == kFwd1 ? t.mt * BM : t.mt * 2 * BM;
-            const int m1 = kMode == kFwd1 ? args.N + t.mt * BM : m0 + BM;
-            tma_load_3d(sA, &tmW, fb, kb * BK, m0, t.wslot);
-            if (two) tma_load_3d(sA + A_BYTES / 2, &tmW, fb, kb * BK, m1, t.wslot);
-          }
+          const int m0 = kMode == kFwd1 ? t.mt * BM : t.mt * 2 * BM;
+          const int m1 = kMode == kFwd1 ? args.N + t.mt * BM : m0 + BM;
+          tma_load_3d(sA, &tmW, fb, kb * BK, m0, t.wslot);
+          if (two) tma_load_3d(sA + A_BYTES / 2, &tmW, fb, kb * BK, m1, t.wslot);
           for (int j = 0; j < boxes; ++j) tma_load_2d(sB + j * BOX_N * BK * 2, &tmX, fb, kb * BK, t.row + j * BOX_N);
           if (++stage == STAGES) {
             stage = 0;
@@ -219,7 +212,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         acc_phase[buf] ^= 1u;
         tc_fence_after();
         const uint32_t d0 = tmem_base + (uint32_t)(buf * 2 * NT), d1 = d0 + NT;
-        const uint32_t idesc = make_idesc(kAMn, false, max(16, round_up(t.n, 16)), BM);
+        const uint32_t idesc = make_idesc(false, false, max(16, round_up(t.n, 16)), BM);
         if (args.trace != nullptr && local == 0) {
           // profiling aid: when did the first tile of the launch have its operands? (the wait repeats below)
           if (mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) atomicMin(args.trace + 3, globaltimer_ns());
@@ -232,16 +225,14 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           }
           tc_fence_after();
           const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES), sB = sA + A_BYTES;
-          const uint64_t da = kAMn ? make_desc(sA, 8192, 1024) : make_desc(sA, 16, 1024);
-          const uint64_t db = make_desc(sB, 16, 1024);
-          constexpr uint32_t a_step = kAMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
-          constexpr uint32_t b_step = (UMMA_K * 2) >> 4;
+          const uint64_t da = make_desc(sA, 16, 1024), db = make_desc(sB, 16, 1024);
+          constexpr uint32_t k_step = (UMMA_K * 2) >> 4;
           constexpr uint32_t a_block = (A_BYTES / 2) >> 4;   // second weight block of the stage
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint32_t acc = (kb | k) ? 1u : 0u;
-            umma_bf16(d0, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
-            if (two) umma_bf16(d1, da + (uint64_t)(a_block + k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
+            umma_bf16(d0, da + (uint64_t)(k * k_step), db + (uint64_t)(k * k_step), idesc, acc);
+            if (two) umma_bf16(d1, da + (uint64_t)(a_block + k * k_step), db + (uint64_t)(k * k_step), idesc, acc);
           }
           umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) {
@@ -297,12 +288,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           tmem_ld32(taddr + c * 32, g);
           tmem_ld32(taddr + NT + c * 32, u);
           tmem_ld_wait();
-          if (out0 != nullptr) {
-            char* hrow = real ? out0 + (row * (size_t)(2 * F) + t.mt * BM) * 2 : nullptr;
-            stage_and_flush(stg, half, quarter, lane, hrow, 0, 16, [&](int j) { return __float2bfloat16_rn(__uint_as_float(g[j])); });
-            stage_and_flush(stg, half, quarter, lane, hrow, F * 2, 16, [&](int j) { return __float2bfloat16_rn(__uint_as_float(u[j])); });
-          }
-          stage_and_flush(stg, half, quarter, lane, arow, 0, 16, [&](int j) {
+          stage_and_flush(stg, half, quarter, lane, arow, 16, [&](int j) {
             // activation from the bf16-rounded pre-activations, exactly as the wide kernel computes it
             const float gr = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[j])));
             const float ur = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j])));
@@ -321,15 +307,15 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
             if (args.meta != nullptr) {
               const int2 mt = args.meta[row];
               char* base = args.out_ptrs ? reinterpret_cast<char*>(args.out_ptrs[mt.x]) : out0;
-              orow = base + (size_t)mt.y * args.N * 2;
+              orow = base + ((size_t)mt.y * args.N + col0) * 2;
             } else {
-              orow = out0 + row * (size_t)args.N * 2;
+              orow = out0 + (row * (size_t)args.N + col0) * 2;
             }
           }
           uint32_t v[32];
           tmem_ld32(taddr + half * NT + c * 32, v);
           tmem_ld_wait();
-          stage_and_flush(stg, half, quarter, lane, orow, col0 * 2, pieces, [&](int j) { return __float2bfloat16_rn(__uint_as_float(v[j])); });
+          stage_and_flush(stg, half, quarter, lane, orow, pieces, [&](int j) { return __float2bfloat16_rn(__uint_as_float(v[j])); });
         }
       }
       tc_fence_before();
@@ -381,13 +367,11 @@ cudaError_t launch_narrow_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, c
                                cudaStream_t stream) {
   if (args.n_groups_cap > MAX_GROUPS || args.K <= 0 || args.K % BK != 0 || args.N % 32 != 0) return cudaErrorInvalidValue;
   if (args.arrive != nullptr && args.arrive_tile_rows <= 0) return cudaErrorInvalidValue;
-  if (args.mode == kFwd1 && args.N % BM != 0) return cudaErrorInvalidValue;
+  if (args.mode == kFwd1 && (args.N % BM != 0 || args.out0 != nullptr)) return cudaErrorInvalidValue;
   const bool comm = args.comm.do_dispatch || args.comm.do_pad || args.comm.do_pull;
   switch (args.mode) {
     case kFwd1: return comm ? launch_mode<kFwd1, 1>(tmW, tmX, args, num_sms, stream) : launch_mode<kFwd1, 0>(tmW, tmX, args, num_sms, stream);
-    case kDgrad1: return comm ? launch_mode<kDgrad1, 1>(tmW, tmX, args, num_sms, stream) : launch_mode<kDgrad1, 0>(tmW, tmX, args, num_sms, stream);
     case kFwd2:
-    case kPlain:
       if (comm) return cudaErrorInvalidValue;
       return launch_mode<kFwd2, 0>(tmW, tmX, args, num_sms, stream);
     default: return cudaErrorInvalidValue;

@@ -1,6 +1,6 @@
 // Grouped GEMM for few rows per expert (narrow_gemm.cu): weights on the M side of the tensor core, token rows on its N
-// side.  Takes the GemmArgs of grouped_gemm.h with mode kFwd1 (out0 may be null: the pre-activations are not kept), kFwd2 or
-// kDgrad1, with or without the fused transport.
+// side.  The inference forward's two GEMMs: GemmArgs of grouped_gemm.h with mode kFwd1 (with or without the fused transport;
+// out0 null, the pre-activations are not kept) or kFwd2.
 #pragma once
 
 #include "grouped_gemm.h"
@@ -19,8 +19,8 @@ constexpr int kNarrowBoxRows = 32;  // token rows of one TMA box: box of the tok
 // tiles of the wide kernel are full enough, and move fewer operand bytes per flop.
 constexpr int kNarrowRowsPerSlot = 128;
 
-// tmW: the weight map that grouped_gemm.h's kernels use as B (K-major box {64, 128, 1} for kFwd1 / kFwd2, MN-major box
-// {64, 64, 1} for kDgrad1); tmX: token rows, 2-D, box {64, kNarrowBoxRows}.
+// tmW: the weight map that grouped_gemm.h's kernels use as B (K-major box {64, 128, 1}); tmX: token rows, 2-D, box
+// {64, kNarrowBoxRows}.
 cudaError_t launch_narrow_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmArgs& args, int num_sms,
                                cudaStream_t stream);
 

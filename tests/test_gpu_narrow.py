@@ -7,7 +7,7 @@ import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
 
-MODE = dict(fwd1=0, fwd2=1, dgrad1=3)
+MODE = dict(fwd1=0, fwd2=1)
 # one row, a partial and a full 16-column step, box and tile edges (32, 128), two and three token tiles, an empty group
 ROWS = [1, 0, 16, 33, 128, 129, 300]
 WSLOT = [3, 0, 6, 1, 2, 5, 4]
@@ -51,42 +51,35 @@ def _operand(T, K):
 
 
 @pytest.mark.parametrize("N,K", [(64, 64), (256, 192), (320, 1408), (2048, 768)])
-@pytest.mark.parametrize("mode", ["fwd2", "dgrad1"])
-def test_plain_rows(mode, N, K):
+def test_plain_rows(N, K):
     torch.manual_seed(0)
     T = _rows_total()
     a = _operand(T, K)
-    w = (torch.randn(7, *((N, K) if mode == "fwd2" else (K, N)), device="cuda") * 0.05).bfloat16()
+    w = (torch.randn(7, N, K, device="cuda") * 0.05).bfloat16()
     out = torch.full((T, N), 7.0, device="cuda").bfloat16()
-    off = _run(mode, a, w, out, None)
+    off = _run("fwd2", a, w, out, None)
     for g, r in enumerate(ROWS):
-        ws = w[WSLOT[g]].float()
-        want = a[off[g]:off[g] + r].float() @ (ws.t() if mode == "fwd2" else ws)
+        want = a[off[g]:off[g] + r].float() @ w[WSLOT[g]].float().t()
         if r:
             assert _rel(out[off[g]:off[g] + r], want) < 4e-3  # one bf16 rounding (2^-9 at most) of an fp32 sum
         assert bool((out[off[g] + r:off[g + 1]] == 7.0).all())
 
 
-@pytest.mark.parametrize("keep_h", [True, False])
 @pytest.mark.parametrize("Fd,K", [(128, 64), (384, 512)])
-def test_swiglu(Fd, K, keep_h):
+def test_swiglu(Fd, K):
     torch.manual_seed(1)
     T = _rows_total()
     a = _operand(T, K)
     w = (torch.randn(7, 2 * Fd, K, device="cuda") * 0.05).bfloat16()
-    h = torch.full((T, 2 * Fd), 3.0, device="cuda").bfloat16()
     act = torch.full((T, Fd), 3.0, device="cuda").bfloat16()
-    off = _run("fwd1", a, w, h if keep_h else h[:0], act)
+    off = _run("fwd1", a, w, act[:0], act)  # (no buffer for the pre-activations)
     for g, r in enumerate(ROWS):
         sl = slice(off[g], off[g] + r)
         hh = a[sl].float() @ w[WSLOT[g]].float().t()
         if r:
-            if keep_h:
-                assert _rel(h[sl], hh) < 4e-3
             gate, up = hh.bfloat16().float().chunk(2, dim=-1)
             assert _rel(act[sl], F.silu(gate) * up) < 1e-2  # three bf16 roundings: gate, up, product
         assert bool((act[off[g] + r:off[g + 1]] == 3.0).all())
-    assert keep_h or bool((h == 3.0).all())
 
 
 @pytest.mark.parametrize("tokens,experts,fused_comm", [(1, 8, True), (65, 16, True), (512, 8, True), (700, 8, True), (65, 16, False)])
