@@ -16,6 +16,7 @@
 
 #include "block_scale.cuh"
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace epb {
 namespace {
@@ -33,98 +34,6 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t kSfCol = 256;                   // scale factors live behind the two accumulators
 static_assert((STAGES * 2 + 4) * 8 + 8 + (MAX_GROUPS + 1) * 4 <= kCtrlBytes, "control block does not fit");
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                          int site) {
-  unsigned long long t0 = 0;
-  for (unsigned spin = 0;; ++spin) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 1023u) == 1023u) {
-      if (*abort_flag) return false;
-      unsigned long long now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kWaitBudgetNs) {
-        *abort_flag = 1;
-        set_status(status, kStatusPipeTimeout, site, (int)blockIdx.x);
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols));
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols));
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptors (version 1).  Operand tiles: K-major, 128-byte swizzle, 8-row groups
-// 1024 B apart.  Scale chunks: no swizzle, 8-row x 16-byte core matrices 128 B apart.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(16 >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 struct Tile {
   int g, mt, nt, rows, row0, wslot;
 };
@@ -145,10 +54,6 @@ __device__ __forceinline__ bool find_tile(const Fp8GemmArgs& a, int n_groups, in
   return true;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
 __device__ __forceinline__ void pack_row(const uint32_t (&r)[32], uint4 (&out)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -301,7 +206,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           }
           const uint32_t id = (uint32_t)(kb & 3);
           const uint32_t idesc = make_idesc_scaled(BN, BM, id, id);
-          const uint64_t da = make_desc_sw128(sA), db = make_desc_sw128(sB);
+          const uint64_t da = make_desc(sA, 16, 1024), db = make_desc(sB, 16, 1024);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_fp8_scaled(tmem_d, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, sfa_col,
@@ -396,49 +301,7 @@ struct Geo {
   static constexpr size_t SMEM = STAGES * TILE_BYTES + STAGES * 2048 + 1024 + kCtrlBytes + 8 * kStageWarpBytes + 1024 /*row maxima*/;
 };
 constexpr int TILE_M = 2 * BM;
-constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;               // clears the CTA-rank bit of a shared::cluster address
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(saddr), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar) & kPeerBitMask), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar) & kPeerBitMask), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc2(uint32_t* dst_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void commit2(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
-               : "memory");
-}
 __device__ __forceinline__ void tmem_cp_sf2(uint32_t taddr, uint64_t sdesc) {
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
@@ -518,7 +381,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc2(tmem_slot, TMEM_COLS);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, TMEM_COLS);
   if (warp == 2)
     warp_tile_prefix(tile_prefix, n_groups, lane, [&](int g) { return ceil_div(args.group_rows[g], TILE_M) * n_tiles_n; });
   tc_fence_before();
@@ -556,14 +419,14 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
             uint64_t* fb = &full_bar[stage];
             const bool with_sf = (kb & 3) == 0;
             if (cta_rank == 0) mbar_expect_tx(fb, 2 * (TILE_BYTES + (with_sf ? G::SF_BYTES : 0)));
-            tma_2d(sA, &tmA, fb, kb * BK, row_first);
-            tma_3d(sB, &tmB, fb, kb * BK, b_row, t.wslot);
+            tma_load_2d_pair(sA, &tmA, fb, kb * BK, row_first);
+            tma_load_3d_pair(sB, &tmB, fb, kb * BK, b_row, t.wslot);
             if (with_sf) {
               uint8_t* sS = sf_tiles + stage * SF_BYTES;
-              tma_2d(sS, &tmSFA, fb, 0, sfa_chunk + (kb >> 2));
+              tma_load_2d_pair(sS, &tmSFA, fb, 0, sfa_chunk + (kb >> 2));
 #pragma unroll
               for (int j = 0; j < kBN / 128; ++j)
-                tma_2d(sS + 512 + 512 * j, &tmSFB, fb, 0, sfb_chunk + j * sfb_step + (kb >> 2));
+                tma_load_2d_pair(sS + 512 + 512 * j, &tmSFB, fb, 0, sfb_chunk + j * sfb_step + (kb >> 2));
             }
             if (++stage == STAGES) {
               stage = 0;
@@ -614,14 +477,14 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
           }
           const uint32_t id = (uint32_t)(kb & 3);
           const uint32_t idesc = make_idesc_scaled(kBN, TILE_M, id, id);
-          const uint64_t da = make_desc_sw128(sA), db = make_desc_sw128(sB);
+          const uint64_t da = make_desc(sA, 16, 1024), db = make_desc(sB, 16, 1024);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma2(tmem_d, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, sfa_col, sfb_col,
                   (kb | k) ? 1u : 0u);
           const uint32_t eb = smem_u32(&empty_bar[stage]);
-          commit2(eb);
-          commit2(map_to_cta(eb, 1));
+          umma_commit_pair(eb);
+          umma_commit_pair(map_to_cta(eb, 1));
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -629,8 +492,8 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         }
         if (failed) break;
         const uint32_t ab = smem_u32(&acc_full[buf]);
-        commit2(ab);
-        commit2(map_to_cta(ab, 1));
+        umma_commit_pair(ab);
+        umma_commit_pair(map_to_cta(ab, 1));
       }
     }
     __syncwarp();
@@ -749,7 +612,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
   cluster_sync_all();  // neither CTA leaves while the other may still signal it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc2(tmem_base, TMEM_COLS);
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 

@@ -78,20 +78,6 @@ __device__ __forceinline__ void flush_rows(const uint4* tile, int quarter, int l
     if (base != 0ull && piece < pieces) *reinterpret_cast<uint4*>(base + piece * 16) = tile[tok * 16 + piece];
   }
 }
-// All four warps of a half agree (and meet): true if `ok` holds in each of them.
-__device__ __forceinline__ bool half_all(int half, bool ok) {
-  uint32_t all;
-  asm volatile(
-      "{\n.reg .pred p, q;\n"
-      "setp.ne.u32 p, %1, 0;\n"
-      "bar.red.and.pred q, %2, 128, p;\n"
-      "selp.u32 %0, 1, 0, q;\n}\n"
-      : "=r"(all)
-      : "r"(ok ? 1u : 0u), "r"(1 + half)
-      : "memory");
-  return all != 0u;
-}
-__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
 // Stage one value per (token, feature): lane = feature, element j = token.  A warp writes 64 contiguous bytes per token.
 template <typename F>
 __device__ __forceinline__ void stage_and_flush(__nv_bfloat16* stg, int half, int quarter, int lane, char* mine, int pieces, F value) {

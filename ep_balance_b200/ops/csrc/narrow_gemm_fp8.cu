@@ -55,26 +55,6 @@ __device__ __forceinline__ bool find_tile(const Fp8GemmArgs& a, int n_groups, co
   return true;
 }
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
-// All four warps of a half agree (and meet): true if `ok` holds in each of them.
-__device__ __forceinline__ bool half_all(int half, bool ok) {
-  uint32_t all;
-  asm volatile(
-      "{\n.reg .pred p, q;\n"
-      "setp.ne.u32 p, %1, 0;\n"
-      "bar.red.and.pred q, %2, 128, p;\n"
-      "selp.u32 %0, 1, 0, q;\n}\n"
-      : "=r"(all)
-      : "r"(ok ? 1u : 0u), "r"(1 + half)
-      : "memory");
-  return all != 0u;
-}
-
 template <bool kAct>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 narrow_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,

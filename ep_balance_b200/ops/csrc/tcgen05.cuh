@@ -1,6 +1,6 @@
-// Building blocks of the bf16 grouped-GEMM kernels (grouped_gemm.cu, narrow_gemm.cu): PTX wrappers for mbarriers, TMA
-// loads, tensor memory and tcgen05.mma, shared-memory and instruction descriptors, the group walk and the completion
-// signal.  Every wait is bounded.
+// Building blocks of the grouped-GEMM kernels, bf16 and fp8, wide and narrow: PTX wrappers for mbarriers, TMA and bulk
+// loads, tensor memory and tcgen05.mma, shared-memory and instruction descriptors, meeting points of epilogue warps and the
+// completion signal.  Every wait is bounded.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -91,6 +91,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 // ---- CTA-pair variants (thread-block cluster of 2; no multicast anywhere)
@@ -229,6 +234,21 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t v) {
   return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v));
 }
 __device__ __forceinline__ float sigmoidf_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// Meeting point of the four epilogue warps of a half (named barriers 1 and 2).
+__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
+// All four warps of a half agree (and meet): true if `ok` holds in each of them.
+__device__ __forceinline__ bool half_all(int half, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "bar.red.and.pred q, %2, 128, p;\n"
+      "selp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(all)
+      : "r"(ok ? 1u : 0u), "r"(1 + half)
+      : "memory");
+  return all != 0u;
+}
 
 // ---------------------------------------------------------------- completion
 // One thread per CTA, after the CTA's (peer) stores are fenced: the last CTA of the launch tells every peer.
