@@ -78,9 +78,9 @@ cudaError_t launch_quantize_rows(const void* x, uint8_t* q, uint8_t* sfa, int ro
 // `act` (bf16 [rows, F], may be null) also receives the unquantised activation.
 cudaError_t launch_swiglu_quantize(const void* h, uint8_t* q, uint8_t* sfa, void* act, int rows, int F,
                                    const RowGroups* groups, cudaStream_t stream);
-// Dispatch fused with the 1 x 128 quantisation: every routed unit's token row is quantised in registers and
-// stored as e4m3 bytes (plus its scale bytes) straight into the destination rank's operand buffer, so half
-// the bytes of a bf16 dispatch cross NVLink and no separate quantisation pass runs on the receiver.
+// Dispatch fused with the 1 x 128 quantisation: every token's row is quantised once in registers and stored as e4m3 bytes
+// (plus its scale bytes) straight into the operand buffers of the ranks its units go to, so half the bytes of a bf16
+// dispatch cross NVLink and no separate quantisation pass runs on the receiver.  num_units is a multiple of topk.
 struct DispatchFp8Args {
   const void* rows;             // bf16 [num_tokens, H]
   int num_units, topk, H, R, me;

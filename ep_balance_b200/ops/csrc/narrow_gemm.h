@@ -15,8 +15,9 @@ constexpr int kNarrowBoxRows = 32;  // token rows of one TMA box: box of the tok
 //   2048 x  768 x 128        327 /  212   351 /  254   353 /  260   381 /  322   629 /  536
 //   5120 x 1536 x 160       1856 / 1176  2210 / 1397  2132 / 1867  2246 / 2312  3672 / 3808
 //   2048 x 1408 x  64        302 /  206   295 /  241   311 /  268   337 /  337   570 /  578
-// Below 128 the weights' bytes bound the launch and the narrow tiles win everywhere; from about 190 on the 256-row
-// tiles of the wide kernel are full enough, and move fewer operand bytes per flop.
+// One line for every shape, at the most rows where the narrow kernel won each of them: the weights' bytes bound the launch up
+// to there.  Beyond it the shapes disagree.  Wide rows and many weights do better on the full 256-row tiles, which move fewer
+// operand bytes per flop; the first shape, with its short reductions, would keep 15 % on the narrow kernel up to 384 rows.
 constexpr int kNarrowRowsPerSlot = 128;
 
 // tmW: the weight map that grouped_gemm.h's kernels use as B (K-major box {64, 128, 1}); tmX: token rows, 2-D, box

@@ -8,9 +8,17 @@ namespace epb {
 constexpr int kNarrowFp8BoxRows = 32;  // token rows of one TMA box
 
 // Batches with fewer routed units per weight slot than this take the narrow kernel: with few rows the 256-row tiles of the
-// pair kernel are mostly padding.  (The line was drawn here for the single-CTA kernel that had these batches before.)
-// 32 experts of 7168 x 2048, 16 rows each: both GEMMs 252 us and the activation pass 9 before, the whole decode step of a
-// layer 364 -> 338 us (1.41 GB of weights: 212 us at the HBM rate).
+// pair kernel are mostly padding.  Measured, both GEMMs with the activation in us, pair / narrow, rows per expert spread by a
+// lognormal of 0.35 around the mean:
+//   hidden x ffn x experts   16 rows     96 rows     128 rows    160 rows    191 rows    256 rows
+//   7168 x 2048 x  32        321 / 252   341 / 267   344 / 307   374 / 403   385 / 441   469 / 521
+//   5120 x 1536 x  40        228 / 183   242 / 212   247 / 221   260 / 271   292 / 307   353 / 375
+//   2048 x  768 x 128        210 / 142   202 / 161   214 / 180   228 / 204   249 / 236   284 / 284
+//   2048 x 1408 x  64        167 / 116   166 / 135   175 / 149   191 / 168   203 / 183   232 / 219
+//   1024 x  512 x 256        161 / 119   184 / 172   195 / 191   206 / 209   224 / 234   246 / 274
+// Up to 128 rows the narrow kernel wins everywhere; from there to the line each kernel wins by up to 14 % at some shapes, and
+// by 384 rows the pair kernel is ahead at all of them.  (16 rows of the first shape read 1.41 GB of weights: 215 us at the rate
+// of a copy.)
 constexpr int kNarrowFp8RowsPerSlot = 192;
 
 struct NarrowFp8Args {
