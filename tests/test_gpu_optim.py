@@ -110,3 +110,32 @@ def test_guarded_adamw_skips_the_update_while_a_status_word_is_set():
     opt.step()
     torch.cuda.synchronize()
     assert not torch.equal(p.detach(), before)
+
+
+@pytest.mark.parametrize("grad_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("lr,eps,step", [(1e-5, 1e-8, 1), (0.3, 1e-8, 1000), (1e-3, 0.0, 3)])
+def test_vectors_of_eight_weights_have_the_bits_of_the_plain_formula(grad_dtype, lr, eps, step):
+    """A tensor of seven weights is updated by the formula alone, eight or more by the rounding test in front of it: the
+    same values, ordinary ones and every bf16 pattern (zeros, subnormals, infinities, NaN), have to come out the same."""
+    from ep_balance_b200.ops.extension import load
+
+    ext, gen = load(), torch.Generator(device="cuda").manual_seed(3)
+    n = 7 * 8 * 300
+    rand = lambda scale: (scale * torch.randn(n, device="cuda", generator=gen)).bfloat16()  # noqa: E731
+    anybits = lambda: torch.randint(-32768, 32768, (n,), device="cuda", generator=gen, dtype=torch.int16).view(torch.bfloat16)  # noqa: E731
+    for p, g, m, v in ((rand(0.02), rand(1e-3), rand(1e-3), rand(1e-3).square()),
+                       (rand(0.02), torch.zeros_like(rand(1)), torch.zeros_like(rand(1)), torch.zeros_like(rand(1))),
+                       (anybits(), anybits(), anybits(), anybits().abs())):
+        g = g.to(grad_dtype)
+        plain = [t.clone() for t in (p, m, v)]
+        for i in range(0, 7 * 64, 7):          # 16-byte aligned copies of seven weights each
+            part = [t[i:i + 7].clone() for t in (*plain, g)]
+            ext.adamw_step(part[0], part[3], part[1], part[2], lr, 0.9, 0.999, eps, 0.1, step, None, None)
+            for whole, piece in zip(plain, part):
+                whole[i:i + 7] = piece
+        mine = [t.clone() for t in (p, m, v)]
+        ext.adamw_step(mine[0], g, mine[1], mine[2], lr, 0.9, 0.999, eps, 0.1, step, None, None)
+        for a, b in zip(mine, plain):
+            a, b = a[:7 * 64], b[:7 * 64]
+            same = (a.view(torch.int16) == b.view(torch.int16)) | (a.isnan() & b.isnan())
+            assert bool(same.all()), (a[~same][:4], b[~same][:4])
