@@ -35,12 +35,18 @@ constexpr int TMEM_COLS = 512;
 // rows of A and its own 128 columns of B, so per-SM operand traffic drops from 48 KB to 32 KB per
 // k-block and the shared-memory ring deepens from 4 to 6 stages.
 // The fused-transport variants (kComm != 0) give 64 KB of the operand ring to the transport warps' copy rings.
-template <int kCtas, int kComm = 0>
+// A stage holds kSub k-blocks.  Every tcgen05.commit leaves the tensor pipe idle for some 45 cycles, and a k-block is only
+// 512 cycles of MMAs: with two commits a k-block (one per CTA of the pair) the pipe was at most 78 % busy with no loads and no
+// epilogue at all, with one multicast commit 84 %, with one per two k-blocks 96 %.  Wgrad (K = the rows of a group, often a
+// dozen k-blocks) and the fused-transport variants (four stages) keep one k-block a stage.
+template <int kCtas, int kComm = 0, int kMode = -1>
 struct Geometry {
-  static constexpr int STAGES = (kCtas == 2 ? 6 : 4) - (kComm ? (kCtas == 2 ? 2 : 1) : 0);
+  static constexpr int kSub = kCtas == 2 && kComm == 0 && kMode != kWgrad ? 2 : 1;
+  static constexpr int STAGES = ((kCtas == 2 ? 6 : 4) - (kComm ? (kCtas == 2 ? 2 : 1) : 0)) / kSub;
   static constexpr int COMM_SLOTS = kCtas == 2 ? 8 : 6;  // ring slots of a transport warp: batches of 4 (3) segments of 4 KB
   static constexpr int B_BYTES = BN * BK * 2 / kCtas;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int SUB_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGE_BYTES = SUB_BYTES * kSub;
   static constexpr int TILE_M = BM * kCtas;
 };
 constexpr int NUM_THREADS = 320;  // TMA warp + MMA warp + 8 epilogue warps
@@ -183,8 +189,8 @@ template <int kMode, int kCtas, int kComm, bool kAccum>
 __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ GemmArgs args) {
-  using G = Geometry<kCtas, kComm>;
-  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, TILE_M = G::TILE_M;
+  using G = Geometry<kCtas, kComm, kMode>;
+  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, SUB_BYTES = G::SUB_BYTES, TILE_M = G::TILE_M;
   constexpr bool kAMn = kMode == kWgrad;
   constexpr bool kBMn = kMode == kWgrad || kMode == kDgrad2 || kMode == kDgrad1;
 
@@ -265,34 +271,38 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const int n_off = t.nt * BN + cta_rank * (BN / 2) * (kCtas - 1);  // this CTA's columns of B
           constexpr int kBoxesB = 4 / kCtas;                          // 64-wide MN-major boxes of B
           const int kblocks = k_blocks<kMode>(shape, t);
-          for (int kb = 0; kb < kblocks; ++kb) {
+          for (int kb0 = 0; kb0 < kblocks; kb0 += G::kSub) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_v, args.status, 1)) {
               go = 0;
               break;
             }
-            uint8_t* sA = tiles + stage * STAGE_BYTES;
-            uint8_t* sB = sA + A_BYTES;
             uint64_t* fb = &full_bar[stage];
-            if (cta_rank == 0) mbar_expect_tx(fb, STAGE_BYTES * kCtas);  // both CTAs' bytes land on the leader's barrier
-            if (kMode == kWgrad) {
-              const int krow = t.row0 + kb * BK;
-              for (int i = 0; i < 2; ++i) tma2<kCtas>(sA + i * 8192, &tmA, fb, m_off + 64 * i, krow);
-              for (int j = 0; j < kBoxesB; ++j) tma2<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, krow);
-            } else {
-              tma2<kCtas>(sA, &tmA, fb, kb * BK, t.row0 + m_off);
-              if (kMode == kFwd1) {
-                // gate rows [nt*128, +128) and up rows [F + nt*128, +128): one half per CTA of a pair
-                if (kCtas == 2) {
-                  tma3<kCtas>(sB, &tmB, fb, kb * BK, cta_rank * args.N + t.nt * 128, t.wslot);
-                } else {
-                  tma3<kCtas>(sB, &tmB, fb, kb * BK, t.nt * 128, t.wslot);
-                  tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, args.N + t.nt * 128, t.wslot);
-                }
-              } else if (kBMn) {
-                for (int j = 0; j < kBoxesB; ++j) tma3<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, kb * BK, t.wslot);
+            const int subs = min(G::kSub, kblocks - kb0);
+            if (cta_rank == 0) mbar_expect_tx(fb, subs * SUB_BYTES * kCtas);  // both CTAs' bytes land on the leader's barrier
+            for (int sub = 0; sub < subs; ++sub) {
+              const int kb = kb0 + sub;
+              uint8_t* sA = tiles + stage * STAGE_BYTES + sub * SUB_BYTES;
+              uint8_t* sB = sA + A_BYTES;
+              if (kMode == kWgrad) {
+                const int krow = t.row0 + kb * BK;
+                for (int i = 0; i < 2; ++i) tma2<kCtas>(sA + i * 8192, &tmA, fb, m_off + 64 * i, krow);
+                for (int j = 0; j < kBoxesB; ++j) tma2<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, krow);
               } else {
-                tma3<kCtas>(sB, &tmB, fb, kb * BK, n_off, t.wslot);
-                if (kCtas == 1) tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, n_off + 128, t.wslot);
+                tma2<kCtas>(sA, &tmA, fb, kb * BK, t.row0 + m_off);
+                if (kMode == kFwd1) {
+                  // gate rows [nt*128, +128) and up rows [F + nt*128, +128): one half per CTA of a pair
+                  if (kCtas == 2) {
+                    tma3<kCtas>(sB, &tmB, fb, kb * BK, cta_rank * args.N + t.nt * 128, t.wslot);
+                  } else {
+                    tma3<kCtas>(sB, &tmB, fb, kb * BK, t.nt * 128, t.wslot);
+                    tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, args.N + t.nt * 128, t.wslot);
+                  }
+                } else if (kBMn) {
+                  for (int j = 0; j < kBoxesB; ++j) tma3<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, kb * BK, t.wslot);
+                } else {
+                  tma3<kCtas>(sB, &tmB, fb, kb * BK, n_off, t.wslot);
+                  if (kCtas == 1) tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, n_off + 128, t.wslot);
+                }
               }
             }
             if (++stage == STAGES) {
@@ -337,33 +347,34 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const uint32_t idesc = make_idesc(kAMn, kBMn, ncols, TILE_M);
         bool failed = false;
         const int kblocks = k_blocks<kMode>(shape, t);
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb0 = 0; kb0 < kblocks; kb0 += G::kSub) {
           if (!mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) {
             failed = true;
             break;
           }
           tc_fence_after();
-          const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES);
-          const uint32_t sB = sA + A_BYTES;
-          const uint64_t da = kAMn ? make_desc(sA, 8192, 1024) : make_desc(sA, 16, 1024);
-          const uint64_t db = kBMn ? make_desc(sB, 8192, 1024) : make_desc(sB, 16, 1024);
-          constexpr uint32_t a_step = kAMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
-          constexpr uint32_t b_step = kBMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+          const int subs = min(G::kSub, kblocks - kb0);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            if (kCtas == 2)
-              umma_bf16_pair(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, (kb | k) ? 1u : 0u);
-            else
-              umma_bf16(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, (kb | k) ? 1u : 0u);
+          for (int sub = 0; sub < G::kSub; ++sub) {
+            if (sub >= subs) break;
+            const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES + sub * SUB_BYTES);
+            const uint32_t sB = sA + A_BYTES;
+            const uint64_t da = kAMn ? make_desc(sA, 8192, 1024) : make_desc(sA, 16, 1024);
+            const uint64_t db = kBMn ? make_desc(sB, 8192, 1024) : make_desc(sB, 16, 1024);
+            constexpr uint32_t a_step = kAMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+            constexpr uint32_t b_step = kBMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint32_t acc = (kb0 | sub | k) ? 1u : 0u;
+              if (kCtas == 2)
+                umma_bf16_pair(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
+              else
+                umma_bf16(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
+            }
           }
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
-          if (kCtas == 2) {
-            const uint32_t eb = smem_u32(&empty_bar[stage]);
-            umma_commit_pair(eb);
-            umma_commit_pair(map_to_cta(eb, 1));
-          } else {
-            umma_commit(&empty_bar[stage]);
-          }
+          if (kCtas == 2) umma_commit_both(&empty_bar[stage]);
+          else umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -372,13 +383,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (failed) break;
         if (args.trace != nullptr) atomicMax(args.trace + 2, globaltimer_ns());
         // accumulator ready for the epilogue warps (of both CTAs)
-        if (kCtas == 2) {
-          const uint32_t ab = smem_u32(&acc_full[buf]);
-          umma_commit_pair(ab);
-          umma_commit_pair(map_to_cta(ab, 1));
-        } else {
-          umma_commit(&acc_full[buf]);
-        }
+        if (kCtas == 2) umma_commit_both(&acc_full[buf]);
+        else umma_commit(&acc_full[buf]);
       }
     }
     __syncwarp();
@@ -599,8 +605,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 template <int kCtas, int kComm>
-constexpr size_t smem_bytes() {
-  return Geometry<kCtas, kComm>::STAGES * Geometry<kCtas, kComm>::STAGE_BYTES + 1024 /*align*/ +
+constexpr size_t smem_bytes() {  // the same for every mode: a stage of two k-blocks counts as two
+  return Geometry<kCtas, kComm, kWgrad>::STAGES * Geometry<kCtas, kComm, kWgrad>::STAGE_BYTES + 1024 /*align*/ +
          kCtrlBytes /*barriers, flags, tile prefix*/ + 8 * kStageWarpBytes /*staging*/ +
          (kComm ? COMM_WARPS * comm_warp_bytes<Geometry<kCtas, kComm>::COMM_SLOTS>() : 0) /*transport rings*/;
 }

@@ -289,6 +289,31 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 // the pair's even CTA; that CTA issues the scale copies and the MMAs for both.
 namespace pair {
 
+constexpr int kPairStageBytes = 2048;  // staging tile of one epilogue warp: 16 rows x 128 B, or 32 rows x 64 B
+
+// 128 bytes of each lane's row (p0, then p1) to memory, 16 rows at a time, four rows x 128 contiguous bytes per instruction.
+__device__ __forceinline__ void rows_out(uint4* tile, int lane, const uint4 (&p0)[4], const uint4 (&p1)[4], char* rowptr, int byte_off) {
+  const unsigned long long mine = reinterpret_cast<unsigned long long>(rowptr);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    __syncwarp();
+    if ((lane >> 4) == h) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        tile[wide_index(lane & 15, i)] = p0[i];
+        tile[wide_index(lane & 15, 4 + i)] = p1[i];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int r = it * 4 + (lane >> 3), p = lane & 7;
+      const unsigned long long base = __shfl_sync(0xffffffffu, mine, h * 16 + r);
+      if (base != 0ull) *reinterpret_cast<uint4*>(base + byte_off + p * 16) = tile[wide_index(r, p)];
+    }
+  }
+}
+
 // kBN = 128: two accumulator buffers (epilogue overlaps the next tile).  kBN = 256: one 256-column accumulator
 // (the scale factors need the rest of tensor memory), twice the MMA work per TMA load and per barrier round.
 template <int kBN>
@@ -296,9 +321,12 @@ struct Geo {
   static constexpr int B_HALF = kBN / 2;                     // weight rows staged per CTA
   static constexpr int A_BYTES = BM * BK, B_BYTES = B_HALF * BK, TILE_BYTES = A_BYTES + B_BYTES;
   static constexpr int SF_BYTES = 512 + 512 * (kBN / 128);   // this CTA's SFA chunk + the SFB chunks of the whole tile
-  static constexpr int STAGES = kBN == 128 ? 6 : 5;
+  // A stage holds kSub k-blocks: a tcgen05.commit costs the tensor pipe idle cycles (grouped_gemm.cu), so there is one per stage.
+  static constexpr int kSub = 2;
+  static constexpr int STAGES = 3;
+  static constexpr int STAGE_BYTES = kSub * TILE_BYTES;
   static constexpr int ACC_BUFS = kBN == 128 ? 2 : 1;
-  static constexpr size_t SMEM = STAGES * TILE_BYTES + STAGES * 2048 + 1024 + kCtrlBytes + 8 * kStageWarpBytes + 1024 /*row maxima*/;
+  static constexpr size_t SMEM = STAGES * (STAGE_BYTES + 2048) + 1024 + kCtrlBytes + 8 * kPairStageBytes + 1024 /*row maxima*/;
 };
 constexpr int TILE_M = 2 * BM;
 
@@ -343,12 +371,13 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
                              Fp8GemmArgs args) {
   using G = Geo<kBN>;
   constexpr int STAGES = G::STAGES, TILE_BYTES = G::TILE_BYTES, A_BYTES = G::A_BYTES, B_HALF = G::B_HALF;
+  constexpr int kSub = G::kSub, STAGE_BYTES = G::STAGE_BYTES;
   constexpr int SF_BYTES = 2048;   // slot size; G::SF_BYTES of it are used
   constexpr int ACC_BUFS = G::ACC_BUFS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = smem;
-  uint8_t* sf_tiles = smem + STAGES * TILE_BYTES;
+  uint8_t* sf_tiles = smem + STAGES * STAGE_BYTES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(sf_tiles + STAGES * SF_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;
@@ -409,24 +438,26 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
           const int sfb_chunk = (t.wslot * n128 + t.nt * (kAct ? 1 : kBN / 128)) * kgroups;
           const int sfb_step = (kAct ? args.N / 128 : 1) * kgroups;  // from the tile's first scale block to its second
           const int b_row = kAct ? cta_rank * args.N + t.nt * 128 : t.nt * kBN + cta_rank * B_HALF;
-          for (int kb = 0; kb < kblocks; ++kb) {
+          for (int kb0 = 0; kb0 < kblocks; kb0 += kSub) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_v, args.status, 21)) {
               go = 0;
               break;
             }
-            uint8_t* sA = tiles + stage * TILE_BYTES;
-            uint8_t* sB = sA + A_BYTES;
             uint64_t* fb = &full_bar[stage];
-            const bool with_sf = (kb & 3) == 0;
-            if (cta_rank == 0) mbar_expect_tx(fb, 2 * (TILE_BYTES + (with_sf ? G::SF_BYTES : 0)));
-            tma_load_2d_pair(sA, &tmA, fb, kb * BK, row_first);
-            tma_load_3d_pair(sB, &tmB, fb, kb * BK, b_row, t.wslot);
+            const int subs = min(kSub, kblocks - kb0);
+            const bool with_sf = (kb0 & 3) == 0;
+            if (cta_rank == 0) mbar_expect_tx(fb, 2 * (subs * TILE_BYTES + (with_sf ? G::SF_BYTES : 0)));
+            for (int sub = 0; sub < subs; ++sub) {
+              uint8_t* sA = tiles + stage * STAGE_BYTES + sub * TILE_BYTES;
+              tma_load_2d_pair(sA, &tmA, fb, (kb0 + sub) * BK, row_first);
+              tma_load_3d_pair(sA + A_BYTES, &tmB, fb, (kb0 + sub) * BK, b_row, t.wslot);
+            }
             if (with_sf) {
               uint8_t* sS = sf_tiles + stage * SF_BYTES;
-              tma_load_2d_pair(sS, &tmSFA, fb, 0, sfa_chunk + (kb >> 2));
+              tma_load_2d_pair(sS, &tmSFA, fb, 0, sfa_chunk + (kb0 >> 2));
 #pragma unroll
               for (int j = 0; j < kBN / 128; ++j)
-                tma_load_2d_pair(sS + 512 + 512 * j, &tmSFB, fb, 0, sfb_chunk + j * sfb_step + (kb >> 2));
+                tma_load_2d_pair(sS + 512 + 512 * j, &tmSFB, fb, 0, sfb_chunk + j * sfb_step + (kb0 >> 2));
             }
             if (++stage == STAGES) {
               stage = 0;
@@ -458,15 +489,13 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         const uint32_t tmem_d = tmem_base + (uint32_t)(buf * 128);
         bool failed = false;
         uint32_t sfa_col = 0, sfb_col = 0;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb0 = 0; kb0 < kblocks; kb0 += kSub) {
           if (!mbar_wait(&full_bar[stage], phase, abort_v, args.status, 23)) {
             failed = true;
             break;
           }
           tc_fence_after();
-          const uint32_t sA = smem_u32(tiles + stage * TILE_BYTES);
-          const uint32_t sB = sA + A_BYTES;
-          if ((kb & 3) == 0) {
+          if ((kb0 & 3) == 0) {
             const uint32_t sS = smem_u32(sf_tiles + stage * SF_BYTES);
             sfa_col = tmem_base + kSfCol + sf_buf * 16;
             sfb_col = sfa_col + 4;
@@ -475,25 +504,27 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
             for (int j = 0; j < kBN / 128; ++j) tmem_cp_sf2(sfb_col + 4 * j, make_desc_sf(sS + 512 + 512 * j));
             sf_buf ^= 1u;
           }
-          const uint32_t id = (uint32_t)(kb & 3);
-          const uint32_t idesc = make_idesc_scaled(kBN, TILE_M, id, id);
-          const uint64_t da = make_desc(sA, 16, 1024), db = make_desc(sB, 16, 1024);
+          const int subs = min(kSub, kblocks - kb0);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma2(tmem_d, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, sfa_col, sfb_col,
-                  (kb | k) ? 1u : 0u);
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          umma_commit_pair(eb);
-          umma_commit_pair(map_to_cta(eb, 1));
+          for (int sub = 0; sub < kSub; ++sub) {
+            if (sub >= subs) break;
+            const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES + sub * TILE_BYTES);
+            const uint32_t id = (uint32_t)((kb0 + sub) & 3);
+            const uint32_t idesc = make_idesc_scaled(kBN, TILE_M, id, id);
+            const uint64_t da = make_desc(sA, 16, 1024), db = make_desc(sA + A_BYTES, 16, 1024);
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma2(tmem_d, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, sfa_col, sfb_col,
+                    (kb0 | sub | k) ? 1u : 0u);
+          }
+          umma_commit_both(&empty_bar[stage]);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (failed) break;
-        const uint32_t ab = smem_u32(&acc_full[buf]);
-        umma_commit_pair(ab);
-        umma_commit_pair(map_to_cta(ab, 1));
+        umma_commit_both(&acc_full[buf]);
       }
     }
     __syncwarp();
@@ -501,7 +532,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
     // ------------------------------------------------------------ epilogue (warps 2..9 of both CTAs)
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
-    uint4* stg = stage_tiles + (warp - 2) * (kStageWarpBytes / 16);
+    uint4* stg = stage_tiles + (warp - 2) * (kPairStageBytes / 16);
     uint32_t acc_phase[2] = {0, 0};
     int local = 0, cursor = 0;
     Tile t;
@@ -554,7 +585,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
           }
         }
         // the row's other 64 features are in the warp that shares its quarter
-        float* maxima = reinterpret_cast<float*>(stage_tiles + 8 * (kStageWarpBytes / 16)) + quarter * 64;
+        float* maxima = reinterpret_cast<float*>(stage_tiles + 8 * (kPairStageBytes / 16)) + quarter * 64;
         maxima[half * 32 + lane] = amax;
         rows_sync(quarter);
         amax = fmaxf(amax, maxima[(half ^ 1) * 32 + lane]);
@@ -593,11 +624,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
           uint4 p0[4], p1[4];
           pack_row(v[2 * pairc], p0);
           pack_row(v[2 * pairc + 1], p1);
-          __syncwarp();
-          wide_store_half(stg, lane, p0, 0);
-          wide_store_half(stg, lane, p1, 1);
-          __syncwarp();
-          wide_flush(stg, lane, orow, (t.nt * kBN + half * COLS_PER_WARP + pairc * 64) * 2);
+          rows_out(stg, lane, p0, p1, orow, (t.nt * kBN + half * COLS_PER_WARP + pairc * 64) * 2);
         }
       }
     }

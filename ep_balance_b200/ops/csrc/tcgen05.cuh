@@ -156,10 +156,11 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrives on ONE barrier (own or the peer's, given as a shared::cluster address) once every MMA
-// issued so far by the pair has completed.  Both CTAs are told with two of these.
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
+// Arrives on this barrier of both CTAs of the pair (the same offset in each) once every MMA issued so far by the pair has
+// completed.  One instruction: a commit for each CTA cost the tensor pipe twice the idle cycles.
+__device__ __forceinline__ void umma_commit_both(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
                : "memory");
 }
 
