@@ -29,6 +29,7 @@ namespace {
 constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB: this CTA's 128 rows of the A tile
 constexpr int TMEM_COLS = 512;
+constexpr int kStageWarpBytes = 4096;  // staging tile of one epilogue warp
 
 // kCtas = 1: one CTA computes a 128 x 256 tile.  kCtas = 2: a CTA pair (thread-block cluster of
 // two SMs) computes a 256 x 256 tile with tcgen05.mma.cta_group::2; each CTA stages its own 128
@@ -39,10 +40,12 @@ constexpr int TMEM_COLS = 512;
 // 512 cycles of MMAs: with two commits a k-block (one per CTA of the pair) the pipe was at most 78 % busy with no loads and no
 // epilogue at all, with one multicast commit 84 %, with one per two k-blocks 96 %.  Wgrad (K = the rows of a group, often a
 // dozen k-blocks) and the fused-transport variants (four stages) keep one k-block a stage.
-template <int kCtas, int kComm = 0, int kMode = -1>
+// The accumulating Wgrad (kAccum) holds 128 KB of the fp32 accumulator instead of half its operand ring.
+template <int kCtas, int kComm = 0, int kMode = -1, bool kAccum = false>
 struct Geometry {
   static constexpr int kSub = kCtas == 2 && kComm == 0 && kMode != kWgrad ? 2 : 1;
-  static constexpr int STAGES = ((kCtas == 2 ? 6 : 4) - (kComm ? (kCtas == 2 ? 2 : 1) : 0)) / kSub;
+  static constexpr int STAGES = kAccum ? (kCtas == 2 ? 3 : 2) : ((kCtas == 2 ? 6 : 4) - (kComm ? (kCtas == 2 ? 2 : 1) : 0)) / kSub;
+  static constexpr int STAGE_WARP_BYTES = kAccum ? 4 * kStageWarpBytes : kStageWarpBytes;  // of one epilogue warp
   static constexpr int COMM_SLOTS = kCtas == 2 ? 8 : 6;  // ring slots of a transport warp: batches of 4 (3) segments of 4 KB
   static constexpr int B_BYTES = BN * BK * 2 / kCtas;
   static constexpr int SUB_BYTES = A_BYTES + B_BYTES;
@@ -53,8 +56,7 @@ constexpr int NUM_THREADS = 320;  // TMA warp + MMA warp + 8 epilogue warps
 constexpr int COMM_WARPS = 2;     // transport warps of the fused variants (warps 10, 11): 384 threads keep the 168-register budget
 constexpr int MAX_GROUPS = 320;  // barriers + flags + (MAX_GROUPS + 1) ints must fit in kCtrlBytes
 constexpr int kCtrlBytes = 1536;
-static_assert((6 * 2 + 4) * 8 + 8 + (MAX_GROUPS + 1) * 4 <= kCtrlBytes, "control block does not fit");
-constexpr int kStageWarpBytes = 4096;  // staging tile of one epilogue warp
+static_assert((6 * 2 + 4) * 8 + 8 + (MAX_GROUPS + 1) * 4 <= kCtrlBytes && (3 * 2 + 4 + 8) * 8 + 8 + (MAX_GROUPS + 1) * 4 <= kCtrlBytes, "control block does not fit");
 
 // ---------------------------------------------------------------- tiles
 struct Tile {
@@ -166,30 +168,35 @@ __device__ __forceinline__ void wide_flush(const uint4* tile, int lane, char* ro
     if (base != 0ull && p < pieces) *reinterpret_cast<uint4*>(base + byte_off + p * 16) = tile[wide_index(r, p)];
   }
 }
-// Accumulating form for fp32 rows: 32 rows x 128 B (32 columns) of `tile` are added to memory, eight passes of four rows.  `p`
-// is the lane's address in the first pass, `step` the bytes between passes, `rows` the rows that exist from the lane's first.
-// A vector reduction needs no load to wait for and no registers for the old values; every element has one writer.  Bound by
-// HBM: 8 bytes a weight.  64 experts of 2048 x 1024, two micro-batches of 1531 tokens: 1.62 ms for the four Wgrads (4.0 TB/s
-// of read and write), where plain Wgrads (0.74) and the pass that added their bf16 slots (1.25) took 1.99.
-__device__ __forceinline__ void wide_add(const uint4* tile, int lane, char* p, size_t step, int rows) {
+// Accumulation in fp32: a tile of 32 rows x 32 columns (128 B a row, the 128-byte swizzle of the tensor map, which is wide_index)
+// is loaded, added to and stored back by bulk tensor copies.  Every element has one writer and is touched once a launch.
+__device__ __forceinline__ void accum_store(const CUtensorMap* map, const void* tile, int col, int row, int slot) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem_u32(tile)), "r"(col),
+               "r"(row), "r"(slot)
+               : "memory");
+}
+__device__ __forceinline__ void accum_add(uint4* tile, int lane, const uint32_t (&v)[32]) {
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    if (it * 4 < rows) {
-      const uint4 v = tile[wide_index(it * 4 + (lane >> 3), lane & 7)];
-      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + it * step), "f"(__uint_as_float(v.x)),
-                   "f"(__uint_as_float(v.y)), "f"(__uint_as_float(v.z)), "f"(__uint_as_float(v.w))
-                   : "memory");
-    }
+  for (int i = 0; i < 8; ++i) {
+    float4* p = reinterpret_cast<float4*>(tile + wide_index(lane, i));
+    float4 o = *p;
+    o.x += __uint_as_float(v[4 * i + 0]);
+    o.y += __uint_as_float(v[4 * i + 1]);
+    o.z += __uint_as_float(v[4 * i + 2]);
+    o.w += __uint_as_float(v[4 * i + 3]);
+    *p = o;
   }
 }
 // ---------------------------------------------------------------- kernel
 // kComm: 0 = GEMM only; 1 = plus two transport warps (token or gradient rows to their hosts, replica weights in).
-// kAccum (kWgrad): owned slots are added to args.accum instead of being stored.
+// kAccum (kWgrad): owned slots are added to the fp32 accumulator (map tmAcc) instead of being stored.  Bound by HBM: 8 bytes a
+// weight.  Each epilogue warp loads its 16 KB of the accumulator a tile ahead, so that the loads run beside the tile's MMAs, adds
+// in shared memory and stores by bulk copies.
 template <int kMode, int kCtas, int kComm, bool kAccum>
 __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ GemmArgs args) {
-  using G = Geometry<kCtas, kComm, kMode>;
+                    const __grid_constant__ CUtensorMap tmAcc, const __grid_constant__ GemmArgs args) {
+  using G = Geometry<kCtas, kComm, kMode, kAccum>;
   constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, SUB_BYTES = G::SUB_BYTES, TILE_M = G::TILE_M;
   constexpr bool kAMn = kMode == kWgrad;
   constexpr bool kBMn = kMode == kWgrad || kMode == kDgrad2 || kMode == kDgrad1;
@@ -197,14 +204,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = smem;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);  // barriers start 8-byte aligned
+  uint4* stage_tiles = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES);  // 8 epilogue warps
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + 8 * G::STAGE_WARP_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;  // [2]
   uint64_t* acc_empty = acc_full + 2;       // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* old_full = acc_empty + 2;       // [8] with kAccum: a warp's tiles of the accumulator have landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(old_full + (kAccum ? 8 : 0));
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   int* tile_prefix = abort_flag + 1;  // [MAX_GROUPS + 1]
-  uint4* stage_tiles = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + kCtrlBytes);  // 8 warps x 4 KB
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Shape shape = make_shape<kMode, kCtas>(args);
@@ -220,6 +228,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 8 * kCtas);
     }
+    for (int w = 0; kAccum && w < 8; ++w) mbar_init(&old_full[w], 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -390,7 +399,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __syncwarp();
   } else if (kComm != 0 && warp >= NUM_THREADS / 32) {
     // ------------------------------------------------------------ transport (warps 10, 11)
-    uint8_t* comm_smem_base = reinterpret_cast<uint8_t*>(stage_tiles) + 8 * kStageWarpBytes +
+    uint8_t* comm_smem_base = smem + STAGES * STAGE_BYTES + 8 * kStageWarpBytes + kCtrlBytes +
                               (warp - NUM_THREADS / 32) * comm_warp_bytes<G::COMM_SLOTS>();
     if (args.trace != nullptr && lane == 0) atomicMin(args.trace, globaltimer_ns());
     comm_run<G::COMM_SLOTS>(args.comm, (int)blockIdx.x * COMM_WARPS + (warp - NUM_THREADS / 32), (int)gridDim.x * COMM_WARPS,
@@ -403,14 +412,39 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // tile and written out with row-contiguous 16-byte stores (8 rows x 64 B per instruction).
     const int quarter = warp & 3;      // TMEM lanes [32*quarter, 32*quarter + 32)
     const int half = (warp - 2) >> 2;  // which half of the tile's column chunks this warp handles
-    uint4* stg = stage_tiles + (warp - 2) * (kStageWarpBytes / 16);
+    uint4* stg = stage_tiles + (warp - 2) * (G::STAGE_WARP_BYTES / 16);
     uint32_t acc_phase[2] = {0, 0};
     int local = 0, cursor = 0;
     Tile t;
     char* out0 = reinterpret_cast<char*>(args.out0);
     char* out1 = reinterpret_cast<char*>(args.out1);
+    // kAccum: the tile whose part of the accumulator this warp has asked for is always the one it works on next
+    uint32_t old_phase = 0;
+    auto accumulates = [&](const Tile& x) { return kAccum && x.rows > 0 && x.wslot < args.home_cap; };
+    auto old_chunks = [&](const Tile& x) { return max(0, min(4, (args.N - x.nt * BN) / 32 - half * 4)); };  // of this warp
+    auto old_row = [&](const Tile& x) { return x.mt * TILE_M + cta_rank * BM + quarter * 32; };
+    auto fetch_old = [&](const Tile& x) {
+      const int n = old_chunks(x);
+      if (lane != 0 || !accumulates(x) || n == 0 || old_row(x) >= args.M_out) return;
+      mbar_expect_tx(&old_full[warp - 2], n * kStageWarpBytes);
+      for (int c = 0; c < n; ++c)
+        tma_load_3d(stg + c * (kStageWarpBytes / 16), &tmAcc, &old_full[warp - 2], x.nt * BN + (half * 4 + c) * 32, old_row(x), x.wslot);
+    };
+    int ahead = 0;
+    Tile t_next;
+    bool have_next = false;
+    if (kAccum) {
+      have_next = find_tile(args, shape, tile_prefix, tile_first, ahead, t_next);
+      if (have_next) fetch_old(t_next);
+    }
     for (int ti = tile_first; ti < total_tiles && !*abort_v; ti += tile_stride, ++local) {
-      if (!find_tile(args, shape, tile_prefix, ti, cursor, t)) break;
+      if (kAccum) {
+        if (!have_next) break;
+        t = t_next;
+        have_next = find_tile(args, shape, tile_prefix, ti + tile_stride, ahead, t_next);
+      } else if (!find_tile(args, shape, tile_prefix, ti, cursor, t)) {
+        break;
+      }
       const int buf = local & 1;
       const int r_in_tile = cta_rank * BM + quarter * 32 + lane;  // row inside the (pair's) M tile
       // where this lane's row goes, looked up while the tile is still being computed
@@ -437,28 +471,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
 
       if (kAccum && t.wslot < args.home_cap) {
-        const int col0 = t.nt * BN;
-        const int nchunks = t.rows > 0 ? min(BN / 32, (args.N - col0) / 32) : 0;  // no rows: nothing to add
-        const int cb = half * 4;
-        const int m0 = t.mt * TILE_M + cta_rank * BM + quarter * 32 + (lane >> 3);  // this lane's row of the first pass
-        const int rows = args.M_out - m0;
-        const size_t step = (size_t)args.N * 16;  // four rows of fp32
-        char* p = reinterpret_cast<char*>(args.accum + ((size_t)t.wslot * args.M_out + m0) * (size_t)args.N + col0 + cb * 32) +
-                  (lane & 7) * 16;
-        uint32_t v[2][32];
-        if (cb < nchunks) tmem_ld32(taddr + cb * 32, v[0]);
+        const int n = old_chunks(t);
+        if (accumulates(t) && n > 0 && old_row(t) < args.M_out) {  // no rows: nothing to add
+          const int cb = half * 4;
+          uint32_t v[2][32];
+          tmem_ld32(taddr + cb * 32, v[0]);
+          if (!mbar_wait(&old_full[warp - 2], old_phase, abort_v, args.status, 7)) break;
+          old_phase ^= 1u;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int c = cb + k;
-          if (c < nchunks) {
-            tmem_ld_wait();
-            if (k + 1 < 4 && c + 1 < nchunks) tmem_ld32(taddr + (c + 1) * 32, v[(k + 1) & 1]);
-            uint32_t(&w)[32] = v[k & 1];
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) stg[wide_index(lane, i)] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-            __syncwarp();
-            wide_add(stg, lane, p + k * 128, step, rows);
+          for (int k = 0; k < 4; ++k) {
+            if (k < n) {
+              tmem_ld_wait();
+              if (k + 1 < n) tmem_ld32(taddr + (cb + k + 1) * 32, v[(k + 1) & 1]);
+              uint4* tile = stg + k * (kStageWarpBytes / 16);
+              accum_add(tile, lane, v[k & 1]);
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) {
+                accum_store(&tmAcc, tile, t.nt * BN + (cb + k) * 32, old_row(t), t.wslot);
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              }
+            }
           }
         }
       } else if (kMode == kFwd1) {
@@ -583,7 +616,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (kCtas == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
         else mbar_arrive(&acc_empty[buf]);
       }
+      if (kAccum) {
+        // the stores have read the staging tiles: the next tile's part of the accumulator may land there
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // a replica slot's rows went through them by plain stores
+        __syncwarp();
+        if (have_next) fetch_old(t_next);
+      }
     }
+    if (kAccum && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (args.done_ctr != nullptr) __threadfence_system();  // this warp's (peer) stores before the completion signal
   }
 
@@ -604,13 +645,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
-template <int kCtas, int kComm>
+template <int kCtas, int kComm, bool kAccum = false>
 constexpr size_t smem_bytes() {  // the same for every mode: a stage of two k-blocks counts as two
-  return Geometry<kCtas, kComm, kWgrad>::STAGES * Geometry<kCtas, kComm, kWgrad>::STAGE_BYTES + 1024 /*align*/ +
-         kCtrlBytes /*barriers, flags, tile prefix*/ + 8 * kStageWarpBytes /*staging*/ +
+  using G = Geometry<kCtas, kComm, kWgrad, kAccum>;
+  return G::STAGES * G::STAGE_BYTES + 1024 /*align*/ + kCtrlBytes /*barriers, flags, tile prefix*/ + 8 * G::STAGE_WARP_BYTES /*staging*/ +
          (kComm ? COMM_WARPS * comm_warp_bytes<Geometry<kCtas, kComm>::COMM_SLOTS>() : 0) /*transport rings*/;
 }
-static_assert(smem_bytes<2, 1>() <= 232448 && smem_bytes<1, 1>() <= 232448 && smem_bytes<2, 0>() <= 232448, "shared memory budget");
+static_assert(smem_bytes<2, 1>() <= 232448 && smem_bytes<1, 1>() <= 232448 && smem_bytes<2, 0>() <= 232448 &&
+                  smem_bytes<2, 0, true>() <= 232448 && smem_bytes<1, 0, true>() <= 232448, "shared memory budget");
 
 // ---------------------------------------------------------------- tensor maps
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -657,11 +699,23 @@ bool make_tmap_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t r
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {cols, rows, slots};
+  cuuint64_t strides[2] = {cols * 4, rows * cols * 4};
+  cuuint32_t box[3] = {32, 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int kMode, int kCtas, int kComm, bool kAccum = false>
 static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, const CUtensorMap* accum = nullptr) {
   static bool configured[kMaxTrackedDevices] = {};
-  constexpr size_t smem = smem_bytes<kCtas, kComm>();
+  constexpr size_t smem = smem_bytes<kCtas, kComm, kAccum>();
   int dev;
   if (device_needs_setup(configured, &dev)) {
     cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -681,12 +735,12 @@ static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, c
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, args);
+  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, kAccum ? *accum : tmA, args);
 }
 
 template <int kCtas>
 static cudaError_t launch_ctas(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, const CUtensorMap* accum) {
   const bool comm = args.comm.do_dispatch || args.comm.do_pad || args.comm.do_pull;
   if (comm) {
     // fused transport exists for the two GEMMs that consume freshly dispatched rows
@@ -700,7 +754,7 @@ static cudaError_t launch_ctas(const CUtensorMap& tmA, const CUtensorMap& tmB, c
     case kDgrad2: return launch_mode<kDgrad2, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kDgrad1: return launch_mode<kDgrad1, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kWgrad:
-      if (args.accum != nullptr) return launch_mode<kWgrad, kCtas, 0, true>(tmA, tmB, args, num_sms, stream);
+      if (accum != nullptr) return launch_mode<kWgrad, kCtas, 0, true>(tmA, tmB, args, num_sms, stream, accum);
       return launch_mode<kWgrad, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     case kPlain: return launch_mode<kPlain, kCtas, 0>(tmA, tmB, args, num_sms, stream);
     default: return cudaErrorInvalidValue;
@@ -708,12 +762,12 @@ static cudaError_t launch_ctas(const CUtensorMap& tmA, const CUtensorMap& tmB, c
 }
 
 cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                                cudaStream_t stream) {
+                                cudaStream_t stream, const CUtensorMap* accum) {
   if (args.n_groups_cap > MAX_GROUPS) return cudaErrorInvalidValue;
   if (args.mode == kFwd1 && args.N % 128 != 0) return cudaErrorInvalidValue;
   if (args.N % 32 != 0) return cudaErrorInvalidValue;
-  if (args.ctas == 2) return launch_ctas<2>(tmA, tmB, args, num_sms, stream);
-  return launch_ctas<1>(tmA, tmB, args, num_sms, stream);
+  if (args.ctas == 2) return launch_ctas<2>(tmA, tmB, args, num_sms, stream, accum);
+  return launch_ctas<1>(tmA, tmB, args, num_sms, stream, accum);
 }
 
 }  // namespace epb

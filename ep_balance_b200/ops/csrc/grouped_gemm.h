@@ -43,8 +43,6 @@ struct GemmArgs {
   const float* row_scale;      // kFwd1: optional [T] factor folded into act (the row's gate weight); null: 1
   void* const* out_ptrs;       // scatter modes: R peer buffers [units, N] (null -> local out0)
   const int2* meta;            // scatter modes: {src rank, row in that rank's buffer} per row
-  float* accum;                // kWgrad, may be null: fp32 [home_cap, M_out, N]; the gradient of a slot below home_cap is added
-                               // there from the fp32 accumulators and its slot of out0 is not written
   int* status;
   unsigned long long wait_ns;  // budget of the waits below (0: the library default)
   // ---- operand gating (each may be null).  The TMA producer polls before the first load of a tile:
@@ -86,7 +84,12 @@ bool make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t co
 bool make_tmap_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols,
                   uint32_t box_cols, uint32_t box_rows);
 
+// fp32 accumulator of kWgrad: [slots, rows, cols], box {32, 32, 1}, 128-byte swizzle.
+bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols);
+
+// accum (kWgrad, may be null): map of the fp32 accumulator [home_cap, M_out, N].  The gradient of a slot below home_cap is added
+// there from the fp32 sums and its slot of out0 is not written.
 cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                                cudaStream_t stream);
+                                cudaStream_t stream, const CUtensorMap* accum = nullptr);
 
 }  // namespace epb

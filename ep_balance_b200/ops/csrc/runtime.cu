@@ -141,6 +141,10 @@ MoeRuntime::MoeRuntime(const LayerConfig& cfg, const std::map<std::string, uint6
   tmap2(&tm_dh_mn_, ptr<void>("hbuf"), T, 2 * F, 64, 64);
   tmap2(&tm_x_mn_, ptr<void>("xbuf"), T, H, 64, 64);
 
+  if (fused_accum() && (!make_tmap_accum(&tm_acc1_, ptr<void>("acc_gw1"), c.home_cap, 2 * F, H) ||
+                        !make_tmap_accum(&tm_acc2_, ptr<void>("acc_gw2"), c.home_cap, H, F)))
+    throw std::runtime_error("MoeRuntime: cuTensorMapEncodeTiled (accumulators) failed");
+
   // optional block-scaled fp8 forward
   if (ptr<void>("w1q", false) != nullptr) {
     if (c.H % 128 || c.F % 128) throw std::runtime_error("MoeRuntime: the fp8 path needs H % 128 == 0 and F % 128 == 0");
@@ -330,10 +334,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
     g.done_R = cfg_.R;
   }
   g.row_scale = extra.row_scale;
-  if (extra.accum != nullptr) {
-    g.accum = extra.accum;
-    g.home_cap = cfg_.home_cap;
-  }
+  if (extra.accum != nullptr) g.home_cap = cfg_.home_cap;
   if (extra.comm != nullptr) {
     g.comm = *extra.comm;
     g.trace = ptr<unsigned long long>("gemm_trace", false);  // optional: phase timestamps of the fused kernels
@@ -342,7 +343,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
   if (extra.narrow)  // a: token rows, b: weights, as for the wide kernel
     check(launch_narrow_gemm(b, a, g, cfg_.num_sms, stream), extra.comm ? "narrow_gemm+transport" : "narrow_gemm");
   else
-    check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
+    check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream, extra.accum), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
 }
 
 // An inference batch with few rows per expert reads the weights once and does little else.  (About num_units rows reach
@@ -557,12 +558,12 @@ void MoeRuntime::dispatch_grads(const void* dout, int num_units, cudaStream_t st
 // fp32 accumulation over micro-batches happens in the Wgrad epilogue for the owned slots: the gradient is added from the
 // fp32 accumulators and never takes the detour through the bf16 slot (one write and one read of 2 bytes a weight, and a
 // rounding).  Replica slots keep bf16: their owner adds them (grad_reduce).
-float* MoeRuntime::fused_accum(const char* name) const { return cfg_.accum_fp32 ? ptr<float>(name, false) : nullptr; }
+bool MoeRuntime::fused_accum() const { return cfg_.accum_fp32 && ptr<float>("acc_gw1", false) != nullptr; }
 
 // No gate: Dgrad2, earlier on this stream, has waited for every gradient row of this rank.
 void MoeRuntime::wgrad2(cudaStream_t stream) {
   GemmExtra x;
-  x.accum = fused_accum("acc_gw2");
+  if (fused_accum()) x.accum = &tm_acc2_;
   gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream, x);
 }
 void MoeRuntime::swiglu_pass(cudaStream_t stream) {
@@ -594,7 +595,7 @@ void MoeRuntime::dgrad2_fused(const void* dout, int num_units, cudaStream_t stre
 }
 void MoeRuntime::wgrad1(cudaStream_t stream) {
   GemmExtra x;
-  x.accum = fused_accum("acc_gw1");
+  if (fused_accum()) x.accum = &tm_acc1_;
   gemm(kWgrad, tm_dh_mn_, tm_x_mn_, cfg_.H, 0, 2 * cfg_.F, ptr<void>("gw1"), nullptr, nullptr, nullptr, stream, x);
 }
 void MoeRuntime::dgrad1(cudaStream_t stream) {
@@ -612,7 +613,7 @@ void MoeRuntime::reduce_dtokens(void* dtokens, float* dprob, int num_tokens, cud
 void MoeRuntime::reduce_weight_grads(cudaStream_t stream) {
   void* acc1 = ptr<void>("acc_gw1", false);
   void* acc2 = ptr<void>("acc_gw2", false);
-  const bool own_done = fused_accum("acc_gw1") != nullptr;  // Wgrad has added the owned slots' own gradients already
+  const bool own_done = fused_accum();  // Wgrad has added the owned slots' own gradients already
   if (cfg_.R <= 1 && (acc1 == nullptr || own_done)) return;
   GradReduceArgs a{};
   a.skip_self = own_done;

@@ -127,7 +127,7 @@ class MoeRuntime {
     int done_slot = 0;   // > 0: signal every peer on this slot when the launch is complete
     const float* row_scale = nullptr;
     const CommArgs* comm = nullptr;
-    float* accum = nullptr;  // Wgrad: fp32 accumulation buffer of the owned slots
+    const CUtensorMap* accum = nullptr;  // Wgrad: fp32 accumulation buffer of the owned slots
     bool narrow = false; // few rows per expert: weights on the M side (narrow_gemm.h)
   };
   void gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int N, int K, int M_out, void* out0, void* out1,
@@ -140,7 +140,7 @@ class MoeRuntime {
   CommArgs comm_forward(const void* tokens, const float* topk_prob, bool pad, bool pull) const;
   CommArgs comm_backward(const void* dout) const;
   void swiglu_pass(cudaStream_t stream);
-  float* fused_accum(const char* name) const;
+  bool fused_accum() const;
   bool peers() const { return cfg_.multi_rank_sync && cfg_.R > 1; }
   UnitReduceWait reduce_wait(int slot) const;
   void tmap2(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t bc, uint32_t br);
@@ -164,6 +164,7 @@ class MoeRuntime {
   // tensor maps (built once: every buffer has a fixed address)
   CUtensorMap tm_x_k_, tm_act_k_, tm_dy_k_, tm_dh_k_;           // K-major A operands
   CUtensorMap tm_w1_k_, tm_w2_k_, tm_w1_mn_, tm_w2_mn_;          // weights as B
+  CUtensorMap tm_acc1_, tm_acc2_;                                // fp32 gradient accumulators
   CUtensorMap tm_x_n_, tm_act_n_;                                // token rows as the narrow kernel's N operand
   CUtensorMap tm_dy_mn_, tm_act_mn_, tm_dh_mn_, tm_x_mn_;        // Wgrad operands (MN-major)
   bool fp8_ = false;
