@@ -15,6 +15,7 @@
 #include "narrow_gemm.h"
 #include "onesided.h"
 #include "optim.h"
+#include "ragged_gemm.h"
 #include "rope.h"
 #include "route.h"
 #include "router.h"
@@ -156,6 +157,12 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
   g.out1 = out1.has_value() ? memory(*out1, "out1") : nullptr;
   CUtensorMap tmA, tmB;
   const uint64_t T = a.size(0);
+  // the CTA-pair kernel of the modes whose rows are token rows (kDgrad2 keeps them on the M side)
+  bool ragged = !narrow && ctas == 2 && mode != epb::kWgrad && mode != epb::kDgrad2;
+  if (ragged && mode == epb::kDgrad1 && b.size(2) % 64 != 0) {  // its weights come in blocks of 64 columns
+    ragged = false;
+    g.ctas = 1;
+  }
   const uint32_t box_rows = narrow ? epb::kNarrowBoxRows : 128;  // token rows of a box
   TORCH_CHECK(!narrow || mode == epb::kFwd1 || mode == epb::kFwd2, "the narrow kernel has modes fwd1 and fwd2");
   bool ok = true;
@@ -171,14 +178,16 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
       g.N = (int)b.size(1) / 2;
       g.K = (int)a.size(1);
       ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
-           epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 128);
+           (ragged ? epb::make_tmap_gate_up(&tmB, memory(b, "b"), b.size(0), g.N, b.size(2))
+                   : epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 128));
       break;
     case epb::kDgrad1:
     case epb::kDgrad2:
       g.N = (int)b.size(2);
       g.K = (int)a.size(1);
-      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, 128) &&
-           epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 64);
+      ok = epb::make_tmap_2d(&tmA, memory(a, "a"), T, a.size(1), 64, box_rows) &&
+           (ragged ? epb::make_tmap_blocks(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2))
+                   : epb::make_tmap_3d(&tmB, memory(b, "b"), b.size(0), b.size(1), b.size(2), 64, 64));
       break;
     case epb::kWgrad:
       g.N = (int)b.size(1);
@@ -192,6 +201,10 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
   TORCH_CHECK(ok, "cuTensorMapEncodeTiled failed");
   if (narrow) {
     cuda_check(epb::launch_narrow_gemm(tmB, tmA, g, (int)num_sms, current_stream()), "launch_narrow_gemm");
+    return;
+  }
+  if (ragged) {
+    cuda_check(epb::launch_ragged_gemm(tmB, tmA, g, (int)num_sms, current_stream()), "launch_ragged_gemm");
     return;
   }
   cuda_check(epb::launch_grouped_gemm(tmA, tmB, g, (int)num_sms, current_stream()), "launch_grouped_gemm");

@@ -9,6 +9,9 @@
 // carry two more warps that move token (or gradient) rows and replica weights between ranks (comm.cuh) while the
 // producer warp gates each tile's first load on the arrival counter of that tile.
 //
+// As a CTA pair this kernel computes the weight gradients (and kDgrad2); the other modes of a pair have the weights on the M
+// side (ragged_gemm.cu).  As a single CTA it computes all modes.
+//
 // This replaces torch._grouped_mm / torch.bmm plus the unfused activation, slot sort, index_add
 // and activation-gradient kernels of the reference (eplb/integration/grouped_mlp.py:88-137,
 // 219-236; overlap.py:368-408; manual_block.py:184-221, 293-342).
@@ -35,21 +38,15 @@ constexpr int kStageWarpBytes = 4096;  // staging tile of one epilogue warp
 // two SMs) computes a 256 x 256 tile with tcgen05.mma.cta_group::2; each CTA stages its own 128
 // rows of A and its own 128 columns of B, so per-SM operand traffic drops from 48 KB to 32 KB per
 // k-block and the shared-memory ring deepens from 4 to 6 stages.
-// The fused-transport variants (kComm != 0) give 64 KB of the operand ring to the transport warps' copy rings.
-// A stage holds kSub k-blocks.  Every tcgen05.commit leaves the tensor pipe idle for some 45 cycles, and a k-block is only
-// 512 cycles of MMAs: with two commits a k-block (one per CTA of the pair) the pipe was at most 78 % busy with no loads and no
-// epilogue at all, with one multicast commit 84 %, with one per two k-blocks 96 %.  Wgrad (K = the rows of a group, often a
-// dozen k-blocks) and the fused-transport variants (four stages) keep one k-block a stage.
+// The fused-transport variants (kComm != 0, single CTA) give one stage of the ring to the transport warps' copy rings.
 // The accumulating Wgrad (kAccum) holds 128 KB of the fp32 accumulator instead of half its operand ring.
-template <int kCtas, int kComm = 0, int kMode = -1, bool kAccum = false>
+template <int kCtas, int kComm = 0, bool kAccum = false>
 struct Geometry {
-  static constexpr int kSub = kCtas == 2 && kComm == 0 && kMode != kWgrad ? 2 : 1;
-  static constexpr int STAGES = kAccum ? (kCtas == 2 ? 3 : 2) : ((kCtas == 2 ? 6 : 4) - (kComm ? (kCtas == 2 ? 2 : 1) : 0)) / kSub;
+  static constexpr int STAGES = kAccum ? (kCtas == 2 ? 3 : 2) : (kCtas == 2 ? 6 : 4) - (kComm ? 1 : 0);
   static constexpr int STAGE_WARP_BYTES = kAccum ? 4 * kStageWarpBytes : kStageWarpBytes;  // of one epilogue warp
-  static constexpr int COMM_SLOTS = kCtas == 2 ? 8 : 6;  // ring slots of a transport warp: batches of 4 (3) segments of 4 KB
+  static constexpr int COMM_SLOTS = 6;  // ring slots of a transport warp: batches of 3 segments of 4 KB
   static constexpr int B_BYTES = BN * BK * 2 / kCtas;
-  static constexpr int SUB_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGE_BYTES = SUB_BYTES * kSub;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TILE_M = BM * kCtas;
 };
 constexpr int NUM_THREADS = 320;  // TMA warp + MMA warp + 8 epilogue warps
@@ -196,8 +193,9 @@ template <int kMode, int kCtas, int kComm, bool kAccum>
 __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmAcc, const __grid_constant__ GemmArgs args) {
-  using G = Geometry<kCtas, kComm, kMode, kAccum>;
-  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, SUB_BYTES = G::SUB_BYTES, TILE_M = G::TILE_M;
+  static_assert(kCtas == 1 || kComm == 0, "the fused transport of a CTA pair is in ragged_gemm.cu");
+  using G = Geometry<kCtas, kComm, kAccum>;
+  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, TILE_M = G::TILE_M;
   constexpr bool kAMn = kMode == kWgrad;
   constexpr bool kBMn = kMode == kWgrad || kMode == kDgrad2 || kMode == kDgrad1;
 
@@ -280,38 +278,30 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const int n_off = t.nt * BN + cta_rank * (BN / 2) * (kCtas - 1);  // this CTA's columns of B
           constexpr int kBoxesB = 4 / kCtas;                          // 64-wide MN-major boxes of B
           const int kblocks = k_blocks<kMode>(shape, t);
-          for (int kb0 = 0; kb0 < kblocks; kb0 += G::kSub) {
+          for (int kb = 0; kb < kblocks; ++kb) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_v, args.status, 1)) {
               go = 0;
               break;
             }
+            uint8_t* sA = tiles + stage * STAGE_BYTES;
+            uint8_t* sB = sA + A_BYTES;
             uint64_t* fb = &full_bar[stage];
-            const int subs = min(G::kSub, kblocks - kb0);
-            if (cta_rank == 0) mbar_expect_tx(fb, subs * SUB_BYTES * kCtas);  // both CTAs' bytes land on the leader's barrier
-            for (int sub = 0; sub < subs; ++sub) {
-              const int kb = kb0 + sub;
-              uint8_t* sA = tiles + stage * STAGE_BYTES + sub * SUB_BYTES;
-              uint8_t* sB = sA + A_BYTES;
-              if (kMode == kWgrad) {
-                const int krow = t.row0 + kb * BK;
-                for (int i = 0; i < 2; ++i) tma2<kCtas>(sA + i * 8192, &tmA, fb, m_off + 64 * i, krow);
-                for (int j = 0; j < kBoxesB; ++j) tma2<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, krow);
+            if (cta_rank == 0) mbar_expect_tx(fb, STAGE_BYTES * kCtas);  // both CTAs' bytes land on the leader's barrier
+            if (kMode == kWgrad) {
+              const int krow = t.row0 + kb * BK;
+              for (int i = 0; i < 2; ++i) tma2<kCtas>(sA + i * 8192, &tmA, fb, m_off + 64 * i, krow);
+              for (int j = 0; j < kBoxesB; ++j) tma2<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, krow);
+            } else {
+              tma2<kCtas>(sA, &tmA, fb, kb * BK, t.row0 + m_off);
+              if (kMode == kFwd1) {
+                // gate rows [nt*128, +128) and up rows [F + nt*128, +128)
+                tma3<kCtas>(sB, &tmB, fb, kb * BK, t.nt * 128, t.wslot);
+                tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, args.N + t.nt * 128, t.wslot);
+              } else if (kBMn) {
+                for (int j = 0; j < kBoxesB; ++j) tma3<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, kb * BK, t.wslot);
               } else {
-                tma2<kCtas>(sA, &tmA, fb, kb * BK, t.row0 + m_off);
-                if (kMode == kFwd1) {
-                  // gate rows [nt*128, +128) and up rows [F + nt*128, +128): one half per CTA of a pair
-                  if (kCtas == 2) {
-                    tma3<kCtas>(sB, &tmB, fb, kb * BK, cta_rank * args.N + t.nt * 128, t.wslot);
-                  } else {
-                    tma3<kCtas>(sB, &tmB, fb, kb * BK, t.nt * 128, t.wslot);
-                    tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, args.N + t.nt * 128, t.wslot);
-                  }
-                } else if (kBMn) {
-                  for (int j = 0; j < kBoxesB; ++j) tma3<kCtas>(sB + j * 8192, &tmB, fb, n_off + 64 * j, kb * BK, t.wslot);
-                } else {
-                  tma3<kCtas>(sB, &tmB, fb, kb * BK, n_off, t.wslot);
-                  if (kCtas == 1) tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, n_off + 128, t.wslot);
-                }
+                tma3<kCtas>(sB, &tmB, fb, kb * BK, n_off, t.wslot);
+                tma3<kCtas>(sB + 16384, &tmB, fb, kb * BK, n_off + 128, t.wslot);
               }
             }
             if (++stage == STAGES) {
@@ -356,30 +346,24 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const uint32_t idesc = make_idesc(kAMn, kBMn, ncols, TILE_M);
         bool failed = false;
         const int kblocks = k_blocks<kMode>(shape, t);
-        for (int kb0 = 0; kb0 < kblocks; kb0 += G::kSub) {
+        for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_v, args.status, 3)) {
             failed = true;
             break;
           }
           tc_fence_after();
-          const int subs = min(G::kSub, kblocks - kb0);
+          const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES);
+          const uint32_t sB = sA + A_BYTES;
+          const uint64_t da = kAMn ? make_desc(sA, 8192, 1024) : make_desc(sA, 16, 1024);
+          const uint64_t db = kBMn ? make_desc(sB, 8192, 1024) : make_desc(sB, 16, 1024);
+          constexpr uint32_t a_step = kAMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
+          constexpr uint32_t b_step = kBMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
 #pragma unroll
-          for (int sub = 0; sub < G::kSub; ++sub) {
-            if (sub >= subs) break;
-            const uint32_t sA = smem_u32(tiles + stage * STAGE_BYTES + sub * SUB_BYTES);
-            const uint32_t sB = sA + A_BYTES;
-            const uint64_t da = kAMn ? make_desc(sA, 8192, 1024) : make_desc(sA, 16, 1024);
-            const uint64_t db = kBMn ? make_desc(sB, 8192, 1024) : make_desc(sB, 16, 1024);
-            constexpr uint32_t a_step = kAMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
-            constexpr uint32_t b_step = kBMn ? (UMMA_K * 128) >> 4 : (UMMA_K * 2) >> 4;
-#pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-              const uint32_t acc = (kb0 | sub | k) ? 1u : 0u;
-              if (kCtas == 2)
-                umma_bf16_pair(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
-              else
-                umma_bf16(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
-            }
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            if (kCtas == 2)
+              umma_bf16_pair(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, (kb | k) ? 1u : 0u);
+            else
+              umma_bf16(tmem_d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, (kb | k) ? 1u : 0u);
           }
           // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
           if (kCtas == 2) umma_commit_both(&empty_bar[stage]);
@@ -646,12 +630,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 template <int kCtas, int kComm, bool kAccum = false>
-constexpr size_t smem_bytes() {  // the same for every mode: a stage of two k-blocks counts as two
-  using G = Geometry<kCtas, kComm, kWgrad, kAccum>;
+constexpr size_t smem_bytes() {
+  using G = Geometry<kCtas, kComm, kAccum>;
   return G::STAGES * G::STAGE_BYTES + 1024 /*align*/ + kCtrlBytes /*barriers, flags, tile prefix*/ + 8 * G::STAGE_WARP_BYTES /*staging*/ +
          (kComm ? COMM_WARPS * comm_warp_bytes<Geometry<kCtas, kComm>::COMM_SLOTS>() : 0) /*transport rings*/;
 }
-static_assert(smem_bytes<2, 1>() <= 232448 && smem_bytes<1, 1>() <= 232448 && smem_bytes<2, 0>() <= 232448 &&
+static_assert(smem_bytes<1, 1>() <= 232448 && smem_bytes<2, 0>() <= 232448 &&
                   smem_bytes<2, 0, true>() <= 232448 && smem_bytes<1, 0, true>() <= 232448, "shared memory budget");
 
 // ---------------------------------------------------------------- tensor maps
@@ -699,6 +683,22 @@ bool make_tmap_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t r
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+static bool make_tmap_4d(CUtensorMap* out, const void* base, const cuuint64_t (&dims)[4], const cuuint64_t (&strides)[3]) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint32_t box[4] = {64, 64, 2, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool make_tmap_blocks(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols) {
+  return cols % 64 == 0 && make_tmap_4d(out, base, {64, rows, cols / 64, slots}, {cols * 2, 128, rows * cols * 2});
+}
+bool make_tmap_gate_up(CUtensorMap* out, const void* base, uint64_t slots, uint64_t F, uint64_t K) {
+  return make_tmap_4d(out, base, {K, F, 2, slots}, {K * 2, F * K * 2, 2 * F * K * 2});
+}
+
 bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
@@ -738,36 +738,36 @@ static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, c
   return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, kAccum ? *accum : tmA, args);
 }
 
-template <int kCtas>
-static cudaError_t launch_ctas(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                               cudaStream_t stream, const CUtensorMap* accum) {
-  const bool comm = args.comm.do_dispatch || args.comm.do_pad || args.comm.do_pull;
-  if (comm) {
-    // fused transport exists for the two GEMMs that consume freshly dispatched rows
-    if (args.mode == kFwd1) return launch_mode<kFwd1, kCtas, 1>(tmA, tmB, args, num_sms, stream);
-    if (args.mode == kDgrad1) return launch_mode<kDgrad1, kCtas, 1>(tmA, tmB, args, num_sms, stream);
-    return cudaErrorInvalidValue;
-  }
-  switch (args.mode) {
-    case kFwd1: return launch_mode<kFwd1, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kFwd2: return launch_mode<kFwd2, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kDgrad2: return launch_mode<kDgrad2, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kDgrad1: return launch_mode<kDgrad1, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kWgrad:
-      if (accum != nullptr) return launch_mode<kWgrad, kCtas, 0, true>(tmA, tmB, args, num_sms, stream, accum);
-      return launch_mode<kWgrad, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    case kPlain: return launch_mode<kPlain, kCtas, 0>(tmA, tmB, args, num_sms, stream);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
 cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
                                 cudaStream_t stream, const CUtensorMap* accum) {
   if (args.n_groups_cap > MAX_GROUPS) return cudaErrorInvalidValue;
   if (args.mode == kFwd1 && args.N % 128 != 0) return cudaErrorInvalidValue;
   if (args.N % 32 != 0) return cudaErrorInvalidValue;
-  if (args.ctas == 2) return launch_ctas<2>(tmA, tmB, args, num_sms, stream, accum);
-  return launch_ctas<1>(tmA, tmB, args, num_sms, stream, accum);
+  const bool comm = args.comm.do_dispatch || args.comm.do_pad || args.comm.do_pull;
+  if (args.ctas == 2) {  // the other modes of a CTA pair have the weights on the M side: ragged_gemm.cu
+    if (comm) return cudaErrorInvalidValue;
+    if (args.mode == kDgrad2) return launch_mode<kDgrad2, 2, 0>(tmA, tmB, args, num_sms, stream);
+    if (args.mode != kWgrad) return cudaErrorInvalidValue;
+    if (accum != nullptr) return launch_mode<kWgrad, 2, 0, true>(tmA, tmB, args, num_sms, stream, accum);
+    return launch_mode<kWgrad, 2, 0>(tmA, tmB, args, num_sms, stream);
+  }
+  if (comm) {
+    // fused transport exists for the two GEMMs that consume freshly dispatched rows
+    if (args.mode == kFwd1) return launch_mode<kFwd1, 1, 1>(tmA, tmB, args, num_sms, stream);
+    if (args.mode == kDgrad1) return launch_mode<kDgrad1, 1, 1>(tmA, tmB, args, num_sms, stream);
+    return cudaErrorInvalidValue;
+  }
+  switch (args.mode) {
+    case kFwd1: return launch_mode<kFwd1, 1, 0>(tmA, tmB, args, num_sms, stream);
+    case kFwd2: return launch_mode<kFwd2, 1, 0>(tmA, tmB, args, num_sms, stream);
+    case kDgrad2: return launch_mode<kDgrad2, 1, 0>(tmA, tmB, args, num_sms, stream);
+    case kDgrad1: return launch_mode<kDgrad1, 1, 0>(tmA, tmB, args, num_sms, stream);
+    case kWgrad:
+      if (accum != nullptr) return launch_mode<kWgrad, 1, 0, true>(tmA, tmB, args, num_sms, stream, accum);
+      return launch_mode<kWgrad, 1, 0>(tmA, tmB, args, num_sms, stream);
+    case kPlain: return launch_mode<kPlain, 1, 0>(tmA, tmB, args, num_sms, stream);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace epb

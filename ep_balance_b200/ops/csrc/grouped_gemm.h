@@ -84,6 +84,13 @@ bool make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t co
 bool make_tmap_3d(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols,
                   uint32_t box_cols, uint32_t box_rows);
 
+// Views that let ONE copy bring 128 columns (or 64 gate and their 64 up rows), 16 KB: a copy of 8 KB costs the copy engine nearly
+// as much.
+// MN-major operand [slots, rows, cols] in blocks of 64 columns, cols % 64 == 0: dims {64, rows, cols / 64, slots}, box {64, 64, 2, 1}.
+bool make_tmap_blocks(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols);
+// Gate and up rows [slots, 2 F, K], K-major: dims {K, F, 2, slots}, box {64, 64, 2, 1}.
+bool make_tmap_gate_up(CUtensorMap* out, const void* base, uint64_t slots, uint64_t F, uint64_t K);
+
 // fp32 accumulator of kWgrad: [slots, rows, cols], box {32, 32, 1}, 128-byte swizzle.
 bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols);
 

@@ -321,7 +321,7 @@ struct Geo {
   static constexpr int B_HALF = kBN / 2;                     // weight rows staged per CTA
   static constexpr int A_BYTES = BM * BK, B_BYTES = B_HALF * BK, TILE_BYTES = A_BYTES + B_BYTES;
   static constexpr int SF_BYTES = 512 + 512 * (kBN / 128);   // this CTA's SFA chunk + the SFB chunks of the whole tile
-  // A stage holds kSub k-blocks: a tcgen05.commit costs the tensor pipe idle cycles (grouped_gemm.cu), so there is one per stage.
+  // A stage holds kSub k-blocks: a tcgen05.commit costs the tensor pipe idle cycles (ragged_gemm.cu), so there is one per stage.
   static constexpr int kSub = 2;
   static constexpr int STAGES = 3;
   static constexpr int STAGE_BYTES = kSub * TILE_BYTES;

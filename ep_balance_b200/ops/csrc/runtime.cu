@@ -18,6 +18,8 @@
 
 #include <stdexcept>
 
+#include "ragged_gemm.h"
+
 namespace epb {
 
 template <typename T>
@@ -122,19 +124,26 @@ MoeRuntime::MoeRuntime(const LayerConfig& cfg, const std::map<std::string, uint6
     ptr<void>(name);
 
   const uint64_t T = c.row_capacity, H = c.H, F = c.F, S = c.w_slots;
-  // K-major A operands: box {64 k, 128 rows}
+  // K-major token rows: box {64 k, 128 rows}
   tmap2(&tm_x_k_, ptr<void>("xbuf"), T, H, 64, 128);
   tmap2(&tm_act_k_, ptr<void>("act"), T, F, 64, 128);
   tmap2(&tm_dy_k_, ptr<void>("dybuf"), T, H, 64, 128);
   tmap2(&tm_dh_k_, ptr<void>("hbuf"), T, 2 * F, 64, 128);
   tmap2(&tm_x_n_, ptr<void>("xbuf"), T, H, 64, kNarrowBoxRows);
   tmap2(&tm_act_n_, ptr<void>("act"), T, F, 64, kNarrowBoxRows);
-  // weights, K-major B: box {64 k, 128 n, 1}
+  // weights, K-major: box {64 k, 128 n, 1}
   tmap3(&tm_w1_k_, ptr<void>("w1"), S, 2 * F, H, 64, 128);
   tmap3(&tm_w2_k_, ptr<void>("w2"), S, H, F, 64, 128);
-  // weights, MN-major B: box {64 n, 64 k, 1}
-  tmap3(&tm_w1_mn_, ptr<void>("w1"), S, 2 * F, H, 64, 64);
-  tmap3(&tm_w2_mn_, ptr<void>("w2"), S, H, F, 64, 64);
+  if (c.gemm_ctas == 2) {
+    // GEMM1's weights and the weights in MN-major order: 64 gate and 64 up rows, 128 columns a copy
+    if (!make_tmap_gate_up(&tm_w1_g_, ptr<void>("w1"), S, F, H) || !make_tmap_blocks(&tm_w1_mn_, ptr<void>("w1"), S, 2 * F, H) ||
+        !make_tmap_blocks(&tm_w2_mn_, ptr<void>("w2"), S, H, F))
+      throw std::runtime_error("MoeRuntime: cuTensorMapEncodeTiled (4-D) failed");
+  } else {
+    // weights, MN-major: box {64 n, 64 k, 1}
+    tmap3(&tm_w1_mn_, ptr<void>("w1"), S, 2 * F, H, 64, 64);
+    tmap3(&tm_w2_mn_, ptr<void>("w2"), S, H, F, 64, 64);
+  }
   // Wgrad operands, MN-major: box {64 cols, 64 rows}
   tmap2(&tm_dy_mn_, ptr<void>("dybuf"), T, H, 64, 64);
   tmap2(&tm_act_mn_, ptr<void>("act"), T, F, 64, 64);
@@ -340,8 +349,11 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
     g.trace = ptr<unsigned long long>("gemm_trace", false);  // optional: phase timestamps of the fused kernels
     if (g.trace != nullptr) g.trace += mode == kFwd1 ? 0 : 12;
   }
-  if (extra.narrow)  // a: token rows, b: weights, as for the wide kernel
+  // a: token rows, b: weights
+  if (extra.narrow)
     check(launch_narrow_gemm(b, a, g, cfg_.num_sms, stream), extra.comm ? "narrow_gemm+transport" : "narrow_gemm");
+  else if (mode != kWgrad && cfg_.gemm_ctas == 2)
+    check(launch_ragged_gemm(b, a, g, cfg_.num_sms, stream), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
   else
     check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream, extra.accum), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
 }
@@ -351,13 +363,16 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
 bool MoeRuntime::use_narrow(int num_units) const { return num_units <= kNarrowRowsPerSlot * cfg_.w_slots; }
 bool MoeRuntime::use_narrow_fp8(int num_units) const { return num_units < kNarrowFp8RowsPerSlot * cfg_.w_slots; }
 
+// GEMM1's weights: the CTA-pair kernel loads gate and up rows together.
+const CUtensorMap& MoeRuntime::w1_map(bool narrow) const { return narrow || cfg_.gemm_ctas == 1 ? tm_w1_k_ : tm_w1_g_; }
+
 void MoeRuntime::gemm1(cudaStream_t stream, bool train, bool narrow) {
   GemmExtra x;
   x.narrow = narrow;
   x.gate = 1;
   x.gate_pull = true;
   x.row_scale = ptr<const float>("rowp");
-  gemm(kFwd1, narrow ? tm_x_n_ : tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
+  gemm(kFwd1, narrow ? tm_x_n_ : tm_x_k_, w1_map(narrow), cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
        nullptr, nullptr, stream, x);
 }
 void MoeRuntime::gemm1_fused(const void* tokens, const float* topk_prob, int num_units, cudaStream_t stream, bool train) {
@@ -369,7 +384,7 @@ void MoeRuntime::gemm1_fused(const void* tokens, const float* topk_prob, int num
   x.gate_pull = true;
   x.row_scale = ptr<const float>("rowp");
   x.comm = &a;
-  gemm(kFwd1, x.narrow ? tm_x_n_ : tm_x_k_, tm_w1_k_, cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
+  gemm(kFwd1, x.narrow ? tm_x_n_ : tm_x_k_, w1_map(x.narrow), cfg_.F, cfg_.H, 0, train ? ptr<void>("hbuf") : nullptr, ptr<void>("act"),
        nullptr, nullptr, stream, x);
 }
 void MoeRuntime::gemm2(cudaStream_t stream, bool narrow) {

@@ -141,6 +141,7 @@ class MoeRuntime {
   CommArgs comm_backward(const void* dout) const;
   void swiglu_pass(cudaStream_t stream);
   bool fused_accum() const;
+  const CUtensorMap& w1_map(bool narrow) const;
   bool peers() const { return cfg_.multi_rank_sync && cfg_.R > 1; }
   UnitReduceWait reduce_wait(int slot) const;
   void tmap2(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t bc, uint32_t br);
@@ -164,6 +165,7 @@ class MoeRuntime {
   // tensor maps (built once: every buffer has a fixed address)
   CUtensorMap tm_x_k_, tm_act_k_, tm_dy_k_, tm_dh_k_;           // K-major A operands
   CUtensorMap tm_w1_k_, tm_w2_k_, tm_w1_mn_, tm_w2_mn_;          // weights as B
+  CUtensorMap tm_w1_g_;                                          // gate and up blocks of the CTA-pair kernel
   CUtensorMap tm_acc1_, tm_acc2_;                                // fp32 gradient accumulators
   CUtensorMap tm_x_n_, tm_act_n_;                                // token rows as the narrow kernel's N operand
   CUtensorMap tm_dy_mn_, tm_act_mn_, tm_dh_mn_, tm_x_mn_;        // Wgrad operands (MN-major)
