@@ -35,6 +35,7 @@ struct GemmArgs {
   // problem extents
   int N;                       // output columns (kFwd1: F, gate/up pairs; kWgrad: columns of Q)
   int K;                       // reduction extent (ignored for kWgrad: the group's padded rows)
+  int pad_rows;                // kFwd1 of a CTA pair, out0 kept: zeros follow a group's rows up to a multiple of this (0: 256)
   int M_out;                   // kWgrad only: rows of the output (columns of P)
   // epilogue operands
   void* out0;                  // kFwd1: h [T, 2N] (null: not kept, and no padding row of act is written);  kDgrad2: h (in/out);  kWgrad: dW [slots, M_out, N];

@@ -54,7 +54,7 @@ struct Tile {
   int wt;        // weight tile
   int row, n;    // first buffer row and real rows
   int cols;      // n rounded up to 32: columns of the MMA
-  int pad;       // rows after the n real ones up to the group's end (last tile of a group; else 0)
+  int pad;       // rows of zeros that kFwd1 writes after the n real ones (last tile of a group; else 0)
   int wslot;
 };
 
@@ -71,7 +71,7 @@ __device__ __forceinline__ bool find_tile(const GemmArgs& a, int n_groups, int m
   out.row = a.group_off[g] + tt * per;
   out.n = min(per, rows - tt * per);
   out.cols = round_up(out.n, 32);
-  out.pad = tt == count - 1 ? round_up(rows, NT) - rows : 0;
+  out.pad = tt == count - 1 ? round_up(rows, a.pad_rows > 0 ? a.pad_rows : NT) - rows : 0;
   out.wslot = a.group_wslot[g];
   return true;
 }

@@ -378,7 +378,12 @@ __global__ void __launch_bounds__(256) swiglu_backward_kernel(SwigluBwdArgs a) {
   const uint4* dact = reinterpret_cast<const uint4*>(a.dact);
   uint4* h = reinterpret_cast<uint4*>(a.h);
   const int warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < rows; r += warps) {
+  int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  int2 ahead = r < rows && a.meta != nullptr ? a.meta[r] : make_int2(0, 0);  // looked up a row ahead
+  for (; r < rows; r += warps) {
+    const int2 m = ahead;
+    if (a.meta != nullptr && r + warps < rows) ahead = a.meta[r + warps];
+    if (m.x < 0) continue;  // a padding row: GEMM1 left zeros where Wgrad reads
     const float p = a.rowp != nullptr ? a.rowp[r] : 1.f;
     uint4* hrow = h + (size_t)r * (2 * vec_per_row);
     const uint4* drow = dact + (size_t)r * vec_per_row;
@@ -406,10 +411,7 @@ __global__ void __launch_bounds__(256) swiglu_backward_kernel(SwigluBwdArgs a) {
     }
     if (a.dprob_ptrs != nullptr) {
       for (int off = 16; off > 0; off >>= 1) dot += __shfl_down_sync(kFull, dot, off);
-      if (lane == 0) {
-        const int2 m = a.meta[r];
-        if (m.x >= 0) a.dprob_ptrs[m.x][m.y] = dot;
-      }
+      if (lane == 0) a.dprob_ptrs[m.x][m.y] = dot;
     }
   }
 }

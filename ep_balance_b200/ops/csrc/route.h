@@ -71,6 +71,9 @@ cudaError_t launch_route_assign(const RouteArgs& a, cudaStream_t stream);
 // the weight (and computes the gate-weight gradient) in its SwiGLU-gradient pass.
 // Reference counterparts: all_to_all_single dispatch + slot sort (eplb/integration/comm.py:18-36,
 // eplb_manager.py:1067-1105), replica broadcast (overlap.py:113-148).
+// Wgrad contracts over a group's rows in blocks of this many: the padding up to there has to be zero.
+constexpr int kWgradRows = 64;
+
 struct CommArgs {
   int do_dispatch, do_pad, do_pull;
   int R, me, E, H, topk, row_capacity;

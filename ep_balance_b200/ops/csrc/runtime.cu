@@ -319,6 +319,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
   g.N = N;
   g.K = K;
   g.M_out = M_out;
+  g.pad_rows = kWgradRows;
   g.out0 = out0;
   g.out1 = out1;
   g.out_ptrs = out_ptrs;
