@@ -95,7 +95,12 @@ void solve_plan(torch::Tensor omega, torch::Tensor dom, torch::Tensor cost, torc
                 torch::Tensor control, torch::Tensor sync, torch::Tensor status) {
   const c10::cuda::CUDAGuard guard(device_with_memory(omega));
   epb::SolverParams p{};
-  p.omega = dptr<const int32_t>(omega, "omega", torch::kInt32);
+  if (omega.scalar_type() == torch::kInt64) {
+    p.omega = reinterpret_cast<const int32_t*>(dptr<const int64_t>(omega, "omega", torch::kInt64));
+    p.omega_stride = 2;
+  } else {
+    p.omega = dptr<const int32_t>(omega, "omega", torch::kInt32);
+  }
   p.dom = dptr<const int32_t>(dom, "dom", torch::kInt32);
   p.cost = dptr<const int32_t>(cost, "cost", torch::kInt32);
   p.main_rank = dptr<const int32_t>(main_rank, "main_rank", torch::kInt32);

@@ -24,6 +24,8 @@
 namespace epb {
 namespace {
 
+__device__ __forceinline__ const int32_t* omega_at(const SolverParams& p, size_t i) { return p.omega + i * p.omega_stride; }
+
 constexpr int kWarp = 32;
 constexpr int kRouteThreads = 512;  // CTA of the routing launch
 constexpr unsigned kFull = 0xffffffffu;
@@ -188,7 +190,7 @@ __device__ int phase0_domain(const SolverParams& p, Smem& s, int d) {
     long long T = 0;
     const int owner = __ldg(p.main_rank + e);
     const long long wb = __ldg(p.weight_bytes + e);
-    for (int i = 0; i < n; ++i) T += __ldg(p.omega + (size_t)s.dom_ranks[i] * E + e);
+    for (int i = 0; i < n; ++i) T += __ldg(omega_at(p, (size_t)s.dom_ranks[i] * E + e));
     long long rhs = 2 * T * p.s_tok;
     bool valid = p.allow_cross && s.local_idx[owner] < 0 && T > 0 && wb < rhs;
     s.prio[e] = valid ? rhs - wb : -1;
@@ -382,7 +384,7 @@ __device__ void phase1_routing_masks(const SolverParams& p, unsigned long long* 
   const int width = min(pow2_at_least(R), kWarp), sub = tid & (width - 1);
   for (int pair = gtid / width; pair < R * E; pair += gthreads / width) {
     const int src = pair / E, e = pair - src * E;
-    const int need = p.omega[pair];
+    const int need = *omega_at(p, pair);
     const unsigned long long loc = host[e] & dom_mask[src];
     const unsigned long long act = loc ? loc : host[e];
     int* qrow = p.q + (size_t)pair * R;
@@ -395,7 +397,7 @@ __device__ void phase1_routing_masks(const SolverParams& p, unsigned long long* 
       for (int src = 0; src < R; ++src) {
         const unsigned long long loc = host[e] & dom_mask[src];
         const unsigned long long act = loc ? loc : host[e];
-        if ((act >> dst) & 1ull) acc += even_share(p.omega[(size_t)src * E + e], act, dst, u_min);
+        if ((act >> dst) & 1ull) acc += even_share(*omega_at(p, (size_t)src * E + e), act, dst, u_min);
       }
     }
     p.erl[cell] = acc;
@@ -433,7 +435,7 @@ __device__ void phase1_domain_impl(const SolverParams& p, Smem& s, int n, const 
 #pragma unroll
       for (int j = 0; j < 8; ++j) {  // the loads of up to eight sources are in flight together
         const int src = src0 + j * groups;
-        need_b[j] = src < R ? __ldg(p.omega + (size_t)src * E + e) : 0;
+        need_b[j] = src < R ? __ldg(omega_at(p, (size_t)src * E + e)) : 0;
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -513,7 +515,7 @@ __device__ void phase1_routing(const SolverParams& p) {
     for (int dst = lane; dst < R; dst += kWarp) erl[dst] = 0;
     __syncwarp(kFull);
     for (int src = 0; src < R; ++src) {
-      const int need = p.omega[(size_t)src * E + e];
+      const int need = *omega_at(p, (size_t)src * E + e);
       const int dsrc = p.dom[src];
       int cnt_all = 0, cnt_loc = 0;
       for (int base = 0; base < R; base += kWarp) {
@@ -1162,7 +1164,7 @@ __global__ void __launch_bounds__(1024) single_rank_kernel(SolverParams p, RankT
   for (int e0 = 0; e0 < p.E; e0 += blockDim.x) {
     const int e = e0 + tid;
     const bool hosted = e < p.E && p.main_rank[e] == 0;
-    const int need = e < p.E ? __ldcg(p.omega + e) : 0;
+    const int need = e < p.E ? __ldcg(omega_at(p, e)) : 0;
     const int size = hosted && need > 0 ? need : 0;
     const int padded = t.me >= 0 ? round_up(size, t.row_align) : 0;
     int incl = padded, sum = size;

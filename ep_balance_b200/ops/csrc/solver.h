@@ -9,6 +9,8 @@ namespace epb {
 struct SolverParams {
   // inputs (device pointers)
   const int32_t* omega;         // [R, E] units routed from source rank r to expert e
+  int omega_stride = 1;         // int32 words from one entry to the next: 2 reads the low words of an int64 matrix in place, which
+                                // saves a caller that has one (the public solve()) the launch of a conversion
   const int32_t* dom;           // [R] domain of each rank
   const int32_t* cost;          // [R, R] per-token cost
   const int32_t* main_rank;     // [E] owner of each expert

@@ -2,8 +2,7 @@
 
 ``solve_cuda`` is what :func:`ep_balance_b200.solve` calls for CUDA inputs.  Static inputs
 (domain map, cost, owners, weight bytes) are converted to the kernel's dtypes once per
-``(Topology, ProblemSpec)`` pair; per-call work is one int32 cast of ``omega``, one kernel
-launch and one widening cast of ``q``.  Nothing here reads device memory on the host.
+``(Topology, ProblemSpec)`` pair; per-call work is one kernel launch and one widening cast of ``q``.  Nothing here reads device memory on the host.
 Reference counterpart: eplb/cuda_solve.py:71-119.
 """
 
@@ -71,7 +70,8 @@ def solve_cuda(loads: Loads, topo: Topology, spec: ProblemSpec, cfg: EPLBConfig,
     R, E = topo.num_ranks, spec.num_experts
     dom, cost, main_rank, wbytes = _static_inputs(topo, spec, device)
     ws = workspace(R, E, device)
-    omega = loads.omega.to(torch.int32).contiguous()
+    omega = loads.omega if loads.omega.dtype == torch.int64 else loads.omega.to(torch.int32)
+    omega = omega.contiguous()  # of an int64 matrix the kernel reads the low words in place
     x = torch.empty((E, R), dtype=torch.int8, device=device)
     q = torch.empty((R, E, R), dtype=torch.int32, device=device)
     theta = torch.empty(1, dtype=torch.int64, device=device)
