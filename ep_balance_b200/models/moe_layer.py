@@ -166,8 +166,16 @@ def row_capacity(cfg: MoEConfig, world: int) -> int:
     return (rows + tile - 1) // tile * tile
 
 
-def _split3(w: torch.Tensor) -> torch.Tensor:
-    """fp32 ``[A, B]`` -> bf16 ``[3A, B]`` whose three row blocks sum to ``w`` to 24 mantissa bits."""
+def _split3(w: torch.Tensor, transposed: bool = False) -> torch.Tensor:
+    """fp32 ``[A, B]`` -> bf16 ``[3A, B]`` whose three row blocks sum to ``w`` (``transposed``: ``[3B, A]``, to ``w.t()``) to 24
+    mantissa bits.  One kernel, with the bits of the operations below, where nothing is recorded and nobody watches them."""
+    if (w.is_cuda and w.dtype == torch.float32 and not torch.is_grad_enabled() and eager(w) and w.numel() > 0
+            and w.shape[0] <= 65535 * 32):
+        rows, cols = (w.shape[1], w.shape[0]) if transposed else w.shape
+        stacked = torch.empty((3 * rows, cols), dtype=torch.bfloat16, device=w.device)
+        (load().router_split_transposed if transposed else load().router_split)(w.detach().contiguous(), stacked)
+        return stacked
+    w = w.t().contiguous() if transposed else w
     hi = w.to(torch.bfloat16)
     r1 = w - hi.float()
     mid = r1.to(torch.bfloat16)
@@ -197,7 +205,7 @@ class _RouterLinear(torch.autograd.Function):
         g = g.contiguous()
         dx = dw = None
         if ctx.needs_input_grad[1]:
-            g3 = _split3(g.t().contiguous())                                  # [3E, N] bf16
+            g3 = _split3(g, transposed=True)                                  # [3E, N] bf16
             dw = torch.mm(g3, x, out_dtype=torch.float32).view(3, E, -1).sum(0)
         if ctx.needs_input_grad[0]:
             dx = torch.mm(g.to(torch.bfloat16), w.to(torch.bfloat16))

@@ -431,6 +431,15 @@ void router_split(torch::Tensor w, torch::Tensor stacked) {
              "launch_router_split");
 }
 
+void router_split_transposed(torch::Tensor w, torch::Tensor stacked) {
+  const c10::cuda::CUDAGuard guard(device_with_memory(w));
+  TORCH_CHECK(w.dim() == 2 && w.size(0) <= 65535 * 32 && w.size(1) <= 0x7fffffff && stacked.numel() == 3 * w.numel(),
+              "router_split_transposed: w is [N, E] with at most 2097120 rows, stacked [3 E, N]");
+  cuda_check(epb::launch_router_split_transposed(dptr<float>(w, "w", torch::kFloat32), (int)w.size(0), (int)w.size(1),
+                                                 dptr<void>(stacked, "stacked", torch::kBFloat16), current_stream()),
+             "launch_router_split_transposed");
+}
+
 // grad (bf16) of the mean cross-entropy: log_prob fp32 [rows, vocab], targets int64 [rows], weight and grad_out fp32 scalars
 void cross_entropy_backward(torch::Tensor log_prob, torch::Tensor targets, torch::Tensor weight, torch::Tensor grad_out,
                             torch::Tensor grad) {
@@ -552,6 +561,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("router_topk", &router_topk, py::arg("logits"), py::arg("bias"), py::arg("mode"), py::arg("n_groups"), py::arg("topk_groups"),
         py::arg("scale"), py::arg("idx"), py::arg("weights"), py::arg("parts") = 1);
   m.def("router_split", &router_split);
+  m.def("router_split_transposed", &router_split_transposed);
   m.def("rope", &rope);
   m.def("swiglu", &swiglu);
   m.def("add3", &add3);

@@ -23,5 +23,7 @@ cudaError_t launch_router_split(const float* w, int64_t numel, void* stacked, cu
 // E % n_groups == 0), optional bias fp32 [E] added.  idx int64 [N, K], weights fp32 [N, K]; K <= 32.
 cudaError_t launch_router_topk(const float* logits, const float* bias, int N, int E, int K, int mode, int n_groups,
                                int topk_groups, float scale, int64_t* idx, float* weights, cudaStream_t stream, int parts = 1);
+// The three terms of the transposed matrix: w fp32 [rows, cols] -> stacked bf16 [3 cols, rows].
+cudaError_t launch_router_split_transposed(const float* w, int rows, int cols, void* stacked, cudaStream_t stream);
 
 }  // namespace epb

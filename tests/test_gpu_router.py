@@ -65,3 +65,20 @@ def test_a_nan_logit_spoils_its_own_sigmoid_weight_only():
     val, ridx = torch.topk(x, 4, dim=-1)
     assert torch.equal(idx, ridx)
     assert torch.allclose(prob, torch.sigmoid(val), atol=1e-6, equal_nan=True) and int(prob.isnan().sum()) == 1
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (31, 33), (64, 2048), (1531, 64), (8192, 160)])
+def test_native_split_has_the_bits_of_the_operations(rows, cols):
+    """Three bf16 terms of an fp32 matrix and of its transpose: tile edges of the transposing kernel, subnormals, infinities."""
+    from ep_balance_b200.models.moe_layer import _split3
+
+    torch.manual_seed(rows)
+    w = torch.randn(rows, cols, device="cuda") * torch.logspace(-38, 30, cols, device="cuda")
+    w[0, 0] = float("inf")
+    w[-1, -1] = 1e-41
+    for transposed in (False, True):
+        with torch.no_grad():
+            native = _split3(w, transposed)
+        plain = _split3(w.clone().requires_grad_(True), transposed).detach()  # recorded: the operations themselves
+        same = (native.view(torch.int16) == plain.view(torch.int16)) | (native.isnan() & plain.isnan())
+        assert native.shape == plain.shape and bool(same.all())
