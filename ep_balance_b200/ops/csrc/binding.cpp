@@ -212,7 +212,13 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
     cuda_check(epb::launch_ragged_gemm(tmB, tmA, g, (int)num_sms, current_stream()), "launch_ragged_gemm");
     return;
   }
-  cuda_check(epb::launch_grouped_gemm(tmA, tmB, g, (int)num_sms, current_stream()), "launch_grouped_gemm");
+  CUtensorMap tmC;
+  const bool wgrad = mode == epb::kWgrad;
+  const int64_t slot = (int64_t)g.M_out * g.N;  // elements of a gradient slot
+  TORCH_CHECK(!wgrad || (slot > 0 && out0.numel() >= slot), "wgrad: out0 is [slots, M_out, N]");
+  TORCH_CHECK(!wgrad || epb::make_tmap_3d(&tmC, memory(out0, "out0"), out0.numel() / slot, g.M_out, g.N, 64, 32),
+              "cuTensorMapEncodeTiled failed");
+  cuda_check(epb::launch_grouped_gemm(tmA, tmB, g, (int)num_sms, current_stream(), wgrad ? &tmC : nullptr), "launch_grouped_gemm");
 }
 
 // In-place AdamW step on one tensor (param, grad and both moments share dtype and shape).

@@ -167,7 +167,7 @@ __device__ __forceinline__ void wide_flush(const uint4* tile, int lane, char* ro
 }
 // Accumulation in fp32: a tile of 32 rows x 32 columns (128 B a row, the 128-byte swizzle of the tensor map, which is wide_index)
 // is loaded, added to and stored back by bulk tensor copies.  Every element has one writer and is touched once a launch.
-__device__ __forceinline__ void accum_store(const CUtensorMap* map, const void* tile, int col, int row, int slot) {
+__device__ __forceinline__ void tile_store(const CUtensorMap* map, const void* tile, int col, int row, int slot) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem_u32(tile)), "r"(col),
                "r"(row), "r"(slot)
                : "memory");
@@ -186,13 +186,16 @@ __device__ __forceinline__ void accum_add(uint4* tile, int lane, const uint32_t 
 }
 // ---------------------------------------------------------------- kernel
 // kComm: 0 = GEMM only; 1 = plus two transport warps (token or gradient rows to their hosts, replica weights in).
-// kAccum (kWgrad): owned slots are added to the fp32 accumulator (map tmAcc) instead of being stored.  Bound by HBM: 8 bytes a
+// kAccum (kWgrad): owned slots are added to the fp32 accumulator (map tmC) instead of being stored.  Bound by HBM: 8 bytes a
 // weight.  Each epilogue warp loads its 16 KB of the accumulator a tile ahead, so that the loads run beside the tile's MMAs, adds
 // in shared memory and stores by bulk copies.
+// kWgrad without it: tmC is the map of the bf16 gradient; a staged tile of 32 rows x 64 columns leaves by one bulk copy, which
+// spares the epilogue warps eight rounds of shared-memory reads, shuffles and stores.  64 experts of 2048 x 1024 with 191 rows
+// each, where the epilogue is most of a tile: 283 + 151 -> 241 + 131 us; 768 rows: equal (the power limit sets the pace).
 template <int kMode, int kCtas, int kComm, bool kAccum>
 __global__ void __launch_bounds__(NUM_THREADS + (kComm ? COMM_WARPS * 32 : 0), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmAcc, const __grid_constant__ GemmArgs args) {
+                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ GemmArgs args) {
   static_assert(kCtas == 1 || kComm == 0, "the fused transport of a CTA pair is in ragged_gemm.cu");
   using G = Geometry<kCtas, kComm, kAccum>;
   constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, TILE_M = G::TILE_M;
@@ -412,7 +415,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (lane != 0 || !accumulates(x) || n == 0 || old_row(x) >= args.M_out) return;
       mbar_expect_tx(&old_full[warp - 2], n * kStageWarpBytes);
       for (int c = 0; c < n; ++c)
-        tma_load_3d(stg + c * (kStageWarpBytes / 16), &tmAcc, &old_full[warp - 2], x.nt * BN + (half * 4 + c) * 32, old_row(x), x.wslot);
+        tma_load_3d(stg + c * (kStageWarpBytes / 16), &tmC, &old_full[warp - 2], x.nt * BN + (half * 4 + c) * 32, old_row(x), x.wslot);
     };
     int ahead = 0;
     Tile t_next;
@@ -472,7 +475,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
               __syncwarp();
               if (lane == 0) {
-                accum_store(&tmAcc, tile, t.nt * BN + (cb + k) * 32, old_row(t), t.wslot);
+                tile_store(&tmC, tile, t.nt * BN + (cb + k) * 32, old_row(t), t.wslot);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
               }
             }
@@ -570,6 +573,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       } else {
         // kFwd2 / kDgrad1 / kPlain: plain rows, optionally scattered to the unit's source rank.
         // kWgrad: rows of the weight gradient of this group's slot.
+        const int m0 = t.mt * TILE_M + cta_rank * BM + quarter * 32;  // kWgrad: this warp's first output row
         const bool have_acc = kMode != kWgrad || t.rows > 0;  // an expert that received no rows has a zero gradient
         const int col0 = t.nt * BN;
         const int nchunks = min(BN / 32, (args.N - col0) / 32);
@@ -588,6 +592,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             } else {
 #pragma unroll
               for (int i = 0; i < 4; ++i) pk[i] = make_uint4(0, 0, 0, 0);
+            }
+            if (kMode == kWgrad && !kAccum) {
+              if ((k & 1) == 0) {  // the tile's previous copy has read it
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
+              }
+              wide_store_half(stg, lane, pk, k & 1);
+              if ((k & 1) || c + 1 >= nchunks) {  // (columns past N are clipped by the map)
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                  if (m0 < args.M_out) tile_store(&tmC, stg, col0 + (c - (k & 1)) * 32, m0, t.wslot);
+                  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+              }
+              continue;
             }
             wide_store_half(stg, lane, pk, k & 1);
             if ((k & 1) || c + 1 >= nchunks) wide_flush(stg, lane, orow, (col0 + (c - (k & 1)) * 32) * 2, (k & 1) ? 8 : 4);
@@ -608,7 +628,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (have_next) fetch_old(t_next);
       }
     }
-    if (kAccum && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (kMode == kWgrad && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (args.done_ctr != nullptr) __threadfence_system();  // this warp's (peer) stores before the completion signal
   }
 
@@ -713,7 +733,7 @@ bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_
 
 template <int kMode, int kCtas, int kComm, bool kAccum = false>
 static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                               cudaStream_t stream, const CUtensorMap* accum = nullptr) {
+                               cudaStream_t stream, const CUtensorMap* c_map = nullptr) {
   static bool configured[kMaxTrackedDevices] = {};
   constexpr size_t smem = smem_bytes<kCtas, kComm, kAccum>();
   int dev;
@@ -735,11 +755,12 @@ static cudaError_t launch_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, c
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, kAccum ? *accum : tmA, args);
+  return cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<kMode, kCtas, kComm, kAccum>, tmA, tmB, c_map != nullptr ? *c_map : tmA, args);
 }
 
 cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                                cudaStream_t stream, const CUtensorMap* accum) {
+                                cudaStream_t stream, const CUtensorMap* dw, const CUtensorMap* accum) {
+  if (args.mode == kWgrad && dw == nullptr) return cudaErrorInvalidValue;
   if (args.n_groups_cap > MAX_GROUPS) return cudaErrorInvalidValue;
   if (args.mode == kFwd1 && args.N % 128 != 0) return cudaErrorInvalidValue;
   if (args.N % 32 != 0) return cudaErrorInvalidValue;
@@ -749,7 +770,7 @@ cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, 
     if (args.mode == kDgrad2) return launch_mode<kDgrad2, 2, 0>(tmA, tmB, args, num_sms, stream);
     if (args.mode != kWgrad) return cudaErrorInvalidValue;
     if (accum != nullptr) return launch_mode<kWgrad, 2, 0, true>(tmA, tmB, args, num_sms, stream, accum);
-    return launch_mode<kWgrad, 2, 0>(tmA, tmB, args, num_sms, stream);
+    return launch_mode<kWgrad, 2, 0>(tmA, tmB, args, num_sms, stream, dw);
   }
   if (comm) {
     // fused transport exists for the two GEMMs that consume freshly dispatched rows
@@ -764,7 +785,7 @@ cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, 
     case kDgrad1: return launch_mode<kDgrad1, 1, 0>(tmA, tmB, args, num_sms, stream);
     case kWgrad:
       if (accum != nullptr) return launch_mode<kWgrad, 1, 0, true>(tmA, tmB, args, num_sms, stream, accum);
-      return launch_mode<kWgrad, 1, 0>(tmA, tmB, args, num_sms, stream);
+      return launch_mode<kWgrad, 1, 0>(tmA, tmB, args, num_sms, stream, dw);
     case kPlain: return launch_mode<kPlain, 1, 0>(tmA, tmB, args, num_sms, stream);
     default: return cudaErrorInvalidValue;
   }

@@ -95,9 +95,9 @@ bool make_tmap_gate_up(CUtensorMap* out, const void* base, uint64_t slots, uint6
 // fp32 accumulator of kWgrad: [slots, rows, cols], box {32, 32, 1}, 128-byte swizzle.
 bool make_tmap_accum(CUtensorMap* out, const void* base, uint64_t slots, uint64_t rows, uint64_t cols);
 
-// accum (kWgrad, may be null): map of the fp32 accumulator [home_cap, M_out, N].  The gradient of a slot below home_cap is added
+// dw (kWgrad): map of out0 [slots, M_out, N], make_tmap_3d with box {64, 32, 1}; accum (kWgrad, may be null): map of the fp32 accumulator [home_cap, M_out, N].  The gradient of a slot below home_cap is added
 // there from the fp32 sums and its slot of out0 is not written.
 cudaError_t launch_grouped_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, int num_sms,
-                                cudaStream_t stream, const CUtensorMap* accum = nullptr);
+                                cudaStream_t stream, const CUtensorMap* dw = nullptr, const CUtensorMap* accum = nullptr);
 
 }  // namespace epb

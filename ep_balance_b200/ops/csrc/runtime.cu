@@ -150,6 +150,9 @@ MoeRuntime::MoeRuntime(const LayerConfig& cfg, const std::map<std::string, uint6
   tmap2(&tm_dh_mn_, ptr<void>("hbuf"), T, 2 * F, 64, 64);
   tmap2(&tm_x_mn_, ptr<void>("xbuf"), T, H, 64, 64);
 
+  // Wgrad's results, as its epilogue stages them
+  tmap3(&tm_gw1_, ptr<void>("gw1"), S, 2 * F, H, 64, 32);
+  tmap3(&tm_gw2_, ptr<void>("gw2"), S, H, F, 64, 32);
   if (fused_accum() && (!make_tmap_accum(&tm_acc1_, ptr<void>("acc_gw1"), c.home_cap, 2 * F, H) ||
                         !make_tmap_accum(&tm_acc2_, ptr<void>("acc_gw2"), c.home_cap, H, F)))
     throw std::runtime_error("MoeRuntime: cuTensorMapEncodeTiled (accumulators) failed");
@@ -356,7 +359,7 @@ void MoeRuntime::gemm(int mode, const CUtensorMap& a, const CUtensorMap& b, int 
   else if (mode != kWgrad && cfg_.gemm_ctas == 2)
     check(launch_ragged_gemm(b, a, g, cfg_.num_sms, stream), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
   else
-    check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream, extra.accum), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
+    check(launch_grouped_gemm(a, b, g, cfg_.num_sms, stream, extra.dw, extra.accum), extra.comm ? "grouped_gemm+transport" : "grouped_gemm");
 }
 
 // An inference batch with few rows per expert reads the weights once and does little else.  (About num_units rows reach
@@ -579,6 +582,7 @@ bool MoeRuntime::fused_accum() const { return cfg_.accum_fp32 && ptr<float>("acc
 // No gate: Dgrad2, earlier on this stream, has waited for every gradient row of this rank.
 void MoeRuntime::wgrad2(cudaStream_t stream) {
   GemmExtra x;
+  x.dw = &tm_gw2_;
   if (fused_accum()) x.accum = &tm_acc2_;
   gemm(kWgrad, tm_dy_mn_, tm_act_mn_, cfg_.F, 0, cfg_.H, ptr<void>("gw2"), nullptr, nullptr, nullptr, stream, x);
 }
@@ -611,6 +615,7 @@ void MoeRuntime::dgrad2_fused(const void* dout, int num_units, cudaStream_t stre
 }
 void MoeRuntime::wgrad1(cudaStream_t stream) {
   GemmExtra x;
+  x.dw = &tm_gw1_;
   if (fused_accum()) x.accum = &tm_acc1_;
   gemm(kWgrad, tm_dh_mn_, tm_x_mn_, cfg_.H, 0, 2 * cfg_.F, ptr<void>("gw1"), nullptr, nullptr, nullptr, stream, x);
 }

@@ -127,6 +127,7 @@ class MoeRuntime {
     int done_slot = 0;   // > 0: signal every peer on this slot when the launch is complete
     const float* row_scale = nullptr;
     const CommArgs* comm = nullptr;
+    const CUtensorMap* dw = nullptr;     // Wgrad: the gradient slots
     const CUtensorMap* accum = nullptr;  // Wgrad: fp32 accumulation buffer of the owned slots
     bool narrow = false; // few rows per expert: weights on the M side (narrow_gemm.h)
   };
@@ -166,6 +167,7 @@ class MoeRuntime {
   CUtensorMap tm_x_k_, tm_act_k_, tm_dy_k_, tm_dh_k_;           // K-major A operands
   CUtensorMap tm_w1_k_, tm_w2_k_, tm_w1_mn_, tm_w2_mn_;          // weights as B
   CUtensorMap tm_w1_g_;                                          // gate and up blocks of the CTA-pair kernel
+  CUtensorMap tm_gw1_, tm_gw2_;                                  // gradient slots
   CUtensorMap tm_acc1_, tm_acc2_;                                // fp32 gradient accumulators
   CUtensorMap tm_x_n_, tm_act_n_;                                // token rows as the narrow kernel's N operand
   CUtensorMap tm_dy_mn_, tm_act_mn_, tm_dh_mn_, tm_x_mn_;        // Wgrad operands (MN-major)
