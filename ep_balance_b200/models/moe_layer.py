@@ -61,7 +61,7 @@ class MoEConfig:
     inter_cost: int = 8
     router_dtype: torch.dtype = torch.float32
     normalize_topk: bool = True
-    gemm_ctas: int = 2  # 2: CTA-pair grouped GEMM (256-row tiles); 1: single-CTA kernel (128-row tiles)
+    gemm_ctas: int = 2  # 2: CTA-pair grouped GEMMs (groups start at multiples of 256 rows); 1: single-CTA kernel (128-row tiles)
     # None: every backward overwrites ``param.grad``.  torch.bfloat16 / torch.float32: every backward ADDS the
     # expert weight gradients into an accumulation buffer of that dtype (``param.grad`` for bf16,
     # ``param.main_grad`` for fp32), for steps made of several micro-batches; clear it with

@@ -1,12 +1,11 @@
 // Grouped GEMM for few rows per expert: the WEIGHTS are the 128-row operand of the tensor core, the token rows are
 // its N columns.
 //
-// grouped_gemm.cu puts token rows on the M side, in tiles of 256 (or 128) rows.  An expert with 4 or 100 rows then
-// costs as much tensor-core time, shared memory and L2 traffic as one with 256.  Such launches are bound by reading the
-// weights once from HBM; here a tile is 256 weight rows (output features) x up to 128 token rows, N is the real row
-// count rounded up to 16, and every byte that the ring keeps in flight beyond a few KB is a weight byte.  No padding
-// row is read into a result or written, so nothing has to be zero-filled around the rows.  128 experts of 2048 x 768 with 4
-// rows each: GEMM1 141 us (805 MB of weights: 5.7 TB/s) against 203, GEMM2 71 (5.7 TB/s) against 124.  Four 48 KB
+// Launches of 4 or 100 rows an expert are bound by reading the weights once from HBM.  Here one CTA's tile is 256 weight rows
+// (output features) x up to 128 token rows, N is the real row count rounded up to 16, and every byte that the ring keeps in
+// flight beyond a few KB is a weight byte (the CTA-pair kernel of ragged_gemm.cu brings a box of 128 token rows a CTA whatever
+// the tile holds).  No padding row is read into a result or written.  128 experts of 2048 x 768 with 4 rows each: GEMM1 141 us
+// (805 MB of weights: 5.7 TB/s), GEMM2 71 (5.7 TB/s); with token rows in tiles of 256 on the M side they took 203 and 124.  Four 48 KB
 // stages keep 128 KB of weights in flight per SM; pairing SMs would halve the token bytes only, which are few.
 //
 //   kFwd1    act = SwiGLU(X W1^T)   gate block + up block of a tile

@@ -185,7 +185,7 @@ struct SwigluBwdArgs {
   int rows, F;
   const int32_t* row_limit;     // device: rows in use (may be null)
   const float* rowp;            // [rows] or null
-  const int2* meta;             // [rows] {src rank, position at the source}; rows with src < 0 are padding
+  const int2* meta;             // [rows] {src rank, position at the source}; rows with src < 0 are padding and stay as they are
   float* const* dprob_ptrs;     // R peers: float [U] or null
 };
 cudaError_t launch_swiglu_backward(const SwigluBwdArgs& a, cudaStream_t stream);
