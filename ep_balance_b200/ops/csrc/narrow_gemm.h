@@ -10,14 +10,14 @@ namespace epb {
 constexpr int kNarrowBoxRows = 32;  // token rows of one TMA box: box of the token map {64 k, kNarrowBoxRows}
 
 // Inference batches with at most this many routed units per weight slot take the narrow kernel.  Measured, GEMM1 + GEMM2 in us,
-// wide / narrow, rows per expert spread by a lognormal of 0.35 around the mean:
-//   hidden x ffn x experts   4 rows       96 rows      128 rows     192 rows     384 rows
-//   2048 x  768 x 128        327 /  212   351 /  254   353 /  260   381 /  322   629 /  536
-//   5120 x 1536 x 160       1856 / 1176  2210 / 1397  2132 / 1867  2246 / 2312  3672 / 3808
-//   2048 x 1408 x  64        302 /  206   295 /  241   311 /  268   337 /  337   570 /  578
-// One line for every shape, at the most rows where the narrow kernel won each of them: the weights' bytes bound the launch up
-// to there.  Beyond it the shapes disagree.  Wide rows and many weights do better on the full 256-row tiles, which move fewer
-// operand bytes per flop; the first shape, with its short reductions, would keep 15 % on the narrow kernel up to 384 rows.
+// CTA pair (ragged_gemm.cu) / narrow, rows per expert spread by a lognormal of 0.35 around the mean, back to back:
+//   hidden x ffn x experts   96 rows      128 rows     192 rows     384 rows
+//   2048 x  768 x 128        248 /  232   264 /  265   302 /  331   476 /  554
+//   5120 x 1536 x 160       1366 / 1252  1524 / 1514  1584 / 1936  2683 / 3780
+//   2048 x 1408 x  64        258 /  241   267 /  341   289 /  369   409 /  576
+// One line for every shape: below it the weights' bytes bound the launch and the narrow kernel moves fewer others, above it an
+// expert's rows no longer fit one of its tiles.  At the line the two are level, but for the third shape under the power limit
+// (by itself the narrow kernel takes 232-250 there).
 constexpr int kNarrowRowsPerSlot = 128;
 
 // tmW: the weight map that grouped_gemm.h's kernels use as B (K-major box {64, 128, 1}); tmX: token rows, 2-D, box
