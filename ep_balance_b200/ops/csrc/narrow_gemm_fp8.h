@@ -17,7 +17,8 @@ constexpr int kNarrowFp8BoxRows = 32;  // token rows of one TMA box
 //   2048 x 1408 x  64        167 / 116   166 / 135   175 / 149   191 / 168   203 / 183   232 / 219
 //   1024 x  512 x 256        161 / 119   184 / 172   195 / 191   206 / 209   224 / 234   246 / 274
 // Up to 128 rows the narrow kernel wins everywhere; from there to the line each kernel wins by up to 14 % at some shapes, and
-// by 384 rows the pair kernel is ahead at all of them.  (16 rows of the first shape read 1.41 GB of weights: 215 us at the rate
+// by 384 rows the pair kernel is ahead at all of them.  (Pair before its stages of two k-blocks, which took 6 % off
+// a prefill of 1024 rows an expert.)  (16 rows of the first shape read 1.41 GB of weights: 215 us at the rate
 // of a copy.)
 constexpr int kNarrowFp8RowsPerSlot = 192;
 
